@@ -1,0 +1,96 @@
+"""The closest-point query's paths against each other: FP64 queries that prune
+in FP32 against those that take the FP64 nodes, and walks spread over few or
+all lanes of a warp."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def tb(lib_built):
+    import twos_b200
+    return twos_b200
+
+
+def _fan(n):
+    """A closed double cone: n triangles meet at each apex (more than an FP64
+    query holds as candidates)."""
+    t = 2 * np.pi * np.arange(n) / n
+    V = np.concatenate([np.c_[np.cos(t), np.sin(t), np.zeros(n)], [[0, 0, 0.5], [0, 0, -0.5]]])
+    i = np.arange(n)
+    j = (i + 1) % n
+    return V, np.concatenate([np.c_[i, j, np.full(n, n)], np.c_[j, i, np.full(n, n + 1)]]).astype(np.uint32)
+
+
+def _points(V, F, seed):
+    rng = np.random.default_rng(seed)
+    lo, hi = V.min(0), V.max(0)
+    on = V[rng.integers(0, len(V), 40)]
+    mid = V[F[rng.integers(0, len(F), 40)].astype(np.int64)].sum(1) / 3.0  # triangle centroids
+    return np.concatenate([lo + (hi - lo) * rng.random((300, 3)), on * (1 + 1e-9), on, on * 3.0, mid,
+                           V.mean(0, keepdims=True), rng.normal(size=(20, 3)) * 1e3])
+
+
+@pytest.mark.parametrize("shape", ["sphere", "noise", "fan5", "fan64", "sliver"])
+@pytest.mark.parametrize("exponent", [-60, 60])
+def test_fp32_pruning_gives_the_fp64_minimum(tb, shape, exponent):
+    """Scaling by a power of two is exact in FP64, so a mesh too small or too
+    large for FP32 pruning (which takes the FP64 nodes) has exactly the scaled
+    distances of the original, which prunes in FP32."""
+    if shape == "sphere":
+        V, F = tb.geometry.icosphere(3)
+    elif shape == "noise":
+        V, F = tb.geometry.noise_sphere(4, 2)
+    elif shape == "sliver":  # needle triangles, aspect 1e-7
+        V, F = tb.geometry.icosphere(2)
+        V = V * np.array([1.0, 1e-7, 1.0])
+    else:
+        V, F = _fan(int(shape[3:]))
+    P = _points(V, F, 3)
+    s = 2.0 ** exponent
+    with tb.Mesh(V, F) as a, tb.Mesh(V * s, F) as b:
+        da, qa = a.closest_point(P, precision="fp64")
+        db, qb = b.closest_point(P * s, precision="fp64")
+    assert np.array_equal(da * s, db)
+    # The nearest point is unique up to rounding except on the medial axis.
+    assert np.max(np.abs(np.linalg.norm(P - qa, axis=1) - da)) <= 4e-16 * 2e3
+    assert np.max(np.abs(np.linalg.norm(P * s - qb, axis=1) - db)) <= 4e-16 * 2e3 * s
+
+
+@pytest.mark.parametrize("offset", [0.0, 1e4, 1e8])
+def test_far_points_and_offset_meshes(tb, offset):
+    """Points beyond FP32 squares and meshes far from the origin keep their
+    FP64 distances (against every triangle's vertices and faces in numpy: the
+    sphere's nearest point is a vertex or inside a face, within its sagitta)."""
+    V, F = tb.geometry.icosphere(3)
+    d = np.array([[1.0, 2.0, -2.0], [0.3, -0.1, 0.95]]) / np.array([[3.0], [1.0]])
+    P = np.concatenate([d[:1] * r for r in (2.0, 1e6, 2.0 ** 40, 2.0 ** 55, 1e25)] + [d[1:] * 0.4])
+    with tb.Mesh(V + offset, F) as m:
+        dist, _ = m.closest_point(P + offset, precision="fp64")
+    T = V[F.astype(np.int64)]
+    upper = np.min(np.linalg.norm(P[:, None] - V[None], axis=2), axis=1)  # nearest vertex
+    n = np.cross(T[:, 1] - T[:, 0], T[:, 2] - T[:, 0])
+    n /= np.linalg.norm(n, axis=1)[:, None]
+    lower = np.maximum(np.linalg.norm(P, axis=1) - 1.0, 0.0)  # outside the unit ball
+    scale = 1e-15 * (np.linalg.norm(P, axis=1) + 4 * offset + 1)
+    assert np.all(dist <= upper + scale) and np.all(dist >= lower - scale)
+    inner = np.min(np.einsum("fk,fk->f", n, T[:, 0]) - P[-1] @ n.T)
+    assert abs(dist[-1] - inner) <= 1e-15 * (4 * offset + 4)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_walks_do_not_depend_on_the_lanes_that_run_them(tb, precision):
+    """One site per launch (2 to 700 walks: one lane per warp) and all sites in
+    one launch (up to all 32 lanes) walk the same samples."""
+    V, F = tb.geometry.noise_sphere(3, 1)
+    sites = tb.geometry.uniform_ball(200, 0.6, seed=4)
+    with tb.Mesh(V, F) as m:
+        for walks in (2, 33, 700):
+            cfg = tb.Config(walks=walks, precision=precision, seed=6, epsilon=1e-3)
+            every = m.walk_samples(sites, cfg)
+            for s in (0, 17, 199):
+                one = m.walk_samples(sites[s], tb.Config(walks=walks, precision=precision, seed=6, epsilon=1e-3,
+                                                         site_offset=s))
+                assert np.array_equal(one["u"][0], every["u"][s])
+                assert np.array_equal(one["steps"][0], every["steps"][s])

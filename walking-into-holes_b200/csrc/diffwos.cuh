@@ -138,8 +138,7 @@ __device__ double closest_distance_fp64(const GeoDesc &G, double x, double y, do
                                         bool required, uint2 *stack, int stride, uint32_t &err) {
   double best2 = radius2;
   uint32_t tri = 0;
-  const bool found = nearest<double>(G.nodes_d, G.tris_d, G.max_iter, Vec<double>{x, y, z}, best2, tri, stack,
-                                     stride, err);
+  const bool found = nearest_geo(G, Vec<double>{x, y, z}, best2, tri, stack, stride, err);
   if (!found) {
     if (required) err |= TWOS_DEVERR_QUERY;
     return CUDART_INF;
@@ -150,7 +149,7 @@ __device__ double closest_distance_fp64(const GeoDesc &G, double x, double y, do
 }  // namespace
 
 __global__ void __launch_bounds__(128) diff_classify_kernel(const DiffLaunch D) {
-  __shared__ uint2 s_stack[kStack * 128];
+  __shared__ uint2 s_stack[(kStack + kCand) * 128];
   uint2 *stack = s_stack + threadIdx.x;
   const GeoDesc G = *D.geo;
   uint32_t err = 0;

@@ -198,13 +198,18 @@ __device__ __forceinline__ void ldg32(const void *p, float4 &a, float4 &b) {
       : "l"(p));
 }
 
-__device__ __forceinline__ void node_dist2(const NodeF *__restrict__ nodes, int idx, const Vec<float> &p,
-                                           float &dl, float &dr, int &cl, int &cr) {
-  const NodeF *n = nodes + idx;
-  float4 x, y, z, nl, nr, t;
-  ldg32(&n->x, x, y);
-  ldg32(&n->z, z, nl);
-  ldg32(&n->nr, nr, t);
+// ldg32 under a condition; a and b are left alone without it.
+__device__ __forceinline__ void ldg32_if(bool cond, const void *p, float4 &a, float4 &b) {
+  asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %9, 0;\n\t"
+      "@q ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t}"
+      : "+f"(a.x), "+f"(a.y), "+f"(a.z), "+f"(a.w), "+f"(b.x), "+f"(b.y), "+f"(b.z), "+f"(b.w)
+      : "l"(p), "r"(static_cast<int>(cond)));
+}
+
+// The bounds from a loaded node (its six float4 in order).
+__device__ __forceinline__ void node_bounds(const float4 &x, const float4 &y, const float4 &z, const float4 &nl,
+                                            const float4 &nr, const float4 &t, const Vec<float> &p, float &dl,
+                                            float &dr, int &cl, int &cr) {
   const float lx = gap(x.x, x.z, p.x), rx = gap(x.y, x.w, p.x);
   const float ly = gap(y.x, y.z, p.y), ry = gap(y.y, y.w, p.y);
   const float lz = gap(z.x, z.z, p.z), rz = gap(z.y, z.w, p.z);
@@ -215,6 +220,16 @@ __device__ __forceinline__ void node_dist2(const NodeF *__restrict__ nodes, int 
   dr = fmaxf(__fmaf_rn(rx, rx, __fmaf_rn(ry, ry, rz * rz)), gr * gr);
   cl = __float_as_int(t.z);
   cr = __float_as_int(t.w);
+}
+
+__device__ __forceinline__ void node_dist2(const NodeF *__restrict__ nodes, int idx, const Vec<float> &p,
+                                           float &dl, float &dr, int &cl, int &cr) {
+  const NodeF *n = nodes + idx;
+  float4 x, y, z, nl, nr, t;
+  ldg32(&n->x, x, y);
+  ldg32(&n->z, z, nl);
+  ldg32(&n->nr, nr, t);
+  node_bounds(x, y, z, nl, nr, t, p, dl, dr, cl, cr);
 }
 
 __device__ __forceinline__ void node_dist2(const NodeD *__restrict__ nodes, int idx, const Vec<double> &p,
@@ -316,13 +331,16 @@ __device__ __forceinline__ void load_tri(const TriD *__restrict__ tris, uint32_t
 // One triangle against the current best: the plane-slab bound first, the
 // full closest-point test only when the bound is below best.  Returns true
 // when the triangle is strictly closer (best2 updated); `full` counts full tests.
+__device__ __forceinline__ float plane_gap2(const float4 &P, const float4 &A, const Vec<float> &p) {
+  const float s = __fmaf_rn(P.x, p.x, __fmaf_rn(P.y, p.y, P.z * p.z));
+  const float g = gap(P.w, A.w, s);
+  return g * g;
+}
 __device__ __forceinline__ bool tri_test(const TriF *__restrict__ tris, uint32_t i, const Vec<float> &p, float &best2,
                                          uint32_t &full) {
   float4 P, A;
   ldg32(&tris[i].plane, P, A);
-  const float s = __fmaf_rn(P.x, p.x, __fmaf_rn(P.y, p.y, P.z * p.z));
-  const float g = gap(P.w, A.w, s);
-  if (!(g * g < best2)) return false;
+  if (!(plane_gap2(P, A, p) < best2)) return false;
   ++full;
   float4 B, C;
   ldg32(&tris[i].b, B, C);
@@ -358,10 +376,9 @@ __device__ __forceinline__ float lower_f(double v) { return __double2float_rd(v)
 template <typename T>
 __device__ bool nearest(const typename Layout<T>::Node *__restrict__ nodes,
                         const typename Layout<T>::Tri *__restrict__ tris, uint32_t max_iter, const Vec<T> &p,
-                        T &best2, uint32_t &best_tri, uint2 *stack, int stride, uint32_t &err) {
+                        T &best2, uint32_t &best_tri, uint2 *stack, int stride, uint32_t &err, int node = 0) {
   bool found = false;
   int sp = 0;
-  int node = 0;
   bool have = true;
   uint32_t iter = 0;
   while (have) {
@@ -608,6 +625,252 @@ __device__ __forceinline__ bool grid_bound(const GeoDesc &g, const Vec<float> &p
   return grid_bounds(g, p, bound, upper, entry_node);
 }
 
+// ---------------------------------------------------------------- FP64 queries
+// The FP64 form's closest-point query searches the FP32 BVH: whatever only
+// prunes need not be FP64, as long as it leaves room for its error.  `margin`
+// bounds the difference between an FP32 distance bound at p (node boxes,
+// normal slabs, triangle planes, the two bounds of a triangle below) and the
+// FP64 distance: the session's delta (vertices, boxes and slabs rounded to
+// FP32, the arithmetic) plus the rounding of the point itself.  The search
+// keeps the triangles whose lower bound stays below the smallest upper bound
+// plus two margins -- nearly always one or two -- and only those get the FP64
+// closest-point test, together with the warp's next walk step.  Every triangle
+// that could hold the FP64 minimum is among them, so the result is the
+// minimum an FP64 search gives, bit for bit, at half the node bytes and
+// full-rate arithmetic.
+struct Cull {
+  Vec<float> p;   // the query point in the FP32 frame
+  float margin;
+  float limit;    // squared FP32 pruning threshold
+  int count;      // candidates held
+};
+
+// (sqrt(best2) + margin)^2 rounded up (infinite for an unbounded query).
+__device__ __forceinline__ float cull_limit(double best2, float margin) {
+  const float t = __fadd_ru(__fsqrt_ru(__double2float_ru(best2)), margin);
+  return __fmul_ru(t, t);
+}
+
+// Sets up the search at p for distances below sqrt(best2); false when FP32
+// cannot hold the geometry or the point (cull_margin 0: see open_impl; a
+// coordinate beyond 2^50, whose square would overflow, or NaN), and the
+// caller takes the FP64 nodes.
+__device__ __forceinline__ bool cull_begin(const GeoDesc &g, const Vec<double> &p, double best2, Cull &c) {
+  const double xyz[3] = {p.x, p.y, p.z};
+  c.p = to_frame<float>(xyz, g);
+  const float norm1 = fabsf(c.p.x) + fabsf(c.p.y) + fabsf(c.p.z);
+  c.margin = __fmaf_ru(norm1, 0x1.0p-20f, g.cull_margin);
+  c.limit = cull_limit(best2, c.margin);
+  c.count = 0;
+  return g.cull_margin > 0.f && norm1 < 0x1.0p50f;
+}
+
+// A point of the triangle at (nearly) its closest to p: Ericson's regions as
+// tri_closest, with the interior weights clamped so that the point stays in
+// the triangle whatever their rounding (degenerate triangles included).
+__device__ __forceinline__ Vec<float> tri_point(const Vec<float> &ap, const Vec<float> &bp, const Vec<float> &cp,
+                                                const Vec<float> &ab, const Vec<float> &ac) {
+  // Returned as the vector from the point to p.
+  const float d1 = dot3(ab, ap), d2 = dot3(ac, ap);
+  if (d1 <= 0.f && d2 <= 0.f) return ap;
+  const float d3 = dot3(ab, bp), d4 = dot3(ac, bp);
+  if (d3 >= 0.f && d4 <= d3) return bp;
+  const float vc = mad_t(d1, d4, -(d3 * d2));
+  if (vc <= 0.f && d1 >= 0.f && d3 <= 0.f) return add_scaled(ap, ab, -__saturatef(__fdividef(d1, d1 - d3)));
+  const float d5 = dot3(ab, cp), d6 = dot3(ac, cp);
+  if (d6 >= 0.f && d5 <= d6) return cp;
+  const float vb = mad_t(d5, d2, -(d1 * d6));
+  if (vb <= 0.f && d2 >= 0.f && d6 <= 0.f) return add_scaled(ap, ac, -__saturatef(__fdividef(d2, d2 - d6)));
+  const float va = mad_t(d3, d6, -(d5 * d4));
+  if (va <= 0.f && (d4 - d3) >= 0.f && (d5 - d6) >= 0.f)
+    return add_scaled(bp, sub(ac, ab), -__saturatef(__fdividef(d4 - d3, (d4 - d3) + (d5 - d6))));
+  const float denom = __fdividef(1.f, va + vb + vc);
+  const float v = __saturatef(vb * denom);
+  const float w = fminf(__saturatef(vc * denom), 1.f - v);
+  return add_scaled(add_scaled(ap, ab, -v), ac, -w);
+}
+
+// FP64 closest-point test of the held candidates.
+__device__ __forceinline__ bool cull_flush(const GeoDesc &g, const Vec<double> &p, Cull &c, double &best2,
+                                           uint32_t &best_tri, const uint2 *cand, int stride) {
+  bool found = false;
+  for (int k = 0; k < c.count; ++k) {
+    const uint2 e = cand[k * stride];
+    if (!(__uint_as_float(e.y) < c.limit)) continue;  // the limit fell below its bound since
+    Vec<double> ta, tb, tc;
+    load_tri(g.tris_d, e.x, ta, tb, tc);
+    const double d2 = tri_dist2(p, ta, tb, tc);
+    if (d2 < best2) {
+      best2 = d2;
+      best_tri = e.x;
+      found = true;
+    }
+  }
+  c.count = 0;
+  return found;
+}
+
+// Squared lower bound of the distance from p to a triangle along a direction
+// w: the plane through the vertex nearest along w separates them by the
+// smallest w.(p - vertex) / |w|.  Holds for any w; near 0 it bounds nothing.
+__device__ __forceinline__ float support2(const Vec<float> &w, const Vec<float> &ap, const Vec<float> &bp,
+                                          const Vec<float> &cp, float w2) {
+  const float m = fmaxf(fminf(dot3(w, ap), fminf(dot3(w, bp), dot3(w, cp))), 0.f);
+  return w2 > 1e-30f ? __fdividef(m, w2) * m * (1.f - 0x1.0p-18f) : 0.f;
+}
+
+// One triangle of the search: the plane slab, then the bound along the
+// direction to its centroid (it leaves 2.9 of 15.3 triangles a query for the
+// tests below on the 81,920-triangle noise sphere), then two bounds from the
+// vector w from a point of the triangle near its closest to p: |w| from
+// above, and w's own direction from below, whatever the point's rounding.  A
+// triangle within the threshold is held as a candidate; true when the list
+// is full and the caller has to flush it first.
+__device__ __forceinline__ bool cull_tri(uint32_t i, const float4 &P, const float4 &A, const float4 &B,
+                                         const float4 &C, Cull &c, uint2 *cand, int stride, uint32_t &full) {
+  if (!(plane_gap2(P, A, c.p) < c.limit)) return false;
+  if (c.count >= kCand) return true;
+  const Vec<float> a{A.x, A.y, A.z}, b{B.x, B.y, B.z}, cc{C.x, C.y, C.z};
+  const Vec<float> ap = sub(c.p, a), bp = sub(c.p, b), cp = sub(c.p, cc);
+  const Vec<float> t{ap.x + bp.x + cp.x, ap.y + bp.y + cp.y, ap.z + bp.z + cp.z};
+  if (!(support2(t, ap, bp, cp, dot3(t, t)) < c.limit)) return false;
+  ++full;
+  const Vec<float> w = tri_point(ap, bp, cp, sub(b, a), sub(cc, a));
+  const float w2 = dot3(w, w);
+  const float low2 = support2(w, ap, bp, cp, w2);
+  if (!(low2 < c.limit)) return false;
+  cand[c.count * stride] = make_uint2(i, __float_as_uint(low2));
+  ++c.count;
+  const float up = __fmaf_ru(2.f, c.margin, __fsqrt_ru(w2));
+  c.limit = fminf(c.limit, __fmul_ru(up, up));
+  return false;
+}
+
+// Bound and start node of a query from the distance grid: the grid's upper
+// bound plus 6 delta (its 3 delta and the query's own error, with room) is
+// above the distance, so the traversal may prune with it before any triangle
+// is found; when the initial bound is below one entry cell, it starts at the
+// cell's entry node (every triangle outside that subtree is farther).
+__device__ __forceinline__ void grid_start(const GeoDesc &g, const Vec<float> &p, float radius, float &upper,
+                                           int &node) {
+  float bound;
+  int entry = -1;
+  upper = CUDART_INF_F;
+  node = 0;
+  if (!g.grid || !grid_bounds(g, p, bound, upper, entry)) {
+    upper = CUDART_INF_F;
+    return;
+  }
+  upper = __fmaf_ru(6.f, g.delta, upper);
+  if (entry >= 0 && fminf(radius, upper) < g.entry_radius) node = entry;
+}
+
+// nearest() over the FP64 nodes, for what the FP32 bounds cannot hold; out of
+// line and by value, so it costs the callers no registers.
+struct Plain64 {
+  double best2;
+  uint32_t tri;
+  uint32_t flags;  // error bits | found << 31
+};
+__device__ __noinline__ Plain64 nearest_plain64(const GeoDesc *g, double x, double y, double z, double best2) {
+  uint2 stack[kStack];
+  Plain64 r{best2, 0u, 0u};
+  uint32_t err = 0;
+  const bool found = nearest<double>(g->nodes_d, g->tris_d, g->max_iter, Vec<double>{x, y, z}, r.best2, r.tri, stack,
+                                     1, err);
+  r.flags = err | (found ? 0x80000000u : 0u);
+  return r;
+}
+
+// Closest-point query outside the walk kernel, as nearest(), with the
+// distance grid's bound and entry node; the FP64 form culls in FP32.
+__device__ __forceinline__ bool nearest_geo(const GeoDesc &g, const Vec<float> &p, float &best2, uint32_t &best_tri,
+                                            uint2 *stack, int stride, uint32_t &err) {
+  float upper;
+  int node;
+  grid_start(g, p, sqrtf(best2), upper, node);
+  if (upper * upper < best2) best2 = upper * upper;
+  return nearest<float>(g.nodes_f, g.tris_f, g.max_iter, p, best2, best_tri, stack, stride, err, node);
+}
+
+__device__ __forceinline__ bool nearest_geo(const GeoDesc &g, const Vec<double> &p, double &best2,
+                                            uint32_t &best_tri, uint2 *stack, int stride, uint32_t &err) {
+  Cull c;
+  if (!cull_begin(g, p, best2, c)) {
+    const Plain64 r = nearest_plain64(&g, p.x, p.y, p.z, best2);
+    err |= r.flags & 0x7fffffffu;
+    if (!(r.flags >> 31)) return false;
+    best2 = r.best2;
+    best_tri = r.tri;
+    return true;
+  }
+  float upper;
+  int node;
+  grid_start(g, c.p, sqrtf(c.limit), upper, node);
+  const float reach = __fadd_ru(upper, c.margin);
+  c.limit = fminf(c.limit, __fmul_ru(reach, reach));
+  bool found = false;
+  int sp = 0;
+  uint32_t iter = 0;
+  for (bool have = true; have;) {
+    if (++iter > g.max_iter) {
+      err |= TWOS_DEVERR_ITER;
+      break;
+    }
+    if (node >= 0) {
+      float dl, dr;
+      int cl, cr;
+      node_dist2(g.nodes_f, node, c.p, dl, dr, cl, cr);
+      const bool vl = dl < c.limit, vr = dr < c.limit;
+      if (vl && vr) {
+        if (dr < dl) {
+          const float td = dl;
+          dl = dr;
+          dr = td;
+          const int tc = cl;
+          cl = cr;
+          cr = tc;
+        }
+        if (sp >= kStack) {
+          err |= TWOS_DEVERR_STACK;
+          break;
+        }
+        stack[sp * stride] = make_uint2(static_cast<uint32_t>(cr), __float_as_uint(dr));
+        ++sp;
+        node = cl;
+        continue;
+      }
+      if (vl || vr) {
+        node = vl ? cl : cr;
+        continue;
+      }
+    } else {
+      const uint32_t enc = ~static_cast<uint32_t>(node);
+      for (uint32_t i = enc >> 3, e = (enc >> 3) + (enc & 7u), full = 0; i < e; ++i) {
+        float4 P, A, B, C;
+        ldg32(&g.tris_f[i].plane, P, A);
+        ldg32(&g.tris_f[i].b, B, C);
+        if (cull_tri(i, P, A, B, C, c, stack + kStack * stride, stride, full)) {
+          found |= cull_flush(g, p, c, best2, best_tri, stack + kStack * stride, stride);
+          --i;
+        }
+      }
+    }
+    have = false;
+    while (sp > 0) {
+      --sp;
+      const uint2 e = stack[sp * stride];
+      if (__uint_as_float(e.y) < c.limit) {
+        node = static_cast<int>(e.x);
+        have = true;
+        break;
+      }
+    }
+  }
+  found |= cull_flush(g, p, c, best2, best_tri, stack + kStack * stride, stride);
+  return found;
+}
+
 __device__ __forceinline__ uint32_t find_job(const JobDesc *jobs, uint32_t n, uint64_t wid) {
   uint32_t lo = 0, hi = n - 1;
   while (lo < hi) {
@@ -647,7 +910,34 @@ bool launch_tables_in_smem(int precision, uint32_t n_jobs, uint32_t n_geos, uint
                                       : smem_plan<double>(n_jobs, n_geos, n_terms).tables;
 }
 
-enum : int { kIdle = 0, kTraverse = 1, kStep = 2 };
+constexpr int kShared = 8;  // traversal-stack entries per thread in shared memory; the deeper ones are local
+// Shared-memory entries per thread: the traversal stack and, in the FP64
+// form, the candidates of its search.
+template <typename T> __host__ __device__ constexpr int wos_stack_entries() {
+  return sizeof(T) == 4 ? kShared : kShared + kCand;
+}
+
+// A walk's state that its traversal does not touch (position, sums, ids).
+// The mixed form keeps it in registers; the FP64 form, whose state is twice as
+// wide, in shared memory (one word per thread and field, consecutive threads
+// on consecutive words), so the traversal runs without spills: with them, the
+// local memory of 768 threads took the L1 from the BVH's nodes.
+template <typename V, bool SHARED> struct Cell {
+  V v;
+  __device__ __forceinline__ operator V() const { return v; }
+  __device__ __forceinline__ void operator=(V x) { v = x; }
+};
+template <typename V> struct Cell<V, true> {
+  volatile V *p;
+  __device__ __forceinline__ operator V() const { return *p; }
+  __device__ __forceinline__ void operator=(V x) { *p = x; }
+};
+// Shared-memory bytes of that state per thread.
+template <typename T> __host__ __device__ constexpr int wos_cold_bytes(bool gradient) {
+  return sizeof(T) == 4 ? 0 : 72 + (gradient ? 96 : 0);
+}
+
+enum : int { kIdle = 0, kTraverse = 1, kStep = 2, kBegin = 3 };
 
 // Persistent walk-on-spheres kernel as a per-lane state machine.  Each loop
 // iteration every traversing lane runs up to `units` units of work back to
@@ -664,9 +954,20 @@ enum : int { kIdle = 0, kTraverse = 1, kStep = 2 };
 // form, FP64 in the plain form).  SRC: TWOS_SOURCE_* (a
 // template argument, so the exact-integral code of TWOS_SOURCE_EXACT adds no
 // registers to the other forms).
+//
+// What bounds it: instruction issue under the traversal's divergence (7 to 9
+// of 32 lanes per instruction) and, between issues, the dependent loads of
+// nodes and triangles.  Hence: one set of loads per unit for both kinds (a
+// warp used to wait for its node lanes, its triangle lanes and its full tests
+// one after another; 50 M walks of the 327,680-triangle noise sphere, mixed:
+// 201 -> 184 ms); every piece of the loop emitted once -- query set-up, grid
+// lookup, candidate test -- because the FP64 kernel stalled on instruction
+// fetch with two copies of them (1.02 M walks, 81,920 triangles: 47 -> 38
+// ms); and few stack entries in shared memory, which leaves it to the L1
+// (FP64 52 -> 47 ms, mixed 204 -> 201).
 // Residency: the FP32 form with the centre-point source fits 64 registers, so
 // 1024 threads (8 blocks of 128) stay resident per SM; the others take up to
-// 80 (768 threads, 6 blocks of 128).
+// 80 (768 threads, 6 blocks of 128; the FP64 form with 64: 50 ms for 47).
 template <typename T, int MODE, int SRC>
 constexpr int wos_min_blocks(int block) {
   return sizeof(T) == 4 && SRC == TWOS_SOURCE_CENTER && MODE != kModeGradient ? 1024 / block
@@ -675,7 +976,7 @@ constexpr int wos_min_blocks(int block) {
 }
 
 // Walks a lane claims from the work queue at once.
-__device__ __forceinline__ uint32_t lane_walks_of(const WosLaunch &L) {
+__host__ __device__ __forceinline__ uint32_t lane_walks_of(const WosLaunch &L) {
   return L.lane_walks > 1 ? static_cast<uint32_t>(L.lane_walks) : 1u;
 }
 
@@ -690,7 +991,8 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
   // column-major so a warp's accesses hit distinct banks), then the tables.
   extern __shared__ __align__(16) unsigned char s_dyn[];
   uint2 *s_stack = reinterpret_cast<uint2 *>(s_dyn);
-  unsigned char *s_tab = s_dyn + kStack * BLOCK * sizeof(uint2);
+  unsigned char *s_cold = s_dyn + wos_stack_entries<T>() * BLOCK * sizeof(uint2);
+  unsigned char *s_tab = s_cold + wos_cold_bytes<T>(GRAD) * BLOCK;
   const SmemPlan plan = smem_plan<T>(L.n_jobs, L.n_geos, L.n_terms);
   const JobDesc *s_jobs = plan.tables ? reinterpret_cast<const JobDesc *>(s_tab) : L.jobs;
   const GeoDesc *s_geos = plan.tables ? reinterpret_cast<const GeoDesc *>(s_tab + plan.geo_offset) : L.geos;
@@ -720,7 +1022,17 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
 
   const unsigned lane = threadIdx.x & 31u;
   const unsigned full = 0xffffffffu;
+  const bool on = static_cast<int>(lane) < L.lanes;  // lanes that take walks
+  const unsigned on_mask = __ballot_sync(full, on);
   uint2 *stack = s_stack + threadIdx.x;
+  uint2 deep[kStack - kShared];
+  auto push = [&](int &sp, uint2 e) {
+    if (sp < kShared)
+      stack[sp * BLOCK] = e;
+    else
+      deep[sp - kShared] = e;
+    ++sp;
+  };
   uint32_t err = 0;
   // Per-thread traversal counters (32-bit: a thread's share of one launch
   // stays far below 2^32), summed in 64 bits at the end.
@@ -730,22 +1042,57 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
   bool exhausted = false;  // warp-uniform
   const int units = L.units > 0 ? L.units : 1;
   // Walk state.
-  uint64_t wid = 0;
-  uint32_t job = 0, site = 0, walk = 0, steps = 0;
-  Vec<T> pos{T(0), T(0), T(0)};
-  T u = T(0), pv = T(0);
-  // Gradient mode: first-ball radius, direction and payoff increments, and
+  constexpr bool COLD = sizeof(T) == 8;
+  auto cell = [&](auto &c, int word) {  // 8-byte words of the thread's column
+    if constexpr (COLD)
+      c.p = reinterpret_cast<decltype(c.p)>(s_cold + (word * BLOCK + threadIdx.x) * 8);
+    else
+      c.v = 0;
+  };
+  auto half = [&](auto &c, int word, int h) {  // 4-byte halves of a word, in separate rows
+    if constexpr (COLD)
+      c.p = reinterpret_cast<decltype(c.p)>(s_cold + word * BLOCK * 8 + (h * BLOCK + threadIdx.x) * 4);
+    else
+      c.v = 0;
+  };
+  uint32_t job = 0;
+  Cell<T, COLD> px, py, pz, u, pv, best2;
+  Cell<uint64_t, COLD> wid;
+  Cell<uint32_t, COLD> site, walk, steps, best_tri;  // best_tri: leaf-order index of the walk's nearest triangle
+  cell(px, 0);
+  cell(py, 1);
+  cell(pz, 2);
+  cell(u, 3);
+  cell(pv, 4);
+  cell(best2, 5);
+  cell(wid, 6);
+  half(site, 7, 0);
+  half(walk, 7, 1);
+  half(steps, 8, 0);
+  half(best_tri, 8, 1);
+  // Gradient mode: first-ball radius, payoff increments and direction, and
   // the ball source terms of grad U / grad P.
-  T g_r0 = T(0), g_u0 = T(0), g_p0 = T(0);
-  Vec<T> g_w0{T(0), T(0), T(0)}, g_su{T(0), T(0), T(0)}, g_sp{T(0), T(0), T(0)};
-  // Query state.
-  T best2 = T(0);
+  Cell<T, COLD> g_r0, g_u0, g_p0, g_w0[3], g_su[3], g_sp[3];
+  if constexpr (GRAD) {
+    cell(g_r0, 9);
+    cell(g_u0, 10);
+    cell(g_p0, 11);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      cell(g_w0[k], 12 + k);
+      cell(g_su[k], 15 + k);
+      cell(g_sp[k], 18 + k);
+    }
+  }
+  // Query state.  The FP64 form prunes in FP32 (cull.p, cull.limit); the
+  // mixed form's position and best2 are FP32 themselves.
+  Cull cull{{0.f, 0.f, 0.f}, 0.f, 0.f, 0};
   int node = 0, sp = 0;
   bool have = false, found = false;
   // Four-wide form: this query continues on the binary BVH (set when a
   // four-wide visit would overflow the stack).
   bool narrow = false;
-  uint32_t best_tri = 0;  // leaf-order index of the nearest triangle found for this walk
+  bool resume = false;  // FP64 form: back to the traversal after the candidates' test
   bool tri_ok = false;    // best_tri belongs to this walk
   uint32_t tri_cur = 0, tri_end = 0, iter = 0;
   // CLAIM: walks a lane claims from the queue at once, run one after
@@ -755,6 +1102,88 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
   __shared__ uint32_t s_claim[CLAIM ? BLOCK : 1];
   if (CLAIM) s_claim[threadIdx.x] = 0u;
 
+  // Squared bound that prunes a subtree.
+  auto prune_limit = [&]() -> float {
+    if constexpr (sizeof(T) == 4)
+      return best2;
+    else
+      return cull.limit;
+  };
+  auto set_best2 = [&](T v) { best2 = v; };
+  // FP64 form: the held candidates' FP64 test.
+  auto flush = [&](const GeoDesc &G, const Vec<T> &pos) {
+    if constexpr (sizeof(T) == 8) {
+      if (cull.count == 0) return;
+      double b2 = best2;
+      uint32_t tri = best_tri;
+      if (cull_flush(G, pos, cull, b2, tri, stack + kShared * BLOCK, BLOCK)) {
+        best2 = b2;
+        best_tri = tri;
+        found = tri_ok = true;
+      }
+    }
+  };
+  // The grid's bounds and entry node at pos.
+  auto walk_grid = [&](const GeoDesc &G, const Vec<T> &pos, float &bound, float &upper, int &entry_node) {
+    if (!G.grid) return false;
+    if constexpr (sizeof(T) == 4) {
+      return grid_bounds(G, pos, bound, upper, entry_node);
+    } else {
+      const double p3[3] = {pos.x, pos.y, pos.z};
+      return grid_bounds(G, to_frame<float>(p3, G), bound, upper, entry_node);
+    }
+  };
+  // Starts the query at pos; `in_grid`: with the grid's upper bound and entry
+  // node there.
+  auto begin_query = [&](const JobDesc &J, const GeoDesc &G, const Vec<T> &pos, bool in_grid, float upper,
+                         int entry_node) {
+    T best2 = static_cast<T>(J.query_radius2);
+    found = false;
+    node = 0;
+    // Entry node: with an initial bound b below one entry cell, every triangle
+    // outside the cell's entry subtree is farther than b (the table keeps every
+    // triangle within a cell size plus 4 delta), so the traversal starts there.
+    // The grid's upper bound plus 6 delta (its 3 delta and the query's own
+    // error, with room) serves as b before any triangle is found.  (The
+    // four-wide form starts at its root: the table holds binary nodes.)
+    if constexpr (sizeof(T) == 8) {
+      if (!cull_begin(G, pos, best2, cull)) {
+        const Plain64 r = nearest_plain64(&G, pos.x, pos.y, pos.z, best2);
+        err |= r.flags & 0x7fffffffu;
+        found = tri_ok = r.flags >> 31;
+        set_best2(r.best2);
+        best_tri = r.tri;
+        phase = kStep;
+        return;
+      }
+    }
+    if (in_grid) {
+      const float ubs = __fmaf_ru(6.f, G.delta, upper);
+      if (!WIDE && entry_node >= 0 && ubs < G.entry_radius) node = entry_node;
+      if constexpr (sizeof(T) == 4) {
+        best2 = fminf(best2, ubs * ubs);
+      } else {
+        const float reach = __fadd_ru(ubs, cull.margin);
+        cull.limit = fminf(cull.limit, __fmul_ru(reach, reach));
+      }
+    }
+    set_best2(best2);
+    sp = 0;
+    have = true;
+    narrow = false;
+    // Warm start: the walk's previous nearest triangle is tested first, so
+    // the search prunes with its distance from the first node on.  (In the
+    // FP64 form the grid's bound prunes as well: 38.0 against 39.3 ms with
+    // both on 1.02 M walks of the 81,920-triangle noise sphere.)
+    tri_cur = tri_end = 0;
+    if (L.warm && tri_ok && (sizeof(T) == 4 || !in_grid)) {
+      tri_cur = best_tri;
+      tri_end = tri_cur + 1;
+    }
+    iter = 0;
+    phase = kTraverse;
+  };
+
   for (;;) {
     // Starts walk `wid` on this lane (its first radius from the per-site
     // pre-pass when there is one).
@@ -763,17 +1192,22 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
       job = find_job(s_jobs, L.n_jobs, id);
       const JobDesc &J = s_jobs[job];
       const uint64_t local = id - J.walk_begin;
-      site = static_cast<uint32_t>(local / J.walks);
-      walk = static_cast<uint32_t>(local - static_cast<uint64_t>(site) * J.walks);
+      const uint32_t at = static_cast<uint32_t>(local / J.walks);
+      site = at;
+      walk = static_cast<uint32_t>(local - static_cast<uint64_t>(at) * J.walks);
       const GeoDesc &G = s_geos[J.geo];
       bool skip = false;
+      Vec<T> pos;
       if (L.walk_start) {
-        const double *st = L.walk_start + 3ull * wid;
+        const double *st = L.walk_start + 3ull * id;
         skip = isnan(st[0]);
         pos = to_frame<T>(st, G);
       } else {
-        pos = to_frame<T>(L.sites + 3ull * (J.site_begin + site), G);
+        pos = to_frame<T>(L.sites + 3ull * (J.site_begin + at), G);
       }
+      px = pos.x;
+      py = pos.y;
+      pz = pos.z;
       u = T(0);
       pv = T(0);
       steps = 0;
@@ -788,39 +1222,31 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
         }
       }
       if (skip) {
-        if (MODE != kModeBoundary) static_cast<T *>(L.u_out)[wid] = T(0);
-        if (PAIRED) static_cast<T *>(L.p_out)[wid] = T(0);
+        if (MODE != kModeBoundary) static_cast<T *>(L.u_out)[id] = T(0);
+        if (PAIRED) static_cast<T *>(L.p_out)[id] = T(0);
         if (GRAD)
-          for (int k = 0; k < 6; ++k) static_cast<T *>(L.grad_out)[6ull * wid + k] = T(0);
-        if (MODE == kModeBoundary) L.hits[wid].cavity = -2;
-        L.steps_out[wid] = 0u;
+          for (int k = 0; k < 6; ++k) static_cast<T *>(L.grad_out)[6ull * id + k] = T(0);
+        if (MODE == kModeBoundary) L.hits[id].cavity = -2;
+        L.steps_out[id] = 0u;
       } else if (L.site_best2 && MODE != kModeBoundary) {
         // First query answered by the per-site pre-pass.
-        best2 = static_cast<const T *>(L.site_best2)[J.site_rank + site];
+        best2 = static_cast<const T *>(L.site_best2)[J.site_rank + at];
         found = best2 >= T(0);
         phase = kStep;
       } else {
-        best2 = static_cast<T>(J.query_radius2);
-        node = 0;
-        sp = 0;
-        have = true;
-        narrow = false;
-        found = false;
-        tri_cur = tri_end = 0;
-        iter = 0;
-        phase = kTraverse;
+        phase = kBegin;
       }
     };
 
     // ---- refill idle lanes from the work queue (CLAIM: from their own
     // claims first)
-    const unsigned idle = __ballot_sync(full, phase == kIdle);
+    const unsigned idle = __ballot_sync(full, on && phase == kIdle);
     if constexpr (CLAIM) {
       if (idle != 0u) {
         const unsigned pending = __ballot_sync(full, s_claim[threadIdx.x] != 0u);
-        if ((!exhausted || pending != 0u) && (__popc(idle) >= L.refill || idle == full)) {
+        if ((!exhausted || pending != 0u) && (__popc(idle) >= L.refill || idle == on_mask)) {
           uint32_t claim_left = s_claim[threadIdx.x];
-          const unsigned claim = __ballot_sync(full, phase == kIdle && claim_left == 0u);
+          const unsigned claim = __ballot_sync(full, on && phase == kIdle && claim_left == 0u);
           if (!exhausted && claim != 0u) {
             const uint64_t span = static_cast<uint64_t>(lane_walks_of(L)) * __popc(claim);
             unsigned long long base = 0;
@@ -828,7 +1254,7 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
             if (static_cast<int>(lane) == leader) base = atomicAdd(L.counter, static_cast<unsigned long long>(span));
             base = __shfl_sync(full, base, leader);
             if (base + span >= L.total_walks) exhausted = true;
-            if (phase == kIdle && claim_left == 0u) {
+            if (on && phase == kIdle && claim_left == 0u) {
               const uint64_t first =
                   base + static_cast<uint64_t>(lane_walks_of(L)) * __popc(claim & ((1u << lane) - 1u));
               if (first < L.total_walks) {
@@ -839,21 +1265,21 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
             }
           }
           if (phase == kIdle && claim_left != 0u) {
-            ++wid;
+            wid = wid + 1;
             --claim_left;
             start_walk();
           }
           s_claim[threadIdx.x] = claim_left;
         }
       }
-    } else if (!exhausted && idle != 0u && (__popc(idle) >= L.refill || idle == full)) {
+    } else if (!exhausted && idle != 0u && (__popc(idle) >= L.refill || idle == on_mask)) {
       unsigned long long base = 0;
       const int leader = __ffs(idle) - 1;
       if (static_cast<int>(lane) == leader)
         base = atomicAdd(L.counter, static_cast<unsigned long long>(__popc(idle)));
       base = __shfl_sync(full, base, leader);
       if (base + __popc(idle) >= L.total_walks) exhausted = true;
-      if (phase == kIdle) {
+      if (on && phase == kIdle) {
         const uint64_t id = base + __popc(idle & ((1u << lane) - 1u));
         if (id < L.total_walks) {
           wid = id;
@@ -863,180 +1289,205 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
     }
 
     // ---- batched walk step for lanes whose query has finished
-    const unsigned ready = __ballot_sync(full, phase == kStep);
+    const unsigned ready = __ballot_sync(full, phase >= kStep);
     const unsigned trav = __ballot_sync(full, phase == kTraverse);
-    if (ready != 0u && (__popc(ready) >= L.step_threshold || trav == 0u) && phase == kStep) {
+    if (ready != 0u && (__popc(ready) >= L.step_threshold || trav == 0u) && phase >= kStep) {
       const JobDesc &J = s_jobs[job];
       const GeoDesc &G = s_geos[J.geo];
       // One pass; `break` leaves it once the lane's next phase is set.
       do {
-        T d = sqrt(best2);
-        if (!found) {
-          err |= TWOS_DEVERR_QUERY;
-          d = T(0);  // ends the walk; the call reports the failure
-        }
-        const T R = to_T<T>(J.cavity_radius);
-        const T dmesh = d;
-        int hit_cav = -1;
-        bool cav_nearer = false;  // gradient mode: the exit is on a cavity
-        for (uint32_t c = 0; c < J.n_cav; ++c) {
-          const Vec<T> cc = to_frame<T>(L.cavities + 3ull * (J.cav_begin + c), G);
-          const Vec<T> dv = sub(pos, cc);
-          const T len = sqrt(dot3(dv, dv));
-          const T dc = len - R;
-          if (MODE == kModeBoundary) {
-            // closest_boundary (wih_twos.cpp:612-624): the first strictly nearer cavity.
-            if (dc < d && len > T(0)) {
-              d = dc;
-              hit_cav = static_cast<int>(c);
-            }
-          } else {
-            d = dc < d ? dc : d;
-            if (GRAD && dc < dmesh) cav_nearer = true;
+        Vec<T> pos{px, py, pz};
+        if (phase == kStep) {
+          flush(G, pos);
+          if (resume) {
+            // Only the full candidate list was due; the search goes on.
+            resume = false;
+            phase = kTraverse;
+            break;
           }
-        }
-        // The mixed form shrinks the radius by the FP32 distance error bound;
-        // the FP64 form uses the distance itself (wih_twos.cpp:645-647).
-        const T r = sizeof(T) == 4 ? d - static_cast<T>(G.delta) : d;
-        bool done = !(r > to_T<T>(J.epsilon));
-        bool cap = false;
-        if (!done) {
-          const uint32_t ctr3 = J.repeat << 3;
-          const Philox4 q0 = philox(J.k0, J.k1, steps, walk, J.site_offset + site, ctr3 | 0u);
-          Vec<T> a = pos;
-          if (GREEN) {
-            const Philox4 q1 = philox(J.k0, J.k1, steps, walk, J.site_offset + site, ctr3 | 1u);
-            const Philox4 q2 = philox(J.k0, J.k1, steps, walk, J.site_offset + site, ctr3 | 2u);
-            const Philox4 q3 = philox(J.k0, J.k1, steps, walk, J.site_offset + site, ctr3 | 3u);
-            const T beta = median3(uniform<T>(q2.x, q2.y), uniform<T>(q2.z, q2.w), uniform<T>(q3.x, q3.y));
-            const Vec<T> g = direction<T>(uniform<T>(q1.x, q1.y), uniform<T>(q1.z, q1.w));
-            a = add_scaled(pos, g, r * beta);
+          T d = sqrt(static_cast<T>(best2));
+          if (!found) {
+            err |= TWOS_DEVERR_QUERY;
+            d = T(0);  // ends the walk; the call reports the failure
           }
-          if (EXACT) {
-            u = exact_source(u, s_terms, J.src_begin, J.n_src, pos, r, err);
-            if (PAIRED) pv = exact_source(pv, s_terms, J.adj_begin, J.n_adj, pos, r, err);
-          } else {
-            const T w = r * r / T(6);
-            if (MODE != kModeBoundary) {
-              const T du = w * source_value(s_terms, J.src_begin, J.n_src, a);
-              u = u + du;
-              if (GRAD && steps == 0) g_u0 = du;
-            }
-            if (PAIRED) {
-              const T dp = w * source_value(s_terms, J.adj_begin, J.n_adj, a);
-              pv = pv + dp;
-              if (GRAD && steps == 0) g_p0 = dp;
-            }
-          }
-          const Vec<T> dir = direction<T>(uniform<T>(q0.x, q0.y), uniform<T>(q0.z, q0.w));
-          if (GRAD && steps == 0) {
-            // First ball: the sphere term's radius and direction, and one draw
-            // (blocks 4-5) for the ball source term of the gradient,
-            // R (1 - t^3) f(x + t R w') w' with t ~ U(0,1), w' uniform.
-            const Philox4 q4 = philox(J.k0, J.k1, 0u, walk, J.site_offset + site, ctr3 | 4u);
-            const Philox4 q5 = philox(J.k0, J.k1, 0u, walk, J.site_offset + site, ctr3 | 5u);
-            const T t = uniform<T>(q4.x, q4.y);
-            const Vec<T> wp = direction<T>(uniform<T>(q4.z, q4.w), uniform<T>(q5.x, q5.y));
-            const Vec<T> z = add_scaled(pos, wp, t * r);
-            const T wt = r * (T(1) - t * t * t);
-            const T fs = wt * source_value(s_terms, J.src_begin, J.n_src, z);
-            const T fq = wt * source_value(s_terms, J.adj_begin, J.n_adj, z);
-            g_su = {wp.x * fs, wp.y * fs, wp.z * fs};
-            g_sp = {wp.x * fq, wp.y * fq, wp.z * fq};
-            g_r0 = r;
-            g_w0 = dir;
-          }
-          pos = add_scaled(pos, dir, r);
-          ++steps;
-          if (static_cast<int>(steps) >= J.max_steps) {
-            done = true;
-            cap = true;
-          }
-        }
-        if (done) {
-          if (MODE == kModeBoundary) {
-            HitRec h;
-            h.pad = 0;
-            Vec<T> q{T(0), T(0), T(0)}, nrm{T(0), T(0), T(0)};
-            if (cap || !found) {
-              h.cavity = -2;
-            } else if (hit_cav >= 0) {
-              // Point on the sphere along the radial direction; the domain
-              // excludes the sphere, so the outward normal points into it.
-              const Vec<T> cc = to_frame<T>(L.cavities + 3ull * (J.cav_begin + hit_cav), G);
-              const Vec<T> dv = sub(pos, cc);
-              const T inv = T(1) / sqrt(dot3(dv, dv));
-              const Vec<T> dir{dv.x * inv, dv.y * inv, dv.z * inv};
-              q = add_scaled(cc, dir, R);
-              nrm = {dir.x * T(-1), dir.y * T(-1), dir.z * T(-1)};
-              h.cavity = hit_cav;
+          const T R = to_T<T>(J.cavity_radius);
+          const T dmesh = d;
+          int hit_cav = -1;
+          bool cav_nearer = false;  // gradient mode: the exit is on a cavity
+          for (uint32_t c = 0; c < J.n_cav; ++c) {
+            const Vec<T> cc = to_frame<T>(L.cavities + 3ull * (J.cav_begin + c), G);
+            const Vec<T> dv = sub(pos, cc);
+            const T len = sqrt(dot3(dv, dv));
+            const T dc = len - R;
+            if (MODE == kModeBoundary) {
+              // closest_boundary (wih_twos.cpp:612-624): the first strictly nearer cavity.
+              if (dc < d && len > T(0)) {
+                d = dc;
+                hit_cav = static_cast<int>(c);
+              }
             } else {
-              Vec<T> ta, tb, tc;
-              load_tri(geo_tris<T>(G), best_tri, ta, tb, tc);
-              q = tri_closest(pos, ta, tb, tc);
-              if (dmesh > T(0)) {
-                const T inv = T(1) / dmesh;
-                const Vec<T> dq = sub(q, pos);
-                nrm = {dq.x * inv, dq.y * inv, dq.z * inv};
-              }
-              h.cavity = -1;
+              d = dc < d ? dc : d;
+              if (GRAD && dc < dmesh) cav_nearer = true;
             }
-            const bool f32 = sizeof(T) == 4;
-            h.point[0] = static_cast<double>(q.x) + (f32 ? G.center[0] : 0.0);
-            h.point[1] = static_cast<double>(q.y) + (f32 ? G.center[1] : 0.0);
-            h.point[2] = static_cast<double>(q.z) + (f32 ? G.center[2] : 0.0);
-            h.normal[0] = static_cast<double>(nrm.x);
-            h.normal[1] = static_cast<double>(nrm.y);
-            h.normal[2] = static_cast<double>(nrm.z);
-            L.hits[wid] = h;
-          } else {
-            if (GRAD) {
-              // Dirichlet data of u at the exit point on the mesh.
-              if (!cap && found && J.n_bnd > 0 && !cav_nearer) {
-                Vec<T> q = pos;
-                if (tri_ok) {
-                  Vec<T> ta, tb, tc;
-                  load_tri(geo_tris<T>(G), best_tri, ta, tb, tc);
-                  q = tri_closest(pos, ta, tb, tc);
-                }
-                u = u + source_value(s_terms, J.bnd_begin, J.n_bnd, q);
-              }
-              T *go = static_cast<T *>(L.grad_out) + 6ull * wid;
-              if (g_r0 > T(0)) {
-                const T k = T(3) / g_r0;
-                const T cu = k * (u - g_u0), cp = k * (pv - g_p0);
-                go[0] = g_w0.x * cu + g_su.x;
-                go[1] = g_w0.y * cu + g_su.y;
-                go[2] = g_w0.z * cu + g_su.z;
-                go[3] = g_w0.x * cp + g_sp.x;
-                go[4] = g_w0.y * cp + g_sp.y;
-                go[5] = g_w0.z * cp + g_sp.z;
-              } else {
-                for (int k = 0; k < 6; ++k) go[k] = T(0);
-              }
-            }
-            static_cast<T *>(L.u_out)[wid] = u;
           }
-          if (PAIRED) static_cast<T *>(L.p_out)[wid] = pv;
-          L.steps_out[wid] = steps | (cap ? 0x80000000u : 0u);
-          phase = kIdle;
-          break;
+          // The mixed form shrinks the radius by the FP32 distance error bound;
+          // the FP64 form uses the distance itself (wih_twos.cpp:645-647).
+          const T r = sizeof(T) == 4 ? d - static_cast<T>(G.delta) : d;
+          bool done = !(r > to_T<T>(J.epsilon));
+          bool cap = false;
+          if (!done) {
+            const uint32_t ctr3 = J.repeat << 3;
+            const uint32_t step = steps, wk = walk, key = J.site_offset + site;
+            const Philox4 q0 = philox(J.k0, J.k1, step, wk, key, ctr3 | 0u);
+            Vec<T> a = pos;
+            if (GREEN) {
+              const Philox4 q1 = philox(J.k0, J.k1, step, wk, key, ctr3 | 1u);
+              const Philox4 q2 = philox(J.k0, J.k1, step, wk, key, ctr3 | 2u);
+              const Philox4 q3 = philox(J.k0, J.k1, step, wk, key, ctr3 | 3u);
+              const T beta = median3(uniform<T>(q2.x, q2.y), uniform<T>(q2.z, q2.w), uniform<T>(q3.x, q3.y));
+              const Vec<T> g = direction<T>(uniform<T>(q1.x, q1.y), uniform<T>(q1.z, q1.w));
+              a = add_scaled(pos, g, r * beta);
+            }
+            if (EXACT) {
+              u = exact_source(static_cast<T>(u), s_terms, J.src_begin, J.n_src, pos, r, err);
+              if (PAIRED) pv = exact_source(static_cast<T>(pv), s_terms, J.adj_begin, J.n_adj, pos, r, err);
+            } else {
+              const T w = r * r / T(6);
+              if (MODE != kModeBoundary) {
+                const T du = w * source_value(s_terms, J.src_begin, J.n_src, a);
+                u = u + du;
+                if (GRAD && step == 0) g_u0 = du;
+              }
+              if (PAIRED) {
+                const T dp = w * source_value(s_terms, J.adj_begin, J.n_adj, a);
+                pv = pv + dp;
+                if (GRAD && step == 0) g_p0 = dp;
+              }
+            }
+            const Vec<T> dir = direction<T>(uniform<T>(q0.x, q0.y), uniform<T>(q0.z, q0.w));
+            if (GRAD && step == 0) {
+              // First ball: the sphere term's radius and direction, and one draw
+              // (blocks 4-5) for the ball source term of the gradient,
+              // R (1 - t^3) f(x + t R w') w' with t ~ U(0,1), w' uniform.
+              const Philox4 q4 = philox(J.k0, J.k1, 0u, wk, key, ctr3 | 4u);
+              const Philox4 q5 = philox(J.k0, J.k1, 0u, wk, key, ctr3 | 5u);
+              const T t = uniform<T>(q4.x, q4.y);
+              const Vec<T> wp = direction<T>(uniform<T>(q4.z, q4.w), uniform<T>(q5.x, q5.y));
+              const Vec<T> z = add_scaled(pos, wp, t * r);
+              const T wt = r * (T(1) - t * t * t);
+              const T fs = wt * source_value(s_terms, J.src_begin, J.n_src, z);
+              const T fq = wt * source_value(s_terms, J.adj_begin, J.n_adj, z);
+              g_su[0] = wp.x * fs;
+              g_su[1] = wp.y * fs;
+              g_su[2] = wp.z * fs;
+              g_sp[0] = wp.x * fq;
+              g_sp[1] = wp.y * fq;
+              g_sp[2] = wp.z * fq;
+              g_r0 = r;
+              g_w0[0] = dir.x;
+              g_w0[1] = dir.y;
+              g_w0[2] = dir.z;
+            }
+            pos = add_scaled(pos, dir, r);
+            px = pos.x;
+            py = pos.y;
+            pz = pos.z;
+            steps = step + 1;
+            if (static_cast<int>(step + 1) >= J.max_steps) {
+              done = true;
+              cap = true;
+            }
+          }
+          if (done) {
+            if (MODE == kModeBoundary) {
+              HitRec h;
+              h.pad = 0;
+              Vec<T> q{T(0), T(0), T(0)}, nrm{T(0), T(0), T(0)};
+              if (cap || !found) {
+                h.cavity = -2;
+              } else if (hit_cav >= 0) {
+                // Point on the sphere along the radial direction; the domain
+                // excludes the sphere, so the outward normal points into it.
+                const Vec<T> cc = to_frame<T>(L.cavities + 3ull * (J.cav_begin + hit_cav), G);
+                const Vec<T> dv = sub(pos, cc);
+                const T inv = T(1) / sqrt(dot3(dv, dv));
+                const Vec<T> dir{dv.x * inv, dv.y * inv, dv.z * inv};
+                q = add_scaled(cc, dir, R);
+                nrm = {dir.x * T(-1), dir.y * T(-1), dir.z * T(-1)};
+                h.cavity = hit_cav;
+              } else {
+                Vec<T> ta, tb, tc;
+                load_tri(geo_tris<T>(G), best_tri, ta, tb, tc);
+                q = tri_closest(pos, ta, tb, tc);
+                if (dmesh > T(0)) {
+                  const T inv = T(1) / dmesh;
+                  const Vec<T> dq = sub(q, pos);
+                  nrm = {dq.x * inv, dq.y * inv, dq.z * inv};
+                }
+                h.cavity = -1;
+              }
+              const bool f32 = sizeof(T) == 4;
+              h.point[0] = static_cast<double>(q.x) + (f32 ? G.center[0] : 0.0);
+              h.point[1] = static_cast<double>(q.y) + (f32 ? G.center[1] : 0.0);
+              h.point[2] = static_cast<double>(q.z) + (f32 ? G.center[2] : 0.0);
+              h.normal[0] = static_cast<double>(nrm.x);
+              h.normal[1] = static_cast<double>(nrm.y);
+              h.normal[2] = static_cast<double>(nrm.z);
+              L.hits[wid] = h;
+            } else {
+              if (GRAD) {
+                // Dirichlet data of u at the exit point on the mesh.
+                if (!cap && found && J.n_bnd > 0 && !cav_nearer) {
+                  Vec<T> q = pos;
+                  if (tri_ok) {
+                    Vec<T> ta, tb, tc;
+                    load_tri(geo_tris<T>(G), best_tri, ta, tb, tc);
+                    q = tri_closest(pos, ta, tb, tc);
+                  }
+                  u = u + source_value(s_terms, J.bnd_begin, J.n_bnd, q);
+                }
+                T *go = static_cast<T *>(L.grad_out) + 6ull * wid;
+                const T r0 = g_r0;
+                if (r0 > T(0)) {
+                  const T k = T(3) / r0;
+                  const T cu = k * (u - g_u0), cp = k * (pv - g_p0);
+#pragma unroll
+                  for (int a = 0; a < 3; ++a) {
+                    go[a] = g_w0[a] * cu + g_su[a];
+                    go[3 + a] = g_w0[a] * cp + g_sp[a];
+                  }
+                } else {
+                  for (int k = 0; k < 6; ++k) go[k] = T(0);
+                }
+              }
+              static_cast<T *>(L.u_out)[wid] = u;
+            }
+            if (PAIRED) static_cast<T *>(L.p_out)[wid] = pv;
+            L.steps_out[wid] = steps | (cap ? 0x80000000u : 0u);
+            phase = kIdle;
+            break;
+          }
         }
-        best2 = static_cast<T>(J.query_radius2);
-        found = false;
-        node = 0;
-        if constexpr (sizeof(T) == 4) {
-          // Distance-bound grid: D(v) - |x - v| over the corners v of x's cell
-          // bounds the mesh distance from below; a bound of at least grid_tau
-          // spacings is the next ball's radius and no query is needed.  A grid
-          // step never ends a walk: the bound must clear the termination
-          // shell with room to spare.
-          float bound, upper = CUDART_INF_F;
-          int entry_node = -1;
-          const bool in_grid = (L.grid_tau > 0.f || L.entry) && G.grid && grid_bounds(G, pos, bound, upper, entry_node);
+        // Distance-bound grid: D(v) - |x - v| over the corners v of x's cell
+        // bounds the mesh distance from below; a bound of at least grid_tau
+        // spacings is the next ball's radius and no query is needed.  A grid
+        // step never ends a walk: the bound must clear the termination shell
+        // with room to spare.  The FP64 form takes no grid steps (with GRID64
+        // it does, a comparison of precision alone); its queries only start
+        // from the grid's upper bound and entry node.  It evaluates the grid
+        // at the FP32 image of the position, within a few 1e-8 of it, and
+        // bound <= d - delta covers that.
+        float bound = 0.f, upper = CUDART_INF_F;
+        int entry_node = -1;
+        bool in_grid = false;
+        if (L.entry || ((sizeof(T) == 4 || GRID64) && L.grid_tau > 0.f))
+          in_grid = walk_grid(G, pos, bound, upper, entry_node);
+        if constexpr (sizeof(T) == 4 || GRID64) {
+          const T b = static_cast<T>(bound);
           if (in_grid && L.grid_tau > 0.f && bound >= L.grid_tau * G.grid_h &&
-              bound > 2.f * (static_cast<float>(J.epsilon) + G.delta) && bound * bound < best2) {
-            best2 = bound * bound;
+              bound > 2.f * (static_cast<float>(J.epsilon) + G.delta) && b * b < static_cast<T>(J.query_radius2) &&
+              phase == kStep) {
+            best2 = b * b;
             found = true;
             ++c_grid;
             if constexpr (TRACE) {
@@ -1046,78 +1497,8 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
             // The step itself comes with the warp's next batch.
             break;
           }
-          if (!(in_grid && L.entry)) entry_node = -1;
-          if (L.warm && tri_ok) {
-            Vec<T> ta, tb, tc;
-            load_tri(geo_tris<T>(G), best_tri, ta, tb, tc);
-            ++c_tris;
-            const T w2 = tri_dist2(pos, ta, tb, tc);
-            if (w2 < best2) {
-              best2 = w2;
-              found = true;
-            }
-          }
-          // Entry node: with an initial bound b below one entry cell, every
-          // triangle outside the cell's entry subtree is farther than b (the
-          // table keeps every triangle within a cell size plus 4 delta), so
-          // the traversal starts there.  The grid's upper bound plus 6 delta
-          // (its 3 delta and the FP32 query's delta, with room) may serve as
-          // b before any triangle is found.  (The four-wide form keeps the
-          // bound but starts at its root: the table holds binary nodes.)
-          if (entry_node >= 0) {
-            const float ubs = upper + 6.f * G.delta;
-            if (fminf(sqrtf(best2), ubs) < G.entry_radius) {
-              if (!WIDE) node = entry_node;
-              if (ubs * ubs < best2) best2 = ubs * ubs;
-            }
-          }
-        } else {
-          // FP64 form.  With GRID64 it takes the same grid steps and entry
-          // nodes as the mixed form (a comparison of precision alone): the
-          // bound is evaluated at the FP32 image p32 of the position, within
-          // a few 1e-8 of it, and bound <= d(p32) - delta covers that.
-          float bound = 0.f, upper = CUDART_INF_F;
-          int entry_node = -1;
-          bool in_grid = false;
-          if constexpr (GRID64) {
-            const double p3[3] = {pos.x, pos.y, pos.z};
-            in_grid = L.grid_tau > 0.f && G.grid && grid_bounds(G, to_frame<float>(p3, G), bound, upper, entry_node);
-            const double b = static_cast<double>(bound);
-            if (in_grid && bound >= L.grid_tau * G.grid_h && bound > 2.f * (static_cast<float>(J.epsilon) + G.delta) &&
-                b * b < best2) {
-              best2 = b * b;
-              found = true;
-              ++c_grid;
-              break;
-            }
-          }
-          if (L.warm && tri_ok) {
-            Vec<T> ta, tb, tc;
-            load_tri(geo_tris<T>(G), best_tri, ta, tb, tc);
-            ++c_tris;
-            const T w2 = tri_dist2(pos, ta, tb, tc);
-            if (w2 < best2) {
-              best2 = w2;
-              found = true;
-            }
-          }
-          if constexpr (GRID64) {
-            if (in_grid && L.entry && entry_node >= 0) {
-              const double ubs = static_cast<double>(upper) + 6.0 * G.delta;
-              if (fmin(sqrt(best2), ubs) < static_cast<double>(G.entry_radius)) {
-                node = entry_node;
-                if (ubs * ubs < best2) best2 = ubs * ubs;
-              }
-            }
-          }
         }
-        sp = 0;
-        have = true;
-        narrow = false;
-        tri_cur = tri_end = 0;
-        iter = 0;
-        phase = kTraverse;
-        break;
+        begin_query(J, G, pos, in_grid && L.entry, upper, entry_node);
       } while (false);
     }
 
@@ -1140,117 +1521,139 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
     }
     if (take) {
       const GeoDesc &G = s_geos[s_jobs[job].geo];
+      const Vec<float> pos = [&]() -> Vec<float> {  // the FP32 query point
+        if constexpr (sizeof(T) == 4)
+          return {px, py, pz};
+        else
+          return cull.p;
+      }();
       // Up to `units` units back to back before the warp returns to the
       // refill and step ballots: the loop overhead is paid once per batch.
+      auto fail = [&](uint32_t bit) {
+        err |= bit;
+        found = false;
+        cull.count = 0;
+        resume = false;
+        phase = kStep;
+      };
 #pragma unroll 1
-      for (int unit = 0; unit < units && phase == kTraverse; ++unit) {
-        if (++iter > G.max_iter) {
-          err |= TWOS_DEVERR_ITER;
-          found = false;
-          phase = kStep;
-        } else if (tri_cur < tri_end) {
-          const typename Layout<T>::Tri *tris = geo_tris<T>(G);
-          ++c_planes;
-          if (tri_test(tris, tri_cur, pos, best2, c_tris)) {
-            found = true;
-            best_tri = tri_cur;
-            tri_ok = true;
-          }
-          ++tri_cur;
-        } else {
-          // Pop the next entry still closer than the current best.
+      for (int unit = 0; unit < units; ++unit) {
+        // The unit's triangle or node: the leaf at hand, else the current
+        // node or the next stack entry still closer than the current best.
+        if (tri_cur >= tri_end) {
           while (!have && sp > 0) {
             --sp;
-            const uint2 e = stack[sp * BLOCK];
-            if (static_cast<T>(__uint_as_float(e.y)) < best2) {
+            const uint2 e = sp < kShared ? stack[sp * BLOCK] : deep[sp - kShared];
+            if (__uint_as_float(e.y) < prune_limit()) {
               node = static_cast<int>(e.x);
               have = true;
             }
           }
           if (!have) {
             phase = kStep;
-          } else {
-            if constexpr (WIDE) {
-              if (node >= 0 && !narrow) {
-                // Four-wide node: its valid children sorted nearest first (a
-                // five-comparator network); the nearest is next, the others
-                // are pushed farthest first.
-                ++c_nodes;
-                float d[4];
-                int c[4];
-                node4_dist2(G.nodes4_f, node, pos, d, c);
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                  if (!(d[k] < best2)) d[k] = CUDART_INF_F;
-                order2(d[0], c[0], d[1], c[1]);
-                order2(d[2], c[2], d[3], c[3]);
-                order2(d[0], c[0], d[2], c[2]);
-                order2(d[1], c[1], d[3], c[3]);
-                order2(d[1], c[1], d[2], c[2]);
-                const int nv = (d[0] < CUDART_INF_F) + (d[1] < CUDART_INF_F) + (d[2] < CUDART_INF_F) +
-                               (d[3] < CUDART_INF_F);
-                if (nv == 0) {
-                  have = false;
-                } else if (sp + nv - 1 > kStack) {
-                  // Up to three pushes per level can outgrow the stack on a
-                  // root-started query with a loose bound.  The query goes
-                  // on from the binary root with the bound found so far
-                  // (one push per level there): every triangle nearer than
-                  // best2 is still reached.
-                  narrow = true;
-                  sp = 0;
-                  node = 0;
-                } else {
-                  if (nv > 3) stack[(sp++) * BLOCK] = make_uint2(static_cast<uint32_t>(c[3]), __float_as_uint(d[3]));
-                  if (nv > 2) stack[(sp++) * BLOCK] = make_uint2(static_cast<uint32_t>(c[2]), __float_as_uint(d[2]));
-                  if (nv > 1) stack[(sp++) * BLOCK] = make_uint2(static_cast<uint32_t>(c[1]), __float_as_uint(d[1]));
-                  node = c[0];
-                }
-              }
-            }
-            if (!WIDE || narrow) {
-              if (node >= 0) {
-                ++c_nodes;
-                T dl, dr;
-                int cl, cr;
-                node_dist2(geo_nodes<T>(G), node, pos, dl, dr, cl, cr);
-                const bool vl = dl < best2, vr = dr < best2;
-                if (vl && vr) {
-                  if (dr < dl) {
-                    const T td = dl;
-                    dl = dr;
-                    dr = td;
-                    const int tc = cl;
-                    cl = cr;
-                    cr = tc;
-                  }
-                  if (sp >= kStack) {
-                    err |= TWOS_DEVERR_STACK;
-                    found = false;
-                    phase = kStep;
-                  } else {
-                    stack[sp * BLOCK] = make_uint2(static_cast<uint32_t>(cr), __float_as_uint(lower_f(dr)));
-                    ++sp;
-                    node = cl;
-                  }
-                } else if (vl) {
-                  node = cl;
-                } else if (vr) {
-                  node = cr;
-                } else {
-                  have = false;
-                }
-              }
-            }
-            // A leaf reached by this unit's visit or pop: its triangle range
-            // is taken in the same unit, so the next unit tests a triangle.
-            if (have && node < 0 && phase == kTraverse) {
-              const uint32_t enc = ~static_cast<uint32_t>(node);
-              tri_cur = enc >> 3;
-              tri_end = tri_cur + (enc & 7u);
-              have = false;
-            }
+            break;
           }
+          if (node < 0) {
+            const uint32_t enc = ~static_cast<uint32_t>(node);
+            tri_cur = enc >> 3;
+            tri_end = tri_cur + (enc & 7u);
+            have = false;
+          }
+        }
+        if (++iter > G.max_iter) {
+          fail(TWOS_DEVERR_ITER);
+          break;
+        }
+        if constexpr (WIDE) {
+          if (tri_cur >= tri_end && have && !narrow) {
+            // Four-wide node: its valid children sorted nearest first (a
+            // five-comparator network); the nearest is next, the others are
+            // pushed farthest first.
+            ++c_nodes;
+            float d[4];
+            int c[4];
+            node4_dist2(G.nodes4_f, node, pos, d, c);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              if (!(d[k] < prune_limit())) d[k] = CUDART_INF_F;
+            order2(d[0], c[0], d[1], c[1]);
+            order2(d[2], c[2], d[3], c[3]);
+            order2(d[0], c[0], d[2], c[2]);
+            order2(d[1], c[1], d[3], c[3]);
+            order2(d[1], c[1], d[2], c[2]);
+            const int nv =
+                (d[0] < CUDART_INF_F) + (d[1] < CUDART_INF_F) + (d[2] < CUDART_INF_F) + (d[3] < CUDART_INF_F);
+            if (nv == 0) {
+              have = false;
+            } else if (sp + nv - 1 > kStack) {
+              // Up to three pushes per level can outgrow the stack on a
+              // root-started query with a loose bound.  The query goes on
+              // from the binary root with the bound found so far (one push
+              // per level there): every triangle nearer than best2 is still
+              // reached.
+              narrow = true;
+              sp = 0;
+              node = 0;
+            } else {
+              if (nv > 3) push(sp, make_uint2(static_cast<uint32_t>(c[3]), __float_as_uint(d[3])));
+              if (nv > 2) push(sp, make_uint2(static_cast<uint32_t>(c[2]), __float_as_uint(d[2])));
+              if (nv > 1) push(sp, make_uint2(static_cast<uint32_t>(c[1]), __float_as_uint(d[1])));
+              node = c[0];
+            }
+            continue;
+          }
+        }
+        // One set of loads for either kind (64 bytes of a triangle or 96 of a
+        // node): lanes on nodes and lanes on triangles wait for memory
+        // together, once per unit, before the warp splits on the arithmetic.
+        const bool on_tri = tri_cur < tri_end;
+        const char *at = on_tri ? reinterpret_cast<const char *>(G.tris_f + tri_cur)
+                                : reinterpret_cast<const char *>(G.nodes_f + node);
+        float4 r0, r1, r2, r3, r4{}, r5{};
+        ldg32(at, r0, r1);
+        ldg32(at + 32, r2, r3);
+        ldg32_if(!on_tri, at + 64, r4, r5);
+        if (on_tri) {
+          ++c_planes;
+          if constexpr (sizeof(T) == 4) {
+            if (plane_gap2(r0, r1, pos) < best2) {
+              ++c_tris;
+              const float d2 = tri_dist2(pos, Vec<float>{r1.x, r1.y, r1.z}, Vec<float>{r2.x, r2.y, r2.z},
+                                         Vec<float>{r3.x, r3.y, r3.z});
+              if (d2 < best2) {
+                best2 = d2;
+                found = true;
+                best_tri = tri_cur;
+                tri_ok = true;
+              }
+            }
+            ++tri_cur;
+          } else {
+            // A full candidate list is tested first; the triangle comes again.
+            if (cull_tri(tri_cur, r0, r1, r2, r3, cull, stack + kShared * BLOCK, BLOCK, c_tris)) {
+              resume = true;
+              phase = kStep;
+              break;
+            }
+            ++tri_cur;
+          }
+        } else {
+          ++c_nodes;
+          float dl, dr;
+          int cl, cr;
+          node_bounds(r0, r1, r2, r3, r4, r5, pos, dl, dr, cl, cr);
+          const float limit = prune_limit();
+          const bool vl = dl < limit, vr = dr < limit;
+          const bool swap = dr < dl;
+          if (vl && vr) {
+            if (sp >= kStack) {
+              fail(TWOS_DEVERR_STACK);
+              break;
+            }
+            push(sp, make_uint2(static_cast<uint32_t>(swap ? cl : cr), __float_as_uint(swap ? dl : dr)));
+          }
+          have = vl || vr;
+          node = vl && !(vr && swap) ? cl : cr;
         }
       }
     }
@@ -1279,7 +1682,7 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
 // distance, or -1 when no surface point lies within the query radius.
 template <typename T>
 __global__ void __launch_bounds__(kWosBlock) site_prepass_kernel(const WosLaunch L) {
-  __shared__ uint2 s_stack[kStack * kWosBlock];
+  __shared__ uint2 s_stack[(kStack + kCand) * kWosBlock];
   uint2 *stack = s_stack + threadIdx.x;
   uint32_t err = 0;
   T *out = static_cast<T *>(L.site_best2);
@@ -1297,7 +1700,7 @@ __global__ void __launch_bounds__(kWosBlock) site_prepass_kernel(const WosLaunch
     const Vec<T> p = to_frame<T>(L.sites + 3ull * (J.site_begin + (g - J.site_rank)), G);
     T best2 = static_cast<T>(J.query_radius2);
     uint32_t tri = 0;
-    const bool found = nearest<T>(geo_nodes<T>(G), geo_tris<T>(G), G.max_iter, p, best2, tri, stack, kWosBlock, err);
+    const bool found = nearest_geo(G, p, best2, tri, stack, kWosBlock, err);
     out[g] = found ? best2 : T(-1);
   }
   if (err) atomicOr(L.error, err);
@@ -1379,8 +1782,11 @@ static const void *select_wos(int precision, int mode, int src, int block, int g
   }
 }
 
-static uint32_t wos_dyn_smem(int precision, const WosLaunch &L, int block) {
-  const uint32_t stack = static_cast<uint32_t>(kStack * block * sizeof(uint2));
+static uint32_t wos_dyn_smem(int precision, int mode, const WosLaunch &L, int block) {
+  const int entries = precision == TWOS_PREC_MIXED ? wos_stack_entries<float>() : wos_stack_entries<double>();
+  const int cold = precision == TWOS_PREC_MIXED ? wos_cold_bytes<float>(mode == kModeGradient)
+                                                : wos_cold_bytes<double>(mode == kModeGradient);
+  const uint32_t stack = static_cast<uint32_t>((entries * sizeof(uint2) + cold) * block);
   return stack + (precision == TWOS_PREC_MIXED ? smem_plan<float>(L.n_jobs, L.n_geos, L.n_terms).bytes
                                                : smem_plan<double>(L.n_jobs, L.n_geos, L.n_terms).bytes);
 }
@@ -1390,12 +1796,13 @@ static uint32_t wos_dyn_smem(int precision, const WosLaunch &L, int block) {
 // check each bound against the FP64 distance.
 cudaError_t launch_wos_traced(const WosLaunch &L, int grid, cudaStream_t s) {
   if (L.n_jobs == 0 || L.n_geos == 0 || !L.trace || !L.trace_count) return cudaErrorInvalidValue;
-  const uint32_t dyn = wos_dyn_smem(TWOS_PREC_MIXED, L, kWosBlock);
+  const uint32_t dyn = wos_dyn_smem(TWOS_PREC_MIXED, TWOS_MODE_COMPLIANCE, L, kWosBlock);
   const void *fn = reinterpret_cast<const void *>(&wos_kernel<float, TWOS_MODE_COMPLIANCE, TWOS_SOURCE_CENTER,
                                                               kWosBlock, true>);
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dyn));
   if (e != cudaSuccess) return e;
   WosLaunch copy = L;
+  copy.lanes = 32;
   void *args[] = {&copy};
   return cudaLaunchKernel(fn, dim3(grid), dim3(kWosBlock), args, dyn, s);
 }
@@ -1403,19 +1810,26 @@ cudaError_t launch_wos_traced(const WosLaunch &L, int grid, cudaStream_t s) {
 cudaError_t launch_wos(int precision, int mode, int src, const WosLaunch &L, int grid, int block,
                        cudaStream_t s) {
   if (L.n_jobs == 0 || L.n_geos == 0) return cudaErrorInvalidValue;
-  const uint32_t dyn = wos_dyn_smem(precision, L, block);
+  const uint32_t dyn = wos_dyn_smem(precision, mode, L, block);
   if (dyn > 200 * 1024) return cudaErrorInvalidValue;
   const void *fn = select_wos(precision, mode, src, block, L.grid64, L.wide, L.lane_walks > 1);
   if (!fn) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dyn));
   if (e != cudaSuccess) return e;
+  // A launch with fewer walks than resident lanes spreads them over all warps:
+  // a warp's divergent lanes take turns, so the fewer the better (256 FP64
+  // walks: 1.88 ms with full warps, 1.57 with 16 lanes, 1.18 with 4, 0.76 with
+  // one; 65,536: 4.8 ms full, 4.4 with 19; 98,304 mixed: 1.28 and 1.18).
   WosLaunch copy = L;
+  const uint64_t warps = static_cast<uint64_t>(grid) * (block / 32);
+  const uint64_t claims = (L.total_walks + lane_walks_of(L) - 1) / lane_walks_of(L);
+  copy.lanes = static_cast<int>(std::min<uint64_t>(32, std::max<uint64_t>(1, (claims + warps - 1) / warps)));
   void *args[] = {&copy};
   return cudaLaunchKernel(fn, dim3(grid), dim3(block), args, dyn, s);
 }
 
 int wos_max_blocks_per_sm(int precision, int mode, int src, int block, const WosLaunch &L) {
-  const uint32_t dyn = wos_dyn_smem(precision, L, block);
+  const uint32_t dyn = wos_dyn_smem(precision, mode, L, block);
   const void *fn = select_wos(precision, mode, src, block, L.grid64, L.wide, L.lane_walks > 1);
   if (!fn || dyn > 200 * 1024) return 0;
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dyn)) != cudaSuccess)
@@ -1716,7 +2130,7 @@ template <typename T>
 __global__ void __launch_bounds__(kWosBlock) closest_kernel(const GeoDesc *geo, const double *pts, uint64_t n,
                                                             double query_radius2, double *dist, double *closest,
                                                             uint32_t *error) {
-  __shared__ uint2 s_stack[kStack * kWosBlock];
+  __shared__ uint2 s_stack[(kStack + kCand) * kWosBlock];
   __shared__ GeoDesc G;
   if (threadIdx.x == 0) G = *geo;
   __syncthreads();
@@ -1727,8 +2141,7 @@ __global__ void __launch_bounds__(kWosBlock) closest_kernel(const GeoDesc *geo, 
     const Vec<T> p = to_frame<T>(pts + 3 * i, G);
     T best2 = static_cast<T>(query_radius2);
     uint32_t best_tri = 0;
-    const bool found =
-        nearest<T>(geo_nodes<T>(G), geo_tris<T>(G), G.max_iter, p, best2, best_tri, stack, kWosBlock, err);
+    const bool found = nearest_geo(G, p, best2, best_tri, stack, kWosBlock, err);
     dist[i] = found ? static_cast<double>(sqrt(best2)) : CUDART_INF;
     if (closest) {
       double q[3] = {CUDART_NAN, CUDART_NAN, CUDART_NAN};

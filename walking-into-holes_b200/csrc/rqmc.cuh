@@ -5,7 +5,7 @@
 //
 // One block per (site, batch), one thread per walk; all walks of the block
 // take their steps together.  At each step a thread answers its walk's
-// closest-point query (nearest<T>, stack in local memory); walks within
+// closest-point query (nearest_geo, stack in local memory); walks within
 // epsilon stop and add the boundary data at their exit point; then, in
 // ARRAY mode, the block sorts (Hilbert key, thread) pairs with a bitonic
 // network in shared memory and the walk of rank i takes the Korobov lattice
@@ -89,14 +89,14 @@ template <typename T> __global__ void __launch_bounds__(1024) rqmc_kernel(const 
   bool active = true, cap = false;
   uint32_t steps = 0, err = 0;
   double vu = 0.0, vp = 0.0;
-  uint2 lstack[kStack];
+  uint2 lstack[kStack + kCand];
   const uint32_t ctr3 = (batch << 16) | (R.repeat << 3);
   for (int k = 0; k < R.max_steps; ++k) {
     T r = T(0);
     if (active) {
       T best2 = static_cast<T>(CUDART_INF);
       uint32_t tri = 0;
-      if (!nearest<T>(geo_nodes<T>(G), geo_tris<T>(G), G.max_iter, pos, best2, tri, lstack, 1, err)) {
+      if (!nearest_geo(G, pos, best2, tri, lstack, 1, err)) {
         err |= TWOS_DEVERR_QUERY;
         active = false;
       } else {

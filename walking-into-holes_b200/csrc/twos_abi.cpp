@@ -244,6 +244,15 @@ int open_impl(std::vector<double> &&v, std::vector<uint32_t> &&f, int device, tw
     g.tris_d = m->tris_d.as<TriD>();
     for (int a = 0; a < 3; ++a) g.center[a] = m->center[a];
     g.delta = static_cast<float>(m->delta);
+    // FP64 queries prune with FP32 bounds where FP32 can hold them: squares
+    // of coordinates and of the margin stay in range, and the FP64 rounding
+    // of coordinates far from the origin (2^-46 of their size, more than the
+    // closest-point arithmetic loses) stays far below the margin.
+    double far = 0.0;
+    for (int a = 0; a < 3; ++a) far = std::max(far, std::max(std::fabs(m->bmin[a]), std::fabs(m->bmax[a])));
+    g.cull_margin = reach >= 1e-12 && reach <= 1e12 && far <= 1e6 * reach
+                        ? static_cast<float>(1.0001 * (m->delta + std::ldexp(far, -46)))
+                        : 0.f;
     // A query visits each node and tests each triangle at most once.
     g.max_iter = static_cast<uint32_t>(
         std::min<uint64_t>(2ull * (m->bvh.nodes.size() + m->faces.size() / 3) + 16, 0xffffffffull));

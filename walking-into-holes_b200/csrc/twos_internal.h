@@ -20,6 +20,7 @@ namespace twos {
 constexpr int kLeafMax = 4;
 constexpr int kMaxDepth = 24;    // builder bound (<= 4 * 2^24 triangles); one stack entry per level
 constexpr int kStack = 24;
+constexpr int kCand = 4;         // candidate triangles an FP64 query holds for their FP64 test
 
 // Each child also carries a normal slab: a unit direction n (the child's
 // area-weighted mean normal) and the interval [smin, smax] of n.v over its
@@ -129,6 +130,7 @@ struct GeoDesc {
   const TriD *tris_d;
   double center[3];   // FP32 frame origin (mixed form)
   float delta;        // FP32 distance error bound (mixed form)
+  float cull_margin;  // FP32 pruning margin of FP64 queries; 0: they take the FP64 nodes
   uint32_t max_iter;  // traversal iteration bound (node + leaf visits)
   // Distance-bound grid of the mixed form (null: none).  Vertex (i, j, k)
   // sits at grid_lo + (i, j, k) * grid_h in the FP32 frame; D(v) * grid_q
@@ -236,7 +238,9 @@ struct WosLaunch {
   // Walks a lane claims from the work queue at once and runs one after
   // another (>= 1).
   int lane_walks;
-  // Mixed form: whether a query may start at the entry-node table's node.
+  // Lanes of a warp that take walks (set by launch_wos).
+  int lanes;
+  // Whether a query may start with the distance grid's bound and at the entry-node table's node.
   int entry;
   // FP64 compliance form with the mixed form's distance grid and entry nodes
   // (a comparison of precision alone; off for the plain FP64 form).

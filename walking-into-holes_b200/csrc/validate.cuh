@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(128) validate_kernel(const ValidateLaunch V) {
 }
 
 __global__ void __launch_bounds__(kWosBlock) validate_center_kernel(const ValidateLaunch V) {
-  __shared__ uint2 s_stack[kStack * kWosBlock];
+  __shared__ uint2 s_stack[(kStack + kCand) * kWosBlock];
   const GeoDesc G = *V.geo;
   uint32_t err = 0;
   for (uint32_t site = blockIdx.x * blockDim.x + threadIdx.x; site < V.n_sites; site += gridDim.x * blockDim.x) {
@@ -225,8 +225,7 @@ __global__ void __launch_bounds__(kWosBlock) validate_center_kernel(const Valida
     double best2 = CUDART_INF;
     uint32_t tri = 0;
     double d = CUDART_INF;
-    if (nearest<double>(G.nodes_d, G.tris_d, G.max_iter, Vec<double>{p[0], p[1], p[2]}, best2, tri,
-                        s_stack + threadIdx.x, kWosBlock, err))
+    if (nearest_geo(G, Vec<double>{p[0], p[1], p[2]}, best2, tri, s_stack + threadIdx.x, kWosBlock, err))
       d = sqrt(best2);
     for (uint32_t i = 0; i < V.n_cav; ++i) {
       const double dx = p[0] - V.cavities[3 * i], dy = p[1] - V.cavities[3 * i + 1], dz = p[2] - V.cavities[3 * i + 2];
