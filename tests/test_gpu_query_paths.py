@@ -94,3 +94,29 @@ def test_walks_do_not_depend_on_the_lanes_that_run_them(tb, precision):
                                                          site_offset=s))
                 assert np.array_equal(one["u"][0], every["u"][s])
                 assert np.array_equal(one["steps"][0], every["steps"][s])
+
+
+@pytest.mark.parametrize("radius_cap", [0.02, 0.1, 1e3])
+@pytest.mark.parametrize("epsilon,n_cav,walks,offset", [(1e-6, 0, 300, 0.0), (1e-6, 2, 33, 0.0), (0.12, 1, 64, 0.0),
+                                                        (1e-6, 1, 64, 4e6)])
+def test_certified_walks_equal_the_oracle(tb, oracle_mod, radius_cap, epsilon, n_cav, walks, offset):
+    """Certified walks over radius caps that skip no query, some and nearly all
+    of them, shells up to beyond radius_cap / 0.95, cavities, a site near the
+    surface, and a mesh too far from the origin for FP32 pruning: the oracle's
+    steps and flags exactly, its values to the parity tests' 1e-10."""
+    V, F = tb.geometry.noise_sphere(3, 1)
+    V = V + offset
+    sites = np.array([[0.05, -0.1, 0.2], [0.3, 0.2, -0.1], [0.0, 0.0, 0.7]]) + offset
+    cav = np.array([[-0.2, 0.1, 0.0], [0.1, -0.3, 0.1]])[:n_cav] + offset
+    common = dict(walks=walks, seed=8, epsilon=epsilon, max_steps=96, cavity_radius=0.065)
+    cfg = tb.Config(precision="fp64", green=True, source=tb.sources.constant(1.0), **common)
+    with tb.Mesh(V, F) as m:
+        s, st, _ = m.validate(sites, cfg, cavities=cav if n_cav else None, radius_cap=radius_cap, value_cap=0.2,
+                              strict=False)
+    o = oracle_mod.OracleMesh(V, F).validate(
+        sites, radius_cap, 0.2, cavities=cav if n_cav else None, rng=oracle_mod.RNG_COUNTER, green=True,
+        source=[oracle_mod.term(oracle_mod.TERM_CONST, 1.0)], **common)
+    for k in ("steps", "capped", "clipped", "contained"):
+        assert np.array_equal(s[k].astype(o[k].dtype), o[k]), k
+    np.testing.assert_allclose(s["value"], o["value"], rtol=1e-10, atol=0)
+    assert np.array_equal(st["center_clearance_lower"][:, 0], o["clearance"])

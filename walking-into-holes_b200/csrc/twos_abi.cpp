@@ -253,6 +253,19 @@ int open_impl(std::vector<double> &&v, std::vector<uint32_t> &&f, int device, tw
     g.cull_margin = reach >= 1e-12 && reach <= 1e12 && far <= 1e6 * reach
                         ? static_cast<float>(1.0001 * (m->delta + std::ldexp(far, -46)))
                         : 0.f;
+    double extent2 = 0.0;
+    for (size_t f = 0; f < m->faces.size(); f += 3) {
+      double d2 = 0.0;
+      for (int a = 0; a < 3; ++a) {
+        const double x = m->vertices[3 * static_cast<size_t>(m->faces[f]) + a],
+                     y = m->vertices[3 * static_cast<size_t>(m->faces[f + 1]) + a],
+                     z = m->vertices[3 * static_cast<size_t>(m->faces[f + 2]) + a];
+        const double e = std::max({x, y, z}) - std::min({x, y, z});
+        d2 += e * e;
+      }
+      extent2 = std::max(extent2, d2);
+    }
+    g.box_extent = static_cast<float>(1.0001 * std::sqrt(extent2));
     // A query visits each node and tests each triangle at most once.
     g.max_iter = static_cast<uint32_t>(
         std::min<uint64_t>(2ull * (m->bvh.nodes.size() + m->faces.size() / 3) + 16, 0xffffffffull));
@@ -1224,7 +1237,7 @@ int twos_validate(twos_mesh *m, const twos_request *r, const twos_validate_param
   const auto t0 = std::chrono::steady_clock::now();
   const size_t walks = static_cast<size_t>(r->walks);
   const size_t total = static_cast<size_t>(n_sites) * walks;
-  DevBuf dsamp, dclear, dcenter, dterms;
+  DevBuf dsamp, dclear, dcenter, dmesh, dterms;
   unsigned long long tot[2] = {0, 0};
   std::vector<double> clearance(n_sites), center(n_sites);
   RunOut ro;
@@ -1246,6 +1259,8 @@ int twos_validate(twos_mesh *m, const twos_request *r, const twos_validate_param
     dsamp.reserve(total * sizeof(twos_cert_sample));
     dclear.reserve(n_sites * sizeof(double));
     dcenter.reserve(n_sites * sizeof(double));
+    dmesh.reserve(n_sites * sizeof(double));
+    check(cudaMemsetAsync(m->counter.ptr, 0, sizeof(unsigned long long), m->stream), "memset");
     begin_totals(m);
     ValidateLaunch V{};
     V.geo = m->geo.as<GeoDesc>();
@@ -1268,6 +1283,9 @@ int twos_validate(twos_mesh *m, const twos_request *r, const twos_validate_param
     V.samples = dsamp.as<twos_cert_sample>();
     V.clearance = dclear.as<double>();
     V.center_distance = dcenter.as<double>();
+    V.mesh_distance = dmesh.as<double>();
+    V.counter = m->counter.as<unsigned long long>();
+    V.cull = m->geo_host.cull_margin > 0.f;
     V.totals = m->totals.as<unsigned long long>() + 3;  // [3] failures, [4] steps
     V.error = reinterpret_cast<uint32_t *>(m->totals.as<unsigned long long>() + 2);
     check(cudaEventRecord(m->ev0, m->stream), "event");
@@ -1287,10 +1305,10 @@ int twos_validate(twos_mesh *m, const twos_request *r, const twos_validate_param
     check(cudaEventElapsedTime(&ms, m->ev0, m->ev1), "event time");
     ro.kernel_seconds = ro.walk_seconds = ms / 1e3;
   } catch (const std::exception &e) {
-    for (DevBuf *b : {&dsamp, &dclear, &dcenter, &dterms}) b->release();
+    for (DevBuf *b : {&dsamp, &dclear, &dcenter, &dmesh, &dterms}) b->release();
     return fail(TWOS_ERR_RUNTIME, e.what());
   }
-  for (DevBuf *b : {&dsamp, &dclear, &dcenter, &dterms}) b->release();
+  for (DevBuf *b : {&dsamp, &dclear, &dcenter, &dmesh, &dterms}) b->release();
   // Stage statistics: prefixes n in {1024, 4096, 16384, 65536} below walks,
   // then walks; sums in long double in sample order (minimum_benefit.hpp:160-176).
   std::vector<uint32_t> ns;

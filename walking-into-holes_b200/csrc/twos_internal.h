@@ -131,6 +131,7 @@ struct GeoDesc {
   double center[3];   // FP32 frame origin (mixed form)
   float delta;        // FP32 distance error bound (mixed form)
   float cull_margin;  // FP32 pruning margin of FP64 queries; 0: they take the FP64 nodes
+  float box_extent;   // largest diagonal of a triangle's bounding box, rounded up
   uint32_t max_iter;  // traversal iteration bound (node + leaf visits)
   // Distance-bound grid of the mixed form (null: none).  Vertex (i, j, k)
   // sits at grid_lo + (i, j, k) * grid_h in the FP32 frame; D(v) * grid_q
@@ -442,6 +443,9 @@ struct ValidateLaunch {
   double epsilon, cavity_radius, radius_cap, value_cap;
   twos_cert_sample *samples;   // [n_sites * walks]
   double *clearance;           // [n_sites] certified distance at the site
+  double *mesh_distance;       // [n_sites] the mesh's part of it
+  unsigned long long *counter; // work-queue head, zeroed before launch
+  int cull;                    // whether FP32 can prune (GeoDesc::cull_margin)
   double *center_distance;     // [n_sites] FP64 domain distance at the site
   unsigned long long *totals;  // [0] containment failures [1] steps
   uint32_t *error;
