@@ -120,3 +120,30 @@ def test_certified_walks_equal_the_oracle(tb, oracle_mod, radius_cap, epsilon, n
         assert np.array_equal(s[k].astype(o[k].dtype), o[k]), k
     np.testing.assert_allclose(s["value"], o["value"], rtol=1e-10, atol=0)
     assert np.array_equal(st["center_clearance_lower"][:, 0], o["clearance"])
+
+
+@pytest.mark.parametrize("level,query_radius", [(1, 4.0), (5, 4.0), (5, None), (3, 0.97)])
+def test_first_queries_among_equidistant_triangles(tb, oracle_mod, level, query_radius):
+    """The centre of a sphere is (nearly) equidistant to every triangle, so the
+    warp's common stack fills up: the walks from it and from points beside it
+    are the oracle's.  With a query radius below the distance, every walk
+    fails the same way."""
+    V, F = tb.geometry.icosphere(level)
+    sites = np.array([[0.0, 0.0, 0.0], [1e-9, 0.0, 0.0], [0.01, -0.02, 0.015], [0.5, 0.1, -0.2]])
+    cfg = tb.Config(walks=20, precision="fp64", seed=12, epsilon=1e-4, source=tb.sources.constant(1.0),
+                    query_radius=query_radius)
+    with tb.Mesh(V, F) as m:
+        if query_radius is not None and query_radius < 1.0:
+            with pytest.raises(tb.TwosError, match="closest-point query failed"):
+                m.walk_samples(sites[:1], cfg)
+            return
+        g = m.walk_samples(sites, cfg)
+        d64 = m.closest_point(sites, precision="fp64", with_points=False)
+        d32 = m.closest_point(sites, precision="mixed", with_points=False)
+        delta = m.info()["mixed_delta"]
+    o = oracle_mod.OracleMesh(V, F).walk_samples(sites, rng=oracle_mod.RNG_COUNTER, walks=20, seed=12, epsilon=1e-4,
+                                                 max_steps=512, source=[oracle_mod.term(oracle_mod.TERM_CONST, 1.0)],
+                                                 weight_order=1)
+    assert np.array_equal(g["steps"], o["steps"])
+    np.testing.assert_allclose(g["u"], o["u"], rtol=1e-10, atol=0)
+    assert np.max(np.abs(d64 - d32)) <= delta

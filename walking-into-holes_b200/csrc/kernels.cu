@@ -1677,16 +1677,169 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
   }
 }
 
+// ---------------------------------------------------------------- warp search
+// One query by a whole warp, for the few long queries a call starts with (a
+// site deep inside visits hundreds of nodes, and one lane waits for memory at
+// each): up to 32 entries of a common stack are taken at once, a lane each.
+// The grid's bound is close to the distance, so almost all of them have to be
+// visited in any order.  `limit` is the squared pruning threshold at entry;
+// leaf(i, rows, limit) tests triangle i (its four float4) and returns the
+// lane's new threshold.  SLABS: node bounds with the normal slabs (distances
+// to triangles) or boxes only.
+//
+// The stack holds kWarpStack entries per warp; near its end one entry at a
+// time is taken, which needs at most one more per level.
+constexpr int kWarpStack = 512;
+template <bool SLABS, typename Leaf>
+__device__ __forceinline__ void warp_search(const GeoDesc &g, const Vec<float> &p, int root, float &limit,
+                                            uint2 *stack, uint32_t &err, Leaf &&leaf) {
+  const unsigned full = 0xffffffffu, lane = threadIdx.x & 31u;
+  __syncwarp();
+  if (lane == 0) stack[0] = make_uint2(static_cast<uint32_t>(root), 0u);
+  __syncwarp();
+  uint32_t iter = 0;
+  for (int size = 1; size > 0;) {
+    if (++iter > g.max_iter) {
+      err |= TWOS_DEVERR_ITER;
+      break;
+    }
+    const int take = size > kWarpStack - 64 ? 1 : min(size, 32);
+    size -= take;
+    uint2 e = make_uint2(0u, 0x7f800000u);
+    if (static_cast<int>(lane) < take) e = stack[size + take - 1 - static_cast<int>(lane)];
+    const bool live = static_cast<int>(lane) < take && __uint_as_float(e.y) < limit;
+    const int node = static_cast<int>(e.x);
+    float dn = CUDART_INF_F, df = CUDART_INF_F;
+    int cn = 0, cf = 0;
+    if (live && node < 0) {
+      const uint32_t enc = ~static_cast<uint32_t>(node);
+      for (uint32_t i = enc >> 3, end = (enc >> 3) + (enc & 7u); i < end; ++i) {
+        float4 r[4];
+        ldg32(&g.tris_f[i].plane, r[0], r[1]);
+        ldg32(&g.tris_f[i].b, r[2], r[3]);
+        limit = fminf(limit, leaf(i, r, limit));
+      }
+    } else if (live) {
+      const NodeF *n = g.nodes_f + node;
+      float4 x, y, z, nl, nr, t;
+      ldg32(&n->x, x, y);
+      ldg32(&n->z, z, nl);
+      ldg32(&n->nr, nr, t);
+      if (!SLABS) nl = nr = t = make_float4(0.f, 0.f, 0.f, 0.f);
+      int cl, cr;
+      node_bounds(x, y, z, nl, nr, t, p, dn, df, cl, cr);
+      if (!SLABS) {
+        cl = __float_as_int(__ldg(&n->tail.z));
+        cr = __float_as_int(__ldg(&n->tail.w));
+      }
+      const bool swap = df < dn;
+      cn = swap ? cr : cl;
+      cf = swap ? cl : cr;
+      const float d = dn;
+      dn = fminf(d, df);
+      df = fmaxf(d, df);
+    }
+    // Nearer children above the farther ones, the first lane's on top.
+    limit = __uint_as_float(__reduce_min_sync(full, __float_as_uint(limit)));
+    const unsigned mf = __ballot_sync(full, df < limit), mn = __ballot_sync(full, dn < limit);
+    const unsigned above = lane == 31u ? 0u : full << (lane + 1u);
+    if (df < limit) stack[size + __popc(mf & above)] = make_uint2(static_cast<uint32_t>(cf), __float_as_uint(df));
+    size += __popc(mf);
+    if (dn < limit) stack[size + __popc(mn & above)] = make_uint2(static_cast<uint32_t>(cn), __float_as_uint(dn));
+    size += __popc(mn);
+    __syncwarp();
+  }
+}
+
+// The smallest value of the warp and its triangle, to every lane (ties: the
+// lower leaf-order index).
+template <typename T> __device__ __forceinline__ void warp_best(T &best, uint32_t &tri) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const T b = __shfl_xor_sync(0xffffffffu, best, o);
+    const uint32_t t = __shfl_xor_sync(0xffffffffu, tri, o);
+    if (b < best || (b == best && t < tri)) {
+      best = b;
+      tri = t;
+    }
+  }
+}
+
+// nearest_geo() by a warp (all lanes with the same arguments).
+__device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<float> &p, float &best2, uint32_t &best_tri,
+                                             uint2 *stack, uint32_t &err) {
+  float upper;
+  int node;
+  grid_start(g, p, sqrtf(best2), upper, node);
+  float limit = fminf(best2, upper * upper), mine = CUDART_INF_F;
+  uint32_t tri = 0xffffffffu;
+  warp_search<true>(g, p, node, limit, stack, err, [&](uint32_t i, const float4 *r, float lim) {
+    if (!(plane_gap2(r[0], r[1], p) < lim)) return lim;
+    const float d2 = tri_dist2(p, Vec<float>{r[1].x, r[1].y, r[1].z}, Vec<float>{r[2].x, r[2].y, r[2].z},
+                               Vec<float>{r[3].x, r[3].y, r[3].z});
+    if (d2 < lim) {
+      mine = d2;
+      tri = i;
+    }
+    return d2;
+  });
+  warp_best(mine, tri);
+  if (!(mine < best2)) return false;
+  best2 = mine;
+  best_tri = tri;
+  return true;
+}
+
+__device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<double> &p, double &best2,
+                                             uint32_t &best_tri, uint2 *stack, uint32_t &err) {
+  Cull c;
+  if (!cull_begin(g, p, best2, c)) {
+    const Plain64 r = nearest_plain64(&g, p.x, p.y, p.z, best2);
+    err |= r.flags & 0x7fffffffu;
+    if (!(r.flags >> 31)) return false;
+    best2 = r.best2;
+    best_tri = r.tri;
+    return true;
+  }
+  float upper;
+  int node;
+  grid_start(g, c.p, sqrtf(c.limit), upper, node);
+  const float reach = __fadd_ru(upper, c.margin);
+  float limit = fminf(c.limit, __fmul_ru(reach, reach));
+  double mine = best2;
+  uint32_t tri = 0xffffffffu;
+  warp_search<true>(g, c.p, node, limit, stack, err, [&](uint32_t i, const float4 *r, float lim) {
+    if (!(plane_gap2(r[0], r[1], c.p) < lim)) return lim;
+    Vec<double> ta, tb, tc;
+    load_tri(g.tris_d, i, ta, tb, tc);
+    const double d2 = tri_dist2(p, ta, tb, tc);
+    if (!(d2 < mine)) return lim;
+    mine = d2;
+    tri = i;
+    return cull_limit(d2, c.margin);
+  });
+  warp_best(mine, tri);
+  if (tri == 0xffffffffu) return false;
+  best2 = mine;
+  best_tri = tri;
+  return true;
+}
+
 // Per-site first query: one closest-point traversal per site of the launch
 // (the N walks of a site all start there), written as the squared mesh
 // distance, or -1 when no surface point lies within the query radius.
+//
+// A warp per site: one thread per site took 634 us for 384 sites of the
+// 20,480-triangle noise sphere (426 with the grid's bound), as long as half
+// their walks; with a warp each the whole call fell from 1.31 to 1.03 ms.
 template <typename T>
 __global__ void __launch_bounds__(kWosBlock) site_prepass_kernel(const WosLaunch L) {
-  __shared__ uint2 s_stack[(kStack + kCand) * kWosBlock];
-  uint2 *stack = s_stack + threadIdx.x;
+  __shared__ uint2 s_stack[kWarpStack * (kWosBlock / 32)];
+  uint2 *stack = s_stack + kWarpStack * (threadIdx.x >> 5);
   uint32_t err = 0;
   T *out = static_cast<T *>(L.site_best2);
-  for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < L.total_sites; g += gridDim.x * blockDim.x) {
+  const uint32_t warps = gridDim.x * (kWosBlock / 32);
+  for (uint32_t g = blockIdx.x * (kWosBlock / 32) + (threadIdx.x >> 5); g < L.total_sites; g += warps) {
     uint32_t lo = 0, hi = L.n_jobs - 1;
     while (lo < hi) {
       const uint32_t mid = (lo + hi + 1) >> 1;
@@ -1700,15 +1853,15 @@ __global__ void __launch_bounds__(kWosBlock) site_prepass_kernel(const WosLaunch
     const Vec<T> p = to_frame<T>(L.sites + 3ull * (J.site_begin + (g - J.site_rank)), G);
     T best2 = static_cast<T>(J.query_radius2);
     uint32_t tri = 0;
-    const bool found = nearest_geo(G, p, best2, tri, stack, kWosBlock, err);
-    out[g] = found ? best2 : T(-1);
+    const bool found = warp_nearest(G, p, best2, tri, stack, err);
+    if ((threadIdx.x & 31u) == 0) out[g] = found ? best2 : T(-1);
   }
   if (err) atomicOr(L.error, err);
 }
 
 cudaError_t launch_site_prepass(int precision, const WosLaunch &L, cudaStream_t s) {
   if (!L.site_best2 || L.total_sites == 0) return cudaSuccess;
-  const int grid = static_cast<int>(std::min<uint32_t>((L.total_sites + kWosBlock - 1) / kWosBlock, 148u * 16));
+  const int grid = static_cast<int>(std::min<uint32_t>((L.total_sites + kWosBlock / 32 - 1) / (kWosBlock / 32), 148u * 16));
   if (precision == TWOS_PREC_MIXED)
     site_prepass_kernel<float><<<grid, kWosBlock, 0, s>>>(L);
   else

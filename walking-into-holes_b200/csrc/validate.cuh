@@ -473,29 +473,47 @@ __global__ void __launch_bounds__(128) validate_kernel(const ValidateLaunch V) {
   if (total_steps) atomicAdd(&V.totals[1], total_steps);
 }
 
+// Distances at each site, a warp per site: the exact FP64 one, and the
+// certified ones to the mesh (every walk's first query) and to the domain.
 __global__ void __launch_bounds__(kWosBlock) validate_center_kernel(const ValidateLaunch V) {
-  __shared__ uint2 s_stack[(kStack + kCand) * kWosBlock];
+  __shared__ uint2 s_stack[kWarpStack * (kWosBlock / 32)];
+  uint2 *stack = s_stack + kWarpStack * (threadIdx.x >> 5);
   const GeoDesc G = *V.geo;
   uint32_t err = 0;
-  for (uint32_t site = blockIdx.x * blockDim.x + threadIdx.x; site < V.n_sites; site += gridDim.x * blockDim.x) {
+  const uint32_t warps = gridDim.x * (kWosBlock / 32);
+  for (uint32_t site = blockIdx.x * (kWosBlock / 32) + (threadIdx.x >> 5); site < V.n_sites; site += warps) {
     const double *p = V.sites + 3ull * site;
+    const Vec<double> v{p[0], p[1], p[2]};
     double best2 = CUDART_INF;
     uint32_t tri = 0;
     double d = CUDART_INF;
-    if (nearest_geo(G, Vec<double>{p[0], p[1], p[2]}, best2, tri, s_stack + threadIdx.x, kWosBlock, err))
-      d = sqrt(best2);
+    if (warp_nearest(G, v, best2, tri, stack, err)) d = sqrt(best2);
+    double dm = CUDART_INF;
+    Cull c;
+    if (cull_begin(G, v, best2, c)) {
+      // Boxes contain their triangles: the exact distance bounds this one.
+      float limit = c.limit;
+      warp_search<false>(G, c.p, 0, limit, stack, err, [&](uint32_t i, const float4 *r, float lim) {
+        const float gx = gap(fminf(fminf(r[1].x, r[2].x), r[3].x), fmaxf(fmaxf(r[1].x, r[2].x), r[3].x), c.p.x);
+        const float gy = gap(fminf(fminf(r[1].y, r[2].y), r[3].y), fmaxf(fmaxf(r[1].y, r[2].y), r[3].y), c.p.y);
+        const float gz = gap(fminf(fminf(r[1].z, r[2].z), r[3].z), fmaxf(fmaxf(r[1].z, r[2].z), r[3].z), c.p.z);
+        if (!(__fmaf_rn(gx, gx, __fmaf_rn(gy, gy, gz * gz)) < lim)) return lim;
+        dm = fmin(dm, cv_tri_box(G, i, p));
+        return cull_limit(dm * dm, c.margin);
+      });
+      warp_best(dm, tri);
+    } else {
+      dm = cv_mesh_distance(G, p, err);
+    }
+    if ((threadIdx.x & 31u) != 0) continue;
+    double clear = dm;
     for (uint32_t i = 0; i < V.n_cav; ++i) {
       const double dx = p[0] - V.cavities[3 * i], dy = p[1] - V.cavities[3 * i + 1], dz = p[2] - V.cavities[3 * i + 2];
       d = fmin(d, sqrt(dx * dx + dy * dy + dz * dz) - V.cavity_radius);
+      clear = fmin(clear, cv_dn(cv_point_distance(p, V.cavities + 3 * i, false) - V.cavity_radius));
     }
     V.center_distance[site] = d;
-    // The certified distances at the site: to the mesh (every walk's first
-    // query) and to the domain.
-    const double dm = cv_mesh_distance(G, p, err);
     V.mesh_distance[site] = dm;
-    double clear = dm;
-    for (uint32_t i = 0; i < V.n_cav; ++i)
-      clear = fmin(clear, cv_dn(cv_point_distance(p, V.cavities + 3 * i, false) - V.cavity_radius));
     V.clearance[site] = fmax(0.0, clear);
   }
   if (err) atomicOr(V.error, err);
@@ -504,7 +522,7 @@ __global__ void __launch_bounds__(kWosBlock) validate_center_kernel(const Valida
 cudaError_t launch_validate(const ValidateLaunch &V, cudaStream_t s) {
   const uint64_t total = static_cast<uint64_t>(V.n_sites) * V.walks;
   if (total == 0) return cudaSuccess;
-  const int grid_c = static_cast<int>(std::min<uint32_t>((V.n_sites + kWosBlock - 1) / kWosBlock, 148u * 4));
+  const int grid_c = static_cast<int>(std::min<uint32_t>((V.n_sites + kWosBlock / 32 - 1) / (kWosBlock / 32), 148u * 4));
   validate_center_kernel<<<grid_c, kWosBlock, 0, s>>>(V);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
