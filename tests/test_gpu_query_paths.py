@@ -147,3 +147,37 @@ def test_first_queries_among_equidistant_triangles(tb, oracle_mod, level, query_
     assert np.array_equal(g["steps"], o["steps"])
     np.testing.assert_allclose(g["u"], o["u"], rtol=1e-10, atol=0)
     assert np.max(np.abs(d64 - d32)) <= delta
+
+
+@pytest.mark.parametrize("shape", ["tetra", "sphere1", "sphere5", "noise6", "fan5", "fan64", "sliver"])
+def test_first_queries_return_the_traversals_value(tb, shape):
+    """A site's first distance, found by a whole warp, is the one a lane's
+    traversal returns, to the last bit: mixed walks that start at the sites
+    against the same walks started by a traversal (the cap of one step makes a
+    walk's value its first radius)."""
+    rng = np.random.default_rng(5)
+    if shape == "tetra":
+        V = np.array([[0.0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1]]) - 0.25
+        F = np.array([[0, 2, 1], [0, 1, 3], [0, 3, 2], [1, 2, 3]], dtype=np.uint32)
+    elif shape.startswith("sphere"):
+        V, F = tb.geometry.icosphere(int(shape[6:]))
+    elif shape.startswith("noise"):
+        V, F = tb.geometry.noise_sphere(int(shape[5:]), 1)
+    elif shape == "sliver":
+        V, F = tb.geometry.icosphere(3)
+        V = V * np.array([1.0, 1e-3, 1.0])
+    else:
+        V, F = _fan(int(shape[3:]))
+    mid = V[F.astype(np.int64)].mean(1)
+    P = np.concatenate([mid[rng.integers(0, len(mid), 2000)] * rng.uniform(0.0, 0.9, (2000, 1)),
+                        V[rng.integers(0, len(V), 300)] * rng.uniform(0.0, 0.95, (300, 1)), np.zeros((1, 3))])
+    with tb.Mesh(V, F) as m:
+        d = m.closest_point(P, precision="mixed", with_points=False)  # one lane per point
+        delta = np.float32(m.info()["mixed_delta"])
+        cfg = tb.Config(walks=2, precision="mixed", seed=3, epsilon=1e-30, max_steps=1, query_radius=None,
+                        source=tb.sources.constant(6.0))
+        got = m.walk_samples(P, cfg)
+    r = d.astype(np.float32) - delta
+    # u = r^2/6 * 6 of the first ball, evaluated in FP32 as the walk does.
+    want = np.where(r > np.float32(1e-30), (r * r / np.float32(6)) * np.float32(6), np.float32(0))
+    assert np.array_equal(got["u"][:, 0].astype(np.float32), want)

@@ -475,6 +475,13 @@ void pack_bvh_f32(const HostBvh &bvh, const std::vector<double> &v, const std::v
   }
 }
 
+std::vector<uint32_t> node_first_triangles(const HostBvh &bvh) {
+  std::vector<uint32_t> first;
+  first.reserve(bvh.nodes.size());
+  for (const Range &r : node_ranges(bvh)) first.push_back(r.begin);
+  return first;
+}
+
 void pack_bvh_f64(const HostBvh &bvh, const std::vector<double> &v, const std::vector<uint32_t> &f,
                   std::vector<NodeD> &nodes, std::vector<TriD> &tris) {
   const size_t nf = bvh.order.size();

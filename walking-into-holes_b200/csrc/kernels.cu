@@ -932,12 +932,13 @@ template <typename V> struct Cell<V, true> {
   __device__ __forceinline__ operator V() const { return *p; }
   __device__ __forceinline__ void operator=(V x) { *p = x; }
 };
-// Shared-memory bytes of that state per thread.
+// Shared-memory bytes of that state per thread (both forms: the nearest
+// cavity's distance and index).
 template <typename T> __host__ __device__ constexpr int wos_cold_bytes(bool gradient) {
-  return sizeof(T) == 4 ? 0 : 72 + (gradient ? 96 : 0);
+  return sizeof(T) == 4 ? 8 : 88 + (gradient ? 96 : 0);
 }
 
-enum : int { kIdle = 0, kTraverse = 1, kStep = 2, kBegin = 3 };
+enum : int { kIdle = 0, kTraverse = 1, kStep = 2, kBegin = 3, kFirst = 4 };
 
 // Persistent walk-on-spheres kernel as a per-lane state machine.  Each loop
 // iteration every traversing lane runs up to `units` units of work back to
@@ -1055,6 +1056,14 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
     else
       c.v = 0;
   };
+  // Distance to the nearest cavity (infinite without one) and, in boundary
+  // mode, its index.
+  Cell<T, true> dcav;
+  Cell<int, true> icav;
+  constexpr int kCavWord = COLD ? 9 : 0;
+  dcav.p = reinterpret_cast<volatile T *>(s_cold + (kCavWord * BLOCK) * 8 + threadIdx.x * sizeof(T));
+  icav.p = reinterpret_cast<volatile int *>(s_cold + (kCavWord * BLOCK) * 8 + BLOCK * sizeof(T) + threadIdx.x * 4);
+
   uint32_t job = 0;
   Cell<T, COLD> px, py, pz, u, pv, best2;
   Cell<uint64_t, COLD> wid;
@@ -1074,14 +1083,14 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
   // the ball source terms of grad U / grad P.
   Cell<T, COLD> g_r0, g_u0, g_p0, g_w0[3], g_su[3], g_sp[3];
   if constexpr (GRAD) {
-    cell(g_r0, 9);
-    cell(g_u0, 10);
-    cell(g_p0, 11);
+    cell(g_r0, 11);
+    cell(g_u0, 12);
+    cell(g_p0, 13);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      cell(g_w0[k], 12 + k);
-      cell(g_su[k], 15 + k);
-      cell(g_sp[k], 18 + k);
+      cell(g_w0[k], 14 + k);
+      cell(g_su[k], 17 + k);
+      cell(g_sp[k], 20 + k);
     }
   }
   // Query state.  The FP64 form prunes in FP32 (cull.p, cull.limit); the
@@ -1135,8 +1144,8 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
   };
   // Starts the query at pos; `in_grid`: with the grid's upper bound and entry
   // node there.
-  auto begin_query = [&](const JobDesc &J, const GeoDesc &G, const Vec<T> &pos, bool in_grid, float upper,
-                         int entry_node) {
+  auto begin_query = [&](const JobDesc &J, const GeoDesc &G, const Vec<T> &pos, bool in_grid, float bound,
+                         float upper, int entry_node, T dc) {
     T best2 = static_cast<T>(J.query_radius2);
     found = false;
     node = 0;
@@ -1157,8 +1166,29 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
         return;
       }
     }
+    const float ubs = __fmaf_ru(6.f, G.delta, upper);
+    // A cavity nearer than the mesh decides the step, so the search goes no
+    // farther than the cavity, and with a mesh known to be beyond there is
+    // none -- once the mesh is known to lie within the query radius.  (Design
+    // loop around an inserted cavity, 262,144 walks on 5,120 triangles with
+    // the grid steps off: 29 ms without, 5 with.)
+    if (dc < static_cast<T>(CUDART_INF_F) &&
+        ((in_grid && static_cast<T>(ubs) * static_cast<T>(ubs) < best2) || J.query_radius2 == CUDART_INF)) {
+      if (dc <= static_cast<T>(in_grid ? fmaxf(bound, 0.f) : 0.f)) {
+        set_best2(static_cast<T>(CUDART_INF_F));
+        found = true;
+        if (sizeof(T) == 8) cull.count = 0;
+        phase = kStep;
+        return;
+      }
+      const T lim = dc * dc * (T(1) + T(0x1.0p-20));
+      if (lim < best2) {
+        best2 = lim;
+        found = true;
+        if constexpr (sizeof(T) == 8) cull.limit = fminf(cull.limit, cull_limit(best2, cull.margin));
+      }
+    }
     if (in_grid) {
-      const float ubs = __fmaf_ru(6.f, G.delta, upper);
       if (!WIDE && entry_node >= 0 && ubs < G.entry_radius) node = entry_node;
       if constexpr (sizeof(T) == 4) {
         best2 = fminf(best2, ubs * ubs);
@@ -1232,7 +1262,8 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
         // First query answered by the per-site pre-pass.
         best2 = static_cast<const T *>(L.site_best2)[J.site_rank + at];
         found = best2 >= T(0);
-        phase = kStep;
+        dcav = CUDART_INF_F;
+        phase = J.n_cav ? kFirst : kStep;
       } else {
         phase = kBegin;
       }
@@ -1310,26 +1341,12 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
             err |= TWOS_DEVERR_QUERY;
             d = T(0);  // ends the walk; the call reports the failure
           }
-          const T R = to_T<T>(J.cavity_radius);
-          const T dmesh = d;
-          int hit_cav = -1;
-          bool cav_nearer = false;  // gradient mode: the exit is on a cavity
-          for (uint32_t c = 0; c < J.n_cav; ++c) {
-            const Vec<T> cc = to_frame<T>(L.cavities + 3ull * (J.cav_begin + c), G);
-            const Vec<T> dv = sub(pos, cc);
-            const T len = sqrt(dot3(dv, dv));
-            const T dc = len - R;
-            if (MODE == kModeBoundary) {
-              // closest_boundary (wih_twos.cpp:612-624): the first strictly nearer cavity.
-              if (dc < d && len > T(0)) {
-                d = dc;
-                hit_cav = static_cast<int>(c);
-              }
-            } else {
-              d = dc < d ? dc : d;
-              if (GRAD && dc < dmesh) cav_nearer = true;
-            }
-          }
+          const T dmesh = d, dc = dcav;
+          if (dc < d) d = dc;
+          // Boundary mode: the first strictly nearer cavity (closest_boundary,
+          // wih_twos.cpp:612-624).  Gradient mode: the exit is on a cavity.
+          const int hit_cav = dc < dmesh ? static_cast<int>(icav) : -1;
+          const bool cav_nearer = dc < dmesh;
           // The mixed form shrinks the radius by the FP32 distance error bound;
           // the FP64 form uses the distance itself (wih_twos.cpp:645-647).
           const T r = sizeof(T) == 4 ? d - static_cast<T>(G.delta) : d;
@@ -1412,7 +1429,7 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
                 const Vec<T> dv = sub(pos, cc);
                 const T inv = T(1) / sqrt(dot3(dv, dv));
                 const Vec<T> dir{dv.x * inv, dv.y * inv, dv.z * inv};
-                q = add_scaled(cc, dir, R);
+                q = add_scaled(cc, dir, to_T<T>(J.cavity_radius));
                 nrm = {dir.x * T(-1), dir.y * T(-1), dir.z * T(-1)};
                 h.cavity = hit_cav;
               } else {
@@ -1468,6 +1485,27 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
             break;
           }
         }
+        // The nearest cavity at the new position.
+        T dc = CUDART_INF_F;
+        if (J.n_cav) {
+          const T R = to_T<T>(J.cavity_radius);
+          int nearest_cav = -1;
+          for (uint32_t c = 0; c < J.n_cav; ++c) {
+            const Vec<T> cc = to_frame<T>(L.cavities + 3ull * (J.cav_begin + c), G);
+            const Vec<T> dv = sub(pos, cc);
+            const T len = sqrt(dot3(dv, dv));
+            if (len - R < dc && (MODE != kModeBoundary || len > T(0))) {
+              dc = len - R;
+              nearest_cav = static_cast<int>(c);
+            }
+          }
+          if (MODE == kModeBoundary) icav = nearest_cav;
+        }
+        dcav = dc;
+        if (phase == kFirst) {
+          phase = kStep;
+          break;
+        }
         // Distance-bound grid: D(v) - |x - v| over the corners v of x's cell
         // bounds the mesh distance from below; a bound of at least grid_tau
         // spacings is the next ball's radius and no query is needed.  A grid
@@ -1498,7 +1536,7 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
             break;
           }
         }
-        begin_query(J, G, pos, in_grid && L.entry, upper, entry_node);
+        begin_query(J, G, pos, in_grid && L.entry, bound, upper, entry_node, dc);
       } while (false);
     }
 
@@ -1766,27 +1804,132 @@ template <typename T> __device__ __forceinline__ void warp_best(T &best, uint32_
 }
 
 // nearest_geo() by a warp (all lanes with the same arguments).
+//
+// FP32: which of several triangles within rounding of the minimum a lane's
+// traversal returns depends on its order, because a node bound can exceed a
+// contained triangle's distance by rounding.  A site's first distance moves
+// all its walks, so the warp's search returns the very value: it collects
+// the triangles within 3 delta of the minimum (bounds are off by less than
+// delta / 2, so no other one can change the outcome), and if there are
+// several, replays the lane's traversal on the nodes that hold them
+// (node_first: a node's first triangle), which are few.
+constexpr int kContend = 64;
+constexpr int kWarpEntries = kWarpStack + kContend + 1;  // shared-memory entries per warp
+__device__ __forceinline__ float widen2(float d2, float by) {
+  const float t = __fadd_ru(__fsqrt_ru(d2), by);
+  return __fmul_ru(t, t);
+}
 __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<float> &p, float &best2, uint32_t &best_tri,
                                              uint2 *stack, uint32_t &err) {
+  const unsigned full = 0xffffffffu, lane = threadIdx.x & 31u;
+  uint2 *list = stack + kWarpStack;
+  uint32_t *count = &list[kContend].x;
   float upper;
-  int node;
-  grid_start(g, p, sqrtf(best2), upper, node);
+  int root;
+  grid_start(g, p, sqrtf(best2), upper, root);
   float limit = fminf(best2, upper * upper), mine = CUDART_INF_F;
-  uint32_t tri = 0xffffffffu;
-  warp_search<true>(g, p, node, limit, stack, err, [&](uint32_t i, const float4 *r, float lim) {
+  if (lane == 0) *count = 0u;
+  warp_search<true>(g, p, root, limit, stack, err, [&](uint32_t i, const float4 *r, float lim) {
     if (!(plane_gap2(r[0], r[1], p) < lim)) return lim;
     const float d2 = tri_dist2(p, Vec<float>{r[1].x, r[1].y, r[1].z}, Vec<float>{r[2].x, r[2].y, r[2].z},
                                Vec<float>{r[3].x, r[3].y, r[3].z});
-    if (d2 < lim) {
-      mine = d2;
-      tri = i;
-    }
-    return d2;
+    if (!(d2 < lim)) return lim;
+    const uint32_t at = atomicAdd(count, 1u);
+    if (at < kContend) list[at] = make_uint2(i, __float_as_uint(d2));
+    mine = fminf(mine, d2);
+    return widen2(d2, 4.f * g.delta);
   });
-  warp_best(mine, tri);
+  mine = __uint_as_float(__reduce_min_sync(full, __float_as_uint(mine)));
   if (!(mine < best2)) return false;
+  // The contenders, one per lane.
+  const float cut = fminf(best2, widen2(mine, 3.f * g.delta));
+  const uint32_t n = *count;
+  uint2 c[2];
+  unsigned m[2];
+  for (uint32_t k = 0; k < 2; ++k) {
+    c[k] = make_uint2(0xffffffffu, 0x7f800000u);
+    if (lane + 32 * k < min(n, static_cast<uint32_t>(kContend))) c[k] = list[lane + 32 * k];
+    m[k] = __ballot_sync(full, __uint_as_float(c[k].y) < cut);
+  }
+  const uint32_t held = __popc(m[0]) + __popc(m[1]);
+  __syncwarp();
+  if (n > kContend || held > 32u) {
+    // Too many to replay: the traversal itself, below the cut.
+    best2 = cut;
+    return nearest<float>(g.nodes_f, g.tris_f, g.max_iter, p, best2, best_tri, stack, 1, err, root);
+  }
+  const unsigned below = (1u << lane) - 1u;
+  if (__uint_as_float(c[0].y) < cut) list[__popc(m[0] & below)] = c[0];
+  if (__uint_as_float(c[1].y) < cut) list[__popc(m[0]) + __popc(m[1] & below)] = c[1];
+  __syncwarp();
+  uint32_t tri = 0xffffffffu;
+  float d2 = CUDART_INF_F, plane2 = CUDART_INF_F;
+  if (lane < held) {
+    tri = list[lane].x;
+    d2 = __uint_as_float(list[lane].y);
+    plane2 = tri_plane_gap2(g.tris_f, tri, p);
+  }
   best2 = mine;
-  best_tri = tri;
+  if (held == 1u) {
+    best_tri = __shfl_sync(full, tri, 0);
+    return true;
+  }
+  // Replay, by all lanes alike; entries: (node, bound) and the end of the
+  // node's triangle range.
+  float r = cut;
+  int sp = 0, node = root;
+  uint32_t end = 0xffffffffu;
+  for (bool have = true; have;) {
+    if (node < 0) {
+      const uint32_t enc = ~static_cast<uint32_t>(node), first = enc >> 3, last = first + (enc & 7u);
+      for (uint32_t i = first; i < last; ++i) {
+        const unsigned who = __ballot_sync(full, tri == i);
+        if (who == 0u) continue;
+        const int src = __ffs(who) - 1;
+        const float pg = __shfl_sync(full, plane2, src), dd = __shfl_sync(full, d2, src);
+        if (pg < r && dd < r) {
+          r = dd;
+          best_tri = i;
+        }
+      }
+    } else {
+      float dl, dr;
+      int cl, cr;
+      node_dist2(g.nodes_f, node, p, dl, dr, cl, cr);
+      // (An empty right child: all triangles are on the left.)
+      const uint32_t mid = cr >= 0                               ? __ldg(g.node_first + cr)
+                           : (~static_cast<uint32_t>(cr) & 7u) ? ~static_cast<uint32_t>(cr) >> 3
+                                                               : end;
+      const uint32_t begin = cl >= 0 ? __ldg(g.node_first + cl) : ~static_cast<uint32_t>(cl) >> 3;
+      const bool vl = __ballot_sync(full, tri >= begin && tri < mid) != 0u && dl < r;
+      const bool vr = __ballot_sync(full, tri >= mid && tri < end && lane < held) != 0u && dr < r;
+      if (vl || vr) {
+        const bool swap = dr < dl;
+        if (vl && vr) {
+          const int far = swap ? cl : cr;
+          stack[2 * sp] = make_uint2(static_cast<uint32_t>(far), __float_as_uint(swap ? dl : dr));
+          stack[2 * sp + 1].x = swap ? mid : end;
+          ++sp;
+        }
+        const bool left = vl && !(vr && swap);
+        node = left ? cl : cr;
+        if (left) end = mid;
+        continue;
+      }
+    }
+    have = false;
+    while (sp > 0) {
+      --sp;
+      const uint2 e = stack[2 * sp];
+      if (__uint_as_float(e.y) < r) {
+        node = static_cast<int>(e.x);
+        end = stack[2 * sp + 1].x;
+        have = true;
+        break;
+      }
+    }
+  }
+  best2 = r;
   return true;
 }
 
@@ -1834,8 +1977,8 @@ __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<double>
 // their walks; with a warp each the whole call fell from 1.31 to 1.03 ms.
 template <typename T>
 __global__ void __launch_bounds__(kWosBlock) site_prepass_kernel(const WosLaunch L) {
-  __shared__ uint2 s_stack[kWarpStack * (kWosBlock / 32)];
-  uint2 *stack = s_stack + kWarpStack * (threadIdx.x >> 5);
+  __shared__ uint2 s_stack[kWarpEntries * (kWosBlock / 32)];
+  uint2 *stack = s_stack + kWarpEntries * (threadIdx.x >> 5);
   uint32_t err = 0;
   T *out = static_cast<T *>(L.site_best2);
   const uint32_t warps = gridDim.x * (kWosBlock / 32);

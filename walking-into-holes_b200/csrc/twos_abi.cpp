@@ -227,6 +227,10 @@ int open_impl(std::vector<double> &&v, std::vector<uint32_t> &&f, int device, tw
     m->tris_f.reserve(tf.size() * sizeof(TriF));
     m->nodes_d.reserve(nd.size() * sizeof(NodeD));
     m->tris_d.reserve(td.size() * sizeof(TriD));
+    const std::vector<uint32_t> first = node_first_triangles(m->bvh);
+    m->node_first.reserve(first.size() * sizeof(uint32_t));
+    check(cudaMemcpy(m->node_first.ptr, first.data(), first.size() * sizeof(uint32_t), cudaMemcpyHostToDevice),
+          "upload");
     check(cudaMemcpy(m->nodes_f.ptr, nf.data(), nf.size() * sizeof(NodeF), cudaMemcpyHostToDevice), "upload");
     m->nodes4_f.reserve(n4.size() * sizeof(Node4F));
     check(cudaMemcpy(m->nodes4_f.ptr, n4.data(), n4.size() * sizeof(Node4F), cudaMemcpyHostToDevice), "upload");
@@ -235,11 +239,12 @@ int open_impl(std::vector<double> &&v, std::vector<uint32_t> &&f, int device, tw
     check(cudaMemcpy(m->tris_d.ptr, td.data(), td.size() * sizeof(TriD), cudaMemcpyHostToDevice), "upload");
     m->resident_bytes = nf.size() * sizeof(NodeF) + n4.size() * sizeof(Node4F) + tf.size() * sizeof(TriF) +
                         nd.size() * sizeof(NodeD) +
-                        td.size() * sizeof(TriD);
+                        td.size() * sizeof(TriD) + first.size() * sizeof(uint32_t);
     GeoDesc &g = m->geo_host;
     g.nodes_f = m->nodes_f.as<NodeF>();
     g.nodes4_f = m->nodes4_f.as<Node4F>();
     g.tris_f = m->tris_f.as<TriF>();
+    g.node_first = m->node_first.as<uint32_t>();
     g.nodes_d = m->nodes_d.as<NodeD>();
     g.tris_d = m->tris_d.as<TriD>();
     for (int a = 0; a < 3; ++a) g.center[a] = m->center[a];
@@ -667,7 +672,7 @@ void twos_mesh_close(twos_mesh *m) {
   if (m->stream) cudaStreamSynchronize(m->stream);
   for (DevBuf *b : {&m->nodes_f, &m->tris_f, &m->nodes_d, &m->tris_d, &m->geo, &m->jobs, &m->geos, &m->terms, &m->cavities,
                     &m->sites, &m->out, &m->u, &m->p, &m->steps, &m->first, &m->counter, &m->totals, &m->points, &m->dist,
-                    &m->closest, &m->topk, &m->grid, &m->grad, &m->nodes4_f, &m->wf})
+                    &m->closest, &m->topk, &m->grid, &m->grad, &m->nodes4_f, &m->wf, &m->node_first})
     b->release();
   if (m->ev0) cudaEventDestroy(m->ev0);
   if (m->ev1) cudaEventDestroy(m->ev1);

@@ -92,6 +92,8 @@ void build_bvh(const std::vector<double> &vertices, const std::vector<uint32_t> 
 // FP32 triangles exactly.
 void pack_bvh_f32(const HostBvh &bvh, const std::vector<double> &vertices, const std::vector<uint32_t> &faces,
                   const double center[3], std::vector<NodeF> &nodes, std::vector<TriF> &tris);
+// Leaf-order index of every node's first triangle.
+std::vector<uint32_t> node_first_triangles(const HostBvh &bvh);
 void pack_bvh_f64(const HostBvh &bvh, const std::vector<double> &vertices, const std::vector<uint32_t> &faces,
                   std::vector<NodeD> &nodes, std::vector<TriD> &tris);
 
@@ -126,6 +128,7 @@ struct GeoDesc {
   const NodeF *nodes_f;
   const Node4F *nodes4_f;  // the same BVH four wide (mixed form, bvh_width 4)
   const TriF *tris_f;
+  const uint32_t *node_first;  // leaf-order index of each node's first triangle
   const NodeD *nodes_d;
   const TriD *tris_d;
   double center[3];   // FP32 frame origin (mixed form)
