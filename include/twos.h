@@ -163,7 +163,8 @@ typedef struct twos_summary {
   uint64_t queries;        /* closest-point queries = steps + paths (wih_twos.cpp:1779) */
   uint64_t h2d_bytes;
   uint64_t d2h_bytes;
-  uint32_t launches;       /* kernels launched by the call */
+  uint32_t launches;       /* kernel stages of the call (Differential WoS: its four stages, whose
+                              first-query and work-list kernels are not counted) */
   uint32_t error_flags;    /* TWOS_DEVERR_* bits raised on the device */
   uint64_t node_tests;     /* BVH node fetches (two child bounds each) */
   uint64_t plane_tests;    /* triangle plane-slab tests */

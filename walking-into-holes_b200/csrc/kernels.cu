@@ -1258,10 +1258,14 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
           for (int k = 0; k < 6; ++k) static_cast<T *>(L.grad_out)[6ull * id + k] = T(0);
         if (MODE == kModeBoundary) L.hits[id].cavity = -2;
         L.steps_out[id] = 0u;
-      } else if (L.site_best2 && MODE != kModeBoundary) {
+      } else if (L.site_best2 && (MODE != kModeBoundary || L.site_tri)) {
         // First query answered by the per-site pre-pass.
         best2 = static_cast<const T *>(L.site_best2)[J.site_rank + at];
         found = best2 >= T(0);
+        if (MODE == kModeBoundary && found) {
+          best_tri = L.site_tri[J.site_rank + at];
+          tri_ok = true;
+        }
         dcav = CUDART_INF_F;
         phase = J.n_cav ? kFirst : kStep;
       } else {
@@ -1997,7 +2001,10 @@ __global__ void __launch_bounds__(kWosBlock) site_prepass_kernel(const WosLaunch
     T best2 = static_cast<T>(J.query_radius2);
     uint32_t tri = 0;
     const bool found = warp_nearest(G, p, best2, tri, stack, err);
-    if ((threadIdx.x & 31u) == 0) out[g] = found ? best2 : T(-1);
+    if ((threadIdx.x & 31u) == 0) {
+      out[g] = found ? best2 : T(-1);
+      if (L.site_tri) L.site_tri[g] = tri;
+    }
   }
   if (err) atomicOr(L.error, err);
 }

@@ -674,6 +674,7 @@ void twos_mesh_close(twos_mesh *m) {
                     &m->sites, &m->out, &m->u, &m->p, &m->steps, &m->first, &m->counter, &m->totals, &m->points, &m->dist,
                     &m->closest, &m->topk, &m->grid, &m->grad, &m->nodes4_f, &m->wf, &m->node_first})
     b->release();
+  m->scratch.release();
   if (m->ev0) cudaEventDestroy(m->ev0);
   if (m->ev1) cudaEventDestroy(m->ev1);
   if (m->evw) cudaEventDestroy(m->evw);
@@ -989,8 +990,11 @@ int twos_design_loop(twos_mesh *m, const twos_request *scout, const twos_request
   const uint32_t k = P->shortlist;
   const auto t0 = std::chrono::steady_clock::now();
   RunOut ro;
-  DevBuf cand, feas, keys, idx, vsites, rows_s, rows_v, cav, jobs_s, jobs_v, iter, hist, terms_d, topk, dist,
-      first_v;
+  const Scratch::Call scratch_call{m->scratch};
+  DevBuf &cand = m->scratch[0], &feas = m->scratch[1], &keys = m->scratch[2], &idx = m->scratch[3],
+      &vsites = m->scratch[4], &rows_s = m->scratch[5], &rows_v = m->scratch[6], &cav = m->scratch[7],
+      &jobs_s = m->scratch[8], &jobs_v = m->scratch[9], &iter = m->scratch[10], &hist = m->scratch[11],
+      &terms_d = m->scratch[12], &topk = m->scratch[13], &dist = m->scratch[14], &first_v = m->scratch[15];
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   try {
@@ -1181,16 +1185,10 @@ int twos_design_loop(twos_mesh *m, const twos_request *scout, const twos_request
   } catch (const std::exception &e) {
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
-    for (DevBuf *b : {&cand, &feas, &keys, &idx, &vsites, &rows_s, &rows_v, &cav, &jobs_s, &jobs_v, &iter, &hist,
-                      &terms_d, &topk, &dist, &first_v})
-      b->release();
     return fail(TWOS_ERR_RUNTIME, e.what());
   }
   if (exec) cudaGraphExecDestroy(exec);
   if (graph) cudaGraphDestroy(graph);
-  for (DevBuf *b : {&cand, &feas, &keys, &idx, &vsites, &rows_s, &rows_v, &cav, &jobs_s, &jobs_v, &iter, &hist,
-                    &terms_d, &topk, &dist, &first_v})
-    b->release();
   const int rc = finish(ro, 0, &rs, summary, seconds_since(t0), 0, 0);
   if (summary) {
     summary->paths = static_cast<uint64_t>(P->iterations) *
@@ -1242,7 +1240,9 @@ int twos_validate(twos_mesh *m, const twos_request *r, const twos_validate_param
   const auto t0 = std::chrono::steady_clock::now();
   const size_t walks = static_cast<size_t>(r->walks);
   const size_t total = static_cast<size_t>(n_sites) * walks;
-  DevBuf dsamp, dclear, dcenter, dmesh, dterms;
+  const Scratch::Call scratch_call{m->scratch};
+  DevBuf &dsamp = m->scratch[0], &dclear = m->scratch[1], &dcenter = m->scratch[2], &dmesh = m->scratch[3],
+      &dterms = m->scratch[4];
   unsigned long long tot[2] = {0, 0};
   std::vector<double> clearance(n_sites), center(n_sites);
   RunOut ro;
@@ -1310,10 +1310,8 @@ int twos_validate(twos_mesh *m, const twos_request *r, const twos_validate_param
     check(cudaEventElapsedTime(&ms, m->ev0, m->ev1), "event time");
     ro.kernel_seconds = ro.walk_seconds = ms / 1e3;
   } catch (const std::exception &e) {
-    for (DevBuf *b : {&dsamp, &dclear, &dcenter, &dmesh, &dterms}) b->release();
     return fail(TWOS_ERR_RUNTIME, e.what());
   }
-  for (DevBuf *b : {&dsamp, &dclear, &dcenter, &dmesh, &dterms}) b->release();
   // Stage statistics: prefixes n in {1024, 4096, 16384, 65536} below walks,
   // then walks; sums in long double in sample order (minimum_benefit.hpp:160-176).
   std::vector<uint32_t> ns;
@@ -1378,7 +1376,8 @@ int twos_estimate_gradient(twos_mesh *m, const twos_request *r, const double *si
   if (!sites || !out || (n_cav && !cavities)) return fail(TWOS_ERR_USAGE, "null buffer");
   const auto t0 = std::chrono::steady_clock::now();
   RunOut ro;
-  DevBuf rows;
+  const Scratch::Call scratch_call{m->scratch};
+  DevBuf &rows = m->scratch[0];
   try {
     check(cudaSetDevice(m->device), "cudaSetDevice");
     m->sites.reserve(static_cast<size_t>(n_sites) * 3 * sizeof(double));
@@ -1401,10 +1400,8 @@ int twos_estimate_gradient(twos_mesh *m, const twos_request *r, const double *si
           "download rows");
     end_totals(m, ro);
   } catch (const std::exception &e) {
-    rows.release();
     return fail(TWOS_ERR_RUNTIME, e.what());
   }
-  rows.release();
   return finish(ro, n_sites, r, summary, seconds_since(t0), static_cast<uint64_t>(n_sites) * 24,
                 static_cast<uint64_t>(n_sites) * sizeof(twos_gradient_result));
 }
@@ -1454,7 +1451,9 @@ int twos_rqmc(twos_mesh *m, const twos_request *r, const twos_rqmc_params *rp, c
   const bool reuse = rp->method == TWOS_RQMC_NEIGHBOUR;
   const bool rec_first = reuse || rp->walk_first || rp->site_radius, rec_walk = reuse || rp->walk_u || rp->walk_p;
   RunOut ro;
-  DevBuf dterms, du, dp, dfirst, dwu, dwp, drad, dsobol;
+  const Scratch::Call scratch_call{m->scratch};
+  DevBuf &dterms = m->scratch[0], &du = m->scratch[1], &dp = m->scratch[2], &dfirst = m->scratch[3],
+      &dwu = m->scratch[4], &dwp = m->scratch[5], &drad = m->scratch[6], &dsobol = m->scratch[7];
   try {
     check(cudaSetDevice(m->device), "cudaSetDevice");
     if (rp->method == TWOS_RQMC_SOBOL) {
@@ -1543,10 +1542,8 @@ int twos_rqmc(twos_mesh *m, const twos_request *r, const twos_rqmc_params *rp, c
     check(cudaEventElapsedTime(&ms, m->ev0, m->ev1), "event time");
     ro.kernel_seconds = ro.walk_seconds = ms / 1e3;
   } catch (const std::exception &e) {
-    for (DevBuf *b : {&dterms, &du, &dp, &dfirst, &dwu, &dwp, &drad, &dsobol}) b->release();
     return fail(TWOS_ERR_RUNTIME, e.what());
   }
-  for (DevBuf *b : {&dterms, &du, &dp, &dfirst, &dwu, &dwp, &drad, &dsobol}) b->release();
   // Cross-fitting over batches (crossfit, sampling.py:90-92).
   const double R = rp->batches;
   for (uint32_t s = 0; s < n_sites; ++s) {
@@ -1604,7 +1601,10 @@ int twos_diffwos(twos_mesh *m, const twos_request *r, double diff_offset, int en
   const auto t0 = std::chrono::steady_clock::now();
   RunOut ro;
   unsigned long long tot[kDiffTotals] = {};
-  DevBuf hits, osteps, flags, start, nu, nsteps, rows, st, dtot;
+  const Scratch::Call scratch_call{m->scratch};
+  DevBuf &hits = m->scratch[0], &osteps = m->scratch[1], &flags = m->scratch[2], &work = m->scratch[3],
+      &site_tri = m->scratch[4], &start = m->scratch[5], &nu = m->scratch[6], &nsteps = m->scratch[7],
+      &rows = m->scratch[8], &st = m->scratch[9], &dtot = m->scratch[10];
   try {
     check(cudaSetDevice(m->device), "cudaSetDevice");
     const bool mixed = r->precision == TWOS_PREC_MIXED;
@@ -1623,6 +1623,9 @@ int twos_diffwos(twos_mesh *m, const twos_request *r, double diff_offset, int en
     hits.reserve(cw * sizeof(HitRec));
     osteps.reserve(cw * sizeof(uint32_t));
     flags.reserve(cw * sizeof(uint32_t));
+    work.reserve((cw + 1) * sizeof(uint32_t));
+    site_tri.reserve(chunk * sizeof(uint32_t));
+    m->first.reserve(chunk * sizeof(double));
     start.reserve(cw * 3 * sizeof(double));
     nu.reserve(cw * vbytes);
     nsteps.reserve(cw * sizeof(uint32_t));
@@ -1679,7 +1682,9 @@ int twos_diffwos(twos_mesh *m, const twos_request *r, double diff_offset, int en
         L.grid64 = m->grid_fp64;
         L.wide = m->bvh_width == 4;
         L.counters = m->totals.as<unsigned long long>() + 3;
-        L.site_best2 = nullptr;
+        // The outer walks of a site share their first query.
+        L.site_best2 = pass == 0 ? m->first.ptr : nullptr;
+        L.site_tri = pass == 0 ? site_tri.as<uint32_t>() : nullptr;
         L.total_sites = count;
         const int mode = pass == 0 ? kModeBoundary : TWOS_MODE_COMPLIANCE;
         const int green = pass == 1 ? rq->green : TWOS_SOURCE_CENTER;
@@ -1696,6 +1701,9 @@ int twos_diffwos(twos_mesh *m, const twos_request *r, double diff_offset, int en
         const int per_sm = wos_max_blocks_per_sm(r->precision, mode, green, block, L);
         if (per_sm <= 0) throw std::runtime_error("WoS kernel cannot be resident on this device");
         const int grid = std::min(per_sm, m->blocks_per_sm > 0 ? m->blocks_per_sm : per_sm) * m->num_sms;
+        // ro.launches counts the four stages (outer walks, classification,
+        // nested walks, reduction), not the helpers of a stage.
+        if (pass == 0) check(launch_site_prepass(r->precision, L, m->stream), "site pre-pass");
         check(launch_wos(r->precision, mode, green, L, grid, block, m->stream), "walk launch");
         ro.launches += 1;
         if (pass == 0) {
@@ -1710,6 +1718,8 @@ int twos_diffwos(twos_mesh *m, const twos_request *r, double diff_offset, int en
           D.total_walks = cwalks;
           D.hits = hits.as<HitRec>();
           D.outer_steps = osteps.as<uint32_t>();
+          D.work = work.as<uint32_t>();
+          D.work_count = work.as<uint32_t>() + cw;
           D.flags = flags.as<uint32_t>();
           D.start = start.as<double>();
           D.totals = dtot.as<unsigned long long>();
@@ -1745,10 +1755,8 @@ int twos_diffwos(twos_mesh *m, const twos_request *r, double diff_offset, int en
     check(cudaMemcpyAsync(tot, dtot.ptr, sizeof(tot), cudaMemcpyDeviceToHost, m->stream), "download totals");
     end_totals(m, ro);
   } catch (const std::exception &e) {
-    for (DevBuf *b : {&hits, &osteps, &flags, &start, &nu, &nsteps, &rows, &st, &dtot}) b->release();
     return fail(TWOS_ERR_RUNTIME, e.what());
   }
-  for (DevBuf *b : {&hits, &osteps, &flags, &start, &nu, &nsteps, &rows, &st, &dtot}) b->release();
   const double secs = seconds_since(t0);
   // Queries as the study backend counts them: one closest-point query per
   // step of the outer and nested walks plus the terminal one of every walk

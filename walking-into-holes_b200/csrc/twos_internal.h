@@ -217,6 +217,7 @@ struct WosLaunch {
   // the pre-pass; every walk of a site starts from the same point, so its
   // first query is answered from here (-1 when nothing is within range).
   void *site_best2;
+  uint32_t *site_tri;  // its nearest triangle (boundary mode; may be null otherwise)
   uint32_t total_sites;
   int vote;  // 1: a warp runs one kind of traversal unit per iteration (majority vote)
   // 1: a step's query starts from the distance to the previous query's
@@ -353,6 +354,8 @@ struct DiffLaunch {
   uint32_t n_sites, walks, site_begin;
   const HitRec *hits;             // outer walks' terminal hits
   const uint32_t *outer_steps;    // steps | cap << 31
+  uint32_t *work;                 // walks that ended on a cavity (total_walks entries)
+  uint32_t *work_count;
   uint32_t *flags;                // kDiff* per walk
   double *start;                  // nested start points [walks][3] (NaN = none)
   const void *nested_u;           // nested walk values (float or double)

@@ -36,6 +36,32 @@ struct DevBuf {
   template <typename T> T *as() const { return static_cast<T *>(ptr); }
 };
 
+// A session's buffers for the calls that need them only while they run
+// (Differential WoS, RQMC, validation, the design loop): kept from one call to
+// the next, since allocating and freeing a dozen buffers took 2 to 8 ms of a
+// call and waited for the device each time.  trim(), at the end of a call,
+// gives back what is larger than kKeepBytes, so a session holds at most
+// kScratch * kKeepBytes; closing it frees the rest.  A session's calls run one
+// at a time on its stream and wait for it before they return.
+constexpr int kScratch = 18;
+constexpr size_t kKeepBytes = size_t(32) << 20;
+struct Scratch {
+  DevBuf buf[kScratch];
+  DevBuf &operator[](int i) { return buf[i]; }
+  void trim() {
+    for (DevBuf &b : buf)
+      if (b.bytes > kKeepBytes) b.release();
+  }
+  void release() {
+    for (DevBuf &b : buf) b.release();
+  }
+  // Trims at the end of the call that holds it, however it ends.
+  struct Call {
+    Scratch &s;
+    ~Call() { s.trim(); }
+  };
+};
+
 // What a group of launches reports back to the entry point that ran them.
 struct RunOut {
   double kernel_seconds = 0.0;
@@ -79,6 +105,7 @@ struct twos_mesh {
   // Scratch, grown on demand.
   twos::DevBuf jobs, geos, terms, cavities, sites, out, u, p, grad, steps, first, counter, totals, points, dist, closest,
       topk, wf;
+  twos::Scratch scratch;
   size_t max_launch_walks = size_t(1) << 30;
   int block = 128;         // walk-kernel threads per block
   int refill = 1;          // lanes idle before a warp refills from the queue
