@@ -152,9 +152,9 @@ def test_first_queries_among_equidistant_triangles(tb, oracle_mod, level, query_
 @pytest.mark.parametrize("shape", ["tetra", "sphere1", "sphere5", "noise6", "fan5", "fan64", "sliver"])
 def test_first_queries_return_the_traversals_value(tb, shape):
     """A site's first distance, found by a whole warp, is the one a lane's
-    traversal returns, to the last bit: mixed walks that start at the sites
-    against the same walks started by a traversal (the cap of one step makes a
-    walk's value its first radius)."""
+    traversal returns, to the last bit (the cap of one step makes a walk's
+    value its first radius; a bulk closest-point call takes a lane per point,
+    a small one a warp)."""
     rng = np.random.default_rng(5)
     if shape == "tetra":
         V = np.array([[0.0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1]]) - 0.25
@@ -172,7 +172,12 @@ def test_first_queries_return_the_traversals_value(tb, shape):
     P = np.concatenate([mid[rng.integers(0, len(mid), 2000)] * rng.uniform(0.0, 0.9, (2000, 1)),
                         V[rng.integers(0, len(V), 300)] * rng.uniform(0.0, 0.95, (300, 1)), np.zeros((1, 3))])
     with tb.Mesh(V, F) as m:
-        d = m.closest_point(P, precision="mixed", with_points=False)  # one lane per point
+        d = m.closest_point(np.tile(P, (9, 1)), precision="mixed", with_points=False)  # a lane per point
+        assert np.array_equal(d, np.tile(d[: len(P)], 9))
+        d = d[: len(P)]
+        assert np.array_equal(d, m.closest_point(P, precision="mixed", with_points=False))  # a warp per point
+        d64 = m.closest_point(np.tile(P, (9, 1)), precision="fp64", with_points=False)
+        assert np.array_equal(d64, np.tile(m.closest_point(P, precision="fp64", with_points=False), 9))
         delta = np.float32(m.info()["mixed_delta"])
         cfg = tb.Config(walks=2, precision="mixed", seed=3, epsilon=1e-30, max_steps=1, query_radius=None,
                         source=tb.sources.constant(6.0))

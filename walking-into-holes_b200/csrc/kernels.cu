@@ -1817,7 +1817,7 @@ template <typename T> __device__ __forceinline__ void warp_best(T &best, uint32_
 // delta / 2, so no other one can change the outcome), and if there are
 // several, replays the lane's traversal on the nodes that hold them
 // (node_first: a node's first triangle), which are few.
-constexpr int kContend = 64;
+constexpr int kContend = 256;
 constexpr int kWarpEntries = kWarpStack + kContend + 1;  // shared-memory entries per warp
 __device__ __forceinline__ float widen2(float d2, float by) {
   const float t = __fadd_ru(__fsqrt_ru(d2), by);
@@ -1848,24 +1848,24 @@ __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<float> 
   // The contenders, one per lane.
   const float cut = fminf(best2, widen2(mine, 3.f * g.delta));
   const uint32_t n = *count;
-  uint2 c[2];
-  unsigned m[2];
-  for (uint32_t k = 0; k < 2; ++k) {
-    c[k] = make_uint2(0xffffffffu, 0x7f800000u);
-    if (lane + 32 * k < min(n, static_cast<uint32_t>(kContend))) c[k] = list[lane + 32 * k];
-    m[k] = __ballot_sync(full, __uint_as_float(c[k].y) < cut);
+  uint32_t held = 0;
+  if (n <= kContend) {
+    for (uint32_t k = 0; k < n; k += 32) {  // in place: an entry moves only forward
+      uint2 c = make_uint2(0u, 0x7f800000u);
+      if (k + lane < n) c = list[k + lane];
+      const bool keep = __uint_as_float(c.y) < cut;
+      const unsigned m = __ballot_sync(full, keep);
+      __syncwarp();
+      if (keep) list[held + __popc(m & ((1u << lane) - 1u))] = c;
+      held += __popc(m);
+      __syncwarp();
+    }
   }
-  const uint32_t held = __popc(m[0]) + __popc(m[1]);
-  __syncwarp();
   if (n > kContend || held > 32u) {
     // Too many to replay: the traversal itself, below the cut.
     best2 = cut;
     return nearest<float>(g.nodes_f, g.tris_f, g.max_iter, p, best2, best_tri, stack, 1, err, root);
   }
-  const unsigned below = (1u << lane) - 1u;
-  if (__uint_as_float(c[0].y) < cut) list[__popc(m[0] & below)] = c[0];
-  if (__uint_as_float(c[1].y) < cut) list[__popc(m[0]) + __popc(m[1] & below)] = c[1];
-  __syncwarp();
   uint32_t tri = 0xffffffffu;
   float d2 = CUDART_INF_F, plane2 = CUDART_INF_F;
   if (lane < held) {
@@ -2429,37 +2429,213 @@ cudaError_t launch_l2_read(const void *buf, uint64_t bytes, int passes, uint32_t
 }
 
 // ================================================================ batched closest point
+// The result of point i: distance (infinite when nothing is within the query
+// radius) and, if wanted, the nearest point.
 template <typename T>
-__global__ void __launch_bounds__(kWosBlock) closest_kernel(const GeoDesc *geo, const double *pts, uint64_t n,
-                                                            double query_radius2, double *dist, double *closest,
-                                                            uint32_t *error) {
-  __shared__ uint2 s_stack[(kStack + kCand) * kWosBlock];
+__device__ __forceinline__ void closest_store(const GeoDesc &G, const Vec<T> &p, bool found, T best2, uint32_t best_tri,
+                                              uint64_t i, double *dist, double *closest) {
+  dist[i] = found ? static_cast<double>(sqrt(best2)) : CUDART_INF;
+  if (!closest) return;
+  double q[3] = {CUDART_NAN, CUDART_NAN, CUDART_NAN};
+  if (found) {
+    Vec<T> a, b, c;
+    load_tri(geo_tris<T>(G), best_tri, a, b, c);
+    const Vec<T> cp = tri_closest(p, a, b, c);
+    const bool f32 = sizeof(T) == 4;
+    q[0] = static_cast<double>(cp.x) + (f32 ? G.center[0] : 0.0);
+    q[1] = static_cast<double>(cp.y) + (f32 ? G.center[1] : 0.0);
+    q[2] = static_cast<double>(cp.z) + (f32 ? G.center[2] : 0.0);
+  }
+  for (int a = 0; a < 3; ++a) closest[3 * i + a] = q[a];
+}
+
+// A warp per point: a call with few points is as long as its longest query,
+// and a lane alone waits for memory at every node (3,000 points, 81,920
+// triangles, FP64: 1.70 ms with a lane each, 0.20 with a warp).
+template <typename T>
+__global__ void __launch_bounds__(kWosBlock) closest_warp_kernel(const GeoDesc *geo, const double *pts, uint64_t n,
+                                                                 double query_radius2, double *dist, double *closest,
+                                                                 uint32_t *error) {
+  __shared__ uint2 s_stack[kWarpEntries * (kWosBlock / 32)];
   __shared__ GeoDesc G;
   if (threadIdx.x == 0) G = *geo;
   __syncthreads();
   uint32_t err = 0;
-  uint2 *stack = s_stack + threadIdx.x;
-  for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+  uint2 *stack = s_stack + kWarpEntries * (threadIdx.x >> 5);
+  const uint64_t warps = static_cast<uint64_t>(gridDim.x) * (kWosBlock / 32);
+  for (uint64_t i = blockIdx.x * (kWosBlock / 32) + (threadIdx.x >> 5); i < n; i += warps) {
     const Vec<T> p = to_frame<T>(pts + 3 * i, G);
     T best2 = static_cast<T>(query_radius2);
     uint32_t best_tri = 0;
-    const bool found = nearest_geo(G, p, best2, best_tri, stack, kWosBlock, err);
-    dist[i] = found ? static_cast<double>(sqrt(best2)) : CUDART_INF;
-    if (closest) {
-      double q[3] = {CUDART_NAN, CUDART_NAN, CUDART_NAN};
-      if (found) {
-        Vec<T> a, b, c;
-        load_tri(geo_tris<T>(G), best_tri, a, b, c);
-        const Vec<T> cp = tri_closest(p, a, b, c);
-        const bool f32 = sizeof(T) == 4;
-        q[0] = static_cast<double>(cp.x) + (f32 ? G.center[0] : 0.0);
-        q[1] = static_cast<double>(cp.y) + (f32 ? G.center[1] : 0.0);
-        q[2] = static_cast<double>(cp.z) + (f32 ? G.center[2] : 0.0);
+    const bool found = warp_nearest(G, p, best2, best_tri, stack, err);
+    if ((threadIdx.x & 31u) == 0) closest_store(G, p, found, best2, best_tri, i, dist, closest);
+  }
+  if (err) atomicOr(error, err);
+}
+
+// A point per lane, for many points: as the walk kernel, a lane runs units of
+// its search, one set of loads per unit, and takes the next point from the
+// queue when it ends, so a warp does not wait for its longest query (call of
+// 122,591 points, 81,920 triangles, FP64: 3.1 ms with a fixed point per
+// thread, 1.9 with the queue).
+template <typename T>
+__global__ void __launch_bounds__(kWosBlock) closest_kernel(const GeoDesc *geo, const double *pts, uint64_t n,
+                                                            double query_radius2, double *dist, double *closest,
+                                                            unsigned long long *counter, uint32_t *error) {
+  constexpr int kLaneStack = 8;
+  __shared__ uint2 s_stack[(kLaneStack + kCand) * kWosBlock];
+  __shared__ GeoDesc G;
+  if (threadIdx.x == 0) G = *geo;
+  __syncthreads();
+  uint2 *stack = s_stack + threadIdx.x, *cand = stack + kLaneStack * kWosBlock;
+  uint2 deep[kStack - kLaneStack];
+  const unsigned lane = threadIdx.x & 31u, full = 0xffffffffu;
+  uint32_t err = 0;
+  uint64_t i = 0;
+  Vec<T> p{T(0), T(0), T(0)};
+  Cull c{{0.f, 0.f, 0.f}, 0.f, 0.f, 0};  // FP32: p and the threshold best2
+  T best2 = T(0);
+  uint32_t best_tri = 0, tri_cur = 0, tri_end = 0, iter = 0;
+  int node = 0, sp = 0;
+  bool have = false, found = false, exhausted = false;  // exhausted is warp-uniform
+  int phase = kIdle;
+  for (;;) {
+    if (phase == kStep) {
+      if constexpr (sizeof(T) == 8) found |= cull_flush(G, p, c, best2, best_tri, cand, kWosBlock);
+      if (have || tri_cur < tri_end || sp > 0) {
+        phase = kTraverse;  // the candidate list was full: the search goes on
+      } else {
+        closest_store(G, p, found, best2, best_tri, i, dist, closest);
+        phase = kIdle;
       }
-      closest[3 * i] = q[0];
-      closest[3 * i + 1] = q[1];
-      closest[3 * i + 2] = q[2];
+    }
+    const unsigned idle = __ballot_sync(full, phase == kIdle);
+    if (!exhausted && idle != 0u) {
+      unsigned long long base = 0;
+      const int leader = __ffs(idle) - 1;
+      if (static_cast<int>(lane) == leader) base = atomicAdd(counter, static_cast<unsigned long long>(__popc(idle)));
+      base = __shfl_sync(full, base, leader);
+      if (base + __popc(idle) >= n) exhausted = true;
+      const uint64_t next = base + __popc(idle & ((1u << lane) - 1u));
+      if (phase == kIdle && next < n) {
+        i = next;
+        p = to_frame<T>(pts + 3 * i, G);
+        best2 = static_cast<T>(query_radius2);
+        found = false;
+        sp = 0;
+        tri_cur = tri_end = iter = 0;
+        bool search = true;
+        if constexpr (sizeof(T) == 4) {
+          c.p = p;
+        } else {
+          if (!cull_begin(G, p, best2, c)) {
+            const Plain64 r = nearest_plain64(&G, p.x, p.y, p.z, best2);
+            err |= r.flags & 0x7fffffffu;
+            found = r.flags >> 31;
+            best2 = r.best2;
+            best_tri = r.tri;
+            have = search = false;
+            phase = kStep;
+          }
+        }
+        if (search) {
+          float upper;
+          if constexpr (sizeof(T) == 4) {
+            grid_start(G, c.p, sqrtf(best2), upper, node);
+            best2 = fminf(best2, upper * upper);
+          } else {
+            grid_start(G, c.p, sqrtf(c.limit), upper, node);
+            const float reach = __fadd_ru(upper, c.margin);
+            c.limit = fminf(c.limit, __fmul_ru(reach, reach));
+          }
+          have = true;
+          phase = kTraverse;
+        }
+      }
+    }
+    if (__ballot_sync(full, phase != kIdle) == 0u) {
+      if (exhausted) break;
+      continue;
+    }
+    if (phase != kTraverse) continue;
+#pragma unroll 1
+    for (int unit = 0; unit < 8; ++unit) {
+      const float limit = [&]() -> float {
+        if constexpr (sizeof(T) == 4)
+          return best2;
+        else
+          return c.limit;
+      }();
+      if (tri_cur >= tri_end) {
+        while (!have && sp > 0) {
+          --sp;
+          const uint2 e = sp < kLaneStack ? stack[sp * kWosBlock] : deep[sp - kLaneStack];
+          if (__uint_as_float(e.y) < limit) {
+            node = static_cast<int>(e.x);
+            have = true;
+          }
+        }
+        if (!have) {
+          phase = kStep;
+          break;
+        }
+        if (node < 0) {
+          const uint32_t enc = ~static_cast<uint32_t>(node);
+          tri_cur = enc >> 3;
+          tri_end = tri_cur + (enc & 7u);
+          have = false;
+        }
+      }
+      if (++iter > G.max_iter || sp >= kStack) {
+        err |= sp >= kStack ? TWOS_DEVERR_STACK : TWOS_DEVERR_ITER;
+        have = false;
+        sp = 0;
+        tri_cur = tri_end;
+        phase = kStep;
+        break;
+      }
+      const bool on_tri = tri_cur < tri_end;
+      const char *at = on_tri ? reinterpret_cast<const char *>(G.tris_f + tri_cur)
+                              : reinterpret_cast<const char *>(G.nodes_f + node);
+      float4 r0, r1, r2, r3, r4{}, r5{};
+      ldg32(at, r0, r1);
+      ldg32(at + 32, r2, r3);
+      ldg32_if(!on_tri, at + 64, r4, r5);
+      if (on_tri) {
+        if constexpr (sizeof(T) == 4) {
+          if (plane_gap2(r0, r1, c.p) < best2) {
+            const float d2 = tri_dist2(c.p, Vec<float>{r1.x, r1.y, r1.z}, Vec<float>{r2.x, r2.y, r2.z},
+                                       Vec<float>{r3.x, r3.y, r3.z});
+            if (d2 < best2) {
+              best2 = d2;
+              best_tri = tri_cur;
+              found = true;
+            }
+          }
+        } else {
+          uint32_t full_tests = 0;
+          if (cull_tri(tri_cur, r0, r1, r2, r3, c, cand, kWosBlock, full_tests)) {
+            phase = kStep;  // a full candidate list is tested first; the triangle comes again
+            break;
+          }
+        }
+        ++tri_cur;
+      } else {
+        float dl, dr;
+        int cl, cr;
+        node_bounds(r0, r1, r2, r3, r4, r5, c.p, dl, dr, cl, cr);
+        const bool vl = dl < limit, vr = dr < limit, swap = dr < dl;
+        if (vl && vr) {
+          const uint2 e = make_uint2(static_cast<uint32_t>(swap ? cl : cr), __float_as_uint(swap ? dl : dr));
+          if (sp < kLaneStack)
+            stack[sp * kWosBlock] = e;
+          else
+            deep[sp - kLaneStack] = e;
+          ++sp;
+        }
+        have = vl || vr;
+        node = vl && !(vr && swap) ? cl : cr;
+      }
     }
   }
   if (err) atomicOr(error, err);
@@ -2484,15 +2660,33 @@ cudaError_t launch_ball_green(const double *cases, uint32_t n, double *out, uint
   return cudaGetLastError();
 }
 
+// Points up to which each gets a warp.  The warp's search costs more
+// instructions in all, so it wins where a call is as long as its longest query
+// (calls, ms, lane / warp, FP64, 327,680 triangles: 3,000 points of the solid
+// 3.6 / 0.28, 30,000 2.4 / 1.3, 122,591 3.5 / 3.8; 30,000 near the surface
+// 0.26 / 0.32).
+constexpr uint64_t kWarpPoints = 16384;
+
 cudaError_t launch_closest(int precision, const GeoDesc *geo_dev, const double *pts, uint64_t n,
-                           double query_radius2, double *dist, double *closest, uint32_t *error, cudaStream_t s) {
+                           double query_radius2, double *dist, double *closest, unsigned long long *counter,
+                           uint32_t *error, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   const int block = kWosBlock;
-  const int grid = static_cast<int>(std::min<uint64_t>((n + block - 1) / block, 148ull * 32));
+  if (n <= kWarpPoints) {
+    const int grid = static_cast<int>((n + block / 32 - 1) / (block / 32));
+    if (precision == TWOS_PREC_MIXED)
+      closest_warp_kernel<float><<<grid, block, 0, s>>>(geo_dev, pts, n, query_radius2, dist, closest, error);
+    else
+      closest_warp_kernel<double><<<grid, block, 0, s>>>(geo_dev, pts, n, query_radius2, dist, closest, error);
+    return cudaGetLastError();
+  }
+  const cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s);
+  if (e != cudaSuccess) return e;
+  const int grid = static_cast<int>(std::min<uint64_t>((n + block - 1) / block, 148ull * 8));
   if (precision == TWOS_PREC_MIXED)
-    closest_kernel<float><<<grid, block, 0, s>>>(geo_dev, pts, n, query_radius2, dist, closest, error);
+    closest_kernel<float><<<grid, block, 0, s>>>(geo_dev, pts, n, query_radius2, dist, closest, counter, error);
   else
-    closest_kernel<double><<<grid, block, 0, s>>>(geo_dev, pts, n, query_radius2, dist, closest, error);
+    closest_kernel<double><<<grid, block, 0, s>>>(geo_dev, pts, n, query_radius2, dist, closest, counter, error);
   return cudaGetLastError();
 }
 

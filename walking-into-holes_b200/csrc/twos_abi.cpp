@@ -767,7 +767,8 @@ int twos_closest_point(twos_mesh *m, int precision, const double *points, uint64
     const double qr = query_radius > 0.0 ? query_radius : std::numeric_limits<double>::infinity();
     uint32_t *err = reinterpret_cast<uint32_t *>(m->totals.as<unsigned long long>() + 2);
     check(launch_closest(precision, m->geo.as<GeoDesc>(), m->points.as<double>(), n, qr * qr,
-                         m->dist.as<double>(), closest ? m->closest.as<double>() : nullptr, err, m->stream),
+                         m->dist.as<double>(), closest ? m->closest.as<double>() : nullptr,
+                         m->counter.as<unsigned long long>(), err, m->stream),
           "closest launch");
     check(cudaMemcpyAsync(distance, m->dist.ptr, n * sizeof(double), cudaMemcpyDeviceToHost, m->stream),
           "download");
@@ -1007,6 +1008,7 @@ int twos_design_loop(twos_mesh *m, const twos_request *scout, const twos_request
     dist.reserve(static_cast<size_t>(n) * sizeof(double));
     check(launch_closest(TWOS_PREC_FP64, m->geo.as<GeoDesc>(), cand.as<double>(), n,
                          std::numeric_limits<double>::infinity(), dist.as<double>(), nullptr,
+                         m->counter.as<unsigned long long>(),
                          reinterpret_cast<uint32_t *>(m->totals.as<unsigned long long>() + 2), m->stream),
           "closest launch");
     std::vector<double> d(n);

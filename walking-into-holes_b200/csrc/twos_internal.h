@@ -463,7 +463,8 @@ cudaError_t launch_ball_green(const double *cases, uint32_t n, double *out, uint
 // L2 read probe: `passes` sweeps of 32-byte loads over `bytes` of buf.
 cudaError_t launch_l2_read(const void *buf, uint64_t bytes, int passes, uint32_t *sink, int blocks, cudaStream_t s);
 cudaError_t launch_closest(int precision, const GeoDesc *geo_dev, const double *pts, uint64_t n,
-                           double query_radius2, double *dist, double *closest, uint32_t *error, cudaStream_t s);
+                           double query_radius2, double *dist, double *closest, unsigned long long *counter,
+                           uint32_t *error, cudaStream_t s);
 // Fills a geometry's distance-bound grid (n = vertices of the grid described
 // in *geo_dev; its `grid` pointer is not read).
 cudaError_t launch_grid_build(const GeoDesc *geo_dev, uint64_t n, double margin, uint16_t *out, uint32_t *error,
