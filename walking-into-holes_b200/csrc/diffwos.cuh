@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(256) diff_list_kernel(const DiffLaunch D) {
 }
 
 __global__ void __launch_bounds__(128) diff_classify_kernel(const DiffLaunch D) {
-  __shared__ uint2 s_stack[(kStack + kCand) * 128];
+  __shared__ uint2 s_stack[near_entries<double>() * 128];
   uint2 *stack = s_stack + threadIdx.x;
   const GeoDesc G = *D.geo;
   uint32_t err = 0;

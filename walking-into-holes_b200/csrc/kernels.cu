@@ -782,92 +782,120 @@ __device__ __noinline__ Plain64 nearest_plain64(const GeoDesc *g, double x, doub
   return r;
 }
 
-// Closest-point query outside the walk kernel, as nearest(), with the
-// distance grid's bound and entry node; the FP64 form culls in FP32.
-__device__ __forceinline__ bool nearest_geo(const GeoDesc &g, const Vec<float> &p, float &best2, uint32_t &best_tri,
-                                            uint2 *stack, int stride, uint32_t &err) {
-  float upper;
-  int node;
-  grid_start(g, p, sqrtf(best2), upper, node);
-  if (upper * upper < best2) best2 = upper * upper;
-  return nearest<float>(g.nodes_f, g.tris_f, g.max_iter, p, best2, best_tri, stack, stride, err, node);
+// Closest-point query outside the walk kernel, as nearest(), from the distance
+// grid's bound and entry node; the FP64 form searches in FP32.  A loop of
+// units with one set of loads for nodes and triangles, as the walk kernel's.
+// `stack`: this thread's column of kNearShared traversal entries and, in the
+// FP64 form, kCand candidates; deeper entries are local.
+constexpr int kNearShared = 8;
+template <typename T> __host__ __device__ constexpr int near_entries() {
+  return kNearShared + (sizeof(T) == 8 ? kCand : 0);
 }
-
-__device__ __forceinline__ bool nearest_geo(const GeoDesc &g, const Vec<double> &p, double &best2,
-                                            uint32_t &best_tri, uint2 *stack, int stride, uint32_t &err) {
-  Cull c;
-  if (!cull_begin(g, p, best2, c)) {
-    const Plain64 r = nearest_plain64(&g, p.x, p.y, p.z, best2);
-    err |= r.flags & 0x7fffffffu;
-    if (!(r.flags >> 31)) return false;
-    best2 = r.best2;
-    best_tri = r.tri;
-    return true;
-  }
+template <typename T>
+__device__ __forceinline__ bool nearest_geo(const GeoDesc &g, const Vec<T> &p, T &best2, uint32_t &best_tri,
+                                            uint2 *stack, int stride, uint32_t &err) {
+  Cull c{{0.f, 0.f, 0.f}, 0.f, 0.f, 0};
+  uint2 *cand = stack + kNearShared * stride;
+  uint2 deep[kStack - kNearShared];
   float upper;
-  int node;
-  grid_start(g, c.p, sqrtf(c.limit), upper, node);
-  const float reach = __fadd_ru(upper, c.margin);
-  c.limit = fminf(c.limit, __fmul_ru(reach, reach));
-  bool found = false;
-  int sp = 0;
-  uint32_t iter = 0;
-  for (bool have = true; have;) {
-    if (++iter > g.max_iter) {
-      err |= TWOS_DEVERR_ITER;
-      break;
+  int node, sp = 0;
+  bool found = false, have = true;
+  if constexpr (sizeof(T) == 4) {
+    c.p = p;
+    grid_start(g, c.p, sqrtf(best2), upper, node);
+    best2 = fminf(best2, upper * upper);
+  } else {
+    if (!cull_begin(g, p, best2, c)) {
+      const Plain64 r = nearest_plain64(&g, p.x, p.y, p.z, best2);
+      err |= r.flags & 0x7fffffffu;
+      if (!(r.flags >> 31)) return false;
+      best2 = r.best2;
+      best_tri = r.tri;
+      return true;
     }
-    if (node >= 0) {
-      float dl, dr;
-      int cl, cr;
-      node_dist2(g.nodes_f, node, c.p, dl, dr, cl, cr);
-      const bool vl = dl < c.limit, vr = dr < c.limit;
-      if (vl && vr) {
-        if (dr < dl) {
-          const float td = dl;
-          dl = dr;
-          dr = td;
-          const int tc = cl;
-          cl = cr;
-          cr = tc;
-        }
-        if (sp >= kStack) {
-          err |= TWOS_DEVERR_STACK;
-          break;
-        }
-        stack[sp * stride] = make_uint2(static_cast<uint32_t>(cr), __float_as_uint(dr));
-        ++sp;
-        node = cl;
-        continue;
-      }
-      if (vl || vr) {
-        node = vl ? cl : cr;
-        continue;
-      }
-    } else {
-      const uint32_t enc = ~static_cast<uint32_t>(node);
-      for (uint32_t i = enc >> 3, e = (enc >> 3) + (enc & 7u), full = 0; i < e; ++i) {
-        float4 P, A, B, C;
-        ldg32(&g.tris_f[i].plane, P, A);
-        ldg32(&g.tris_f[i].b, B, C);
-        if (cull_tri(i, P, A, B, C, c, stack + kStack * stride, stride, full)) {
-          found |= cull_flush(g, p, c, best2, best_tri, stack + kStack * stride, stride);
-          --i;
-        }
-      }
-    }
-    have = false;
-    while (sp > 0) {
-      --sp;
-      const uint2 e = stack[sp * stride];
-      if (__uint_as_float(e.y) < c.limit) {
-        node = static_cast<int>(e.x);
-        have = true;
-        break;
-      }
-    }
+    grid_start(g, c.p, sqrtf(c.limit), upper, node);
+    const float reach = __fadd_ru(upper, c.margin);
+    c.limit = fminf(c.limit, __fmul_ru(reach, reach));
   }
-  found |= cull_flush(g, p, c, best2, best_tri, stack + kStack * stride, stride);
+  uint32_t tri_cur = 0, tri_end = 0, iter = 0;
+#pragma unroll 1
+  for (;;) {
+    const float limit = [&]() -> float {
+      if constexpr (sizeof(T) == 4)
+        return best2;
+      else
+        return c.limit;
+    }();
+    bool flush = false, done = false;
+    if (tri_cur >= tri_end) {
+      while (!have && sp > 0) {
+        --sp;
+        const uint2 e = sp < kNearShared ? stack[sp * stride] : deep[sp - kNearShared];
+        if (__uint_as_float(e.y) < limit) {
+          node = static_cast<int>(e.x);
+          have = true;
+        }
+      }
+      done = !have;
+      if (have && node < 0) {
+        const uint32_t enc = ~static_cast<uint32_t>(node);
+        tri_cur = enc >> 3;
+        tri_end = tri_cur + (enc & 7u);
+        have = false;
+      }
+    }
+    if (!done && (++iter > g.max_iter || sp >= kStack)) {
+      err |= sp >= kStack ? TWOS_DEVERR_STACK : TWOS_DEVERR_ITER;
+      done = true;
+    }
+    if (!done) {
+      const bool on_tri = tri_cur < tri_end;
+      const char *at = on_tri ? reinterpret_cast<const char *>(g.tris_f + tri_cur)
+                              : reinterpret_cast<const char *>(g.nodes_f + node);
+      float4 r0, r1, r2, r3, r4{}, r5{};
+      ldg32(at, r0, r1);
+      ldg32(at + 32, r2, r3);
+      ldg32_if(!on_tri, at + 64, r4, r5);
+      if (on_tri) {
+        if constexpr (sizeof(T) == 4) {
+          if (plane_gap2(r0, r1, c.p) < best2) {
+            const float d2 = tri_dist2(c.p, Vec<float>{r1.x, r1.y, r1.z}, Vec<float>{r2.x, r2.y, r2.z},
+                                       Vec<float>{r3.x, r3.y, r3.z});
+            if (d2 < best2) {
+              best2 = d2;
+              best_tri = tri_cur;
+              found = true;
+            }
+          }
+          ++tri_cur;
+        } else {
+          // A full candidate list is tested first; the triangle comes again.
+          uint32_t full = 0;
+          flush = cull_tri(tri_cur, r0, r1, r2, r3, c, cand, stride, full);
+          if (!flush) ++tri_cur;
+        }
+      } else {
+        float dl, dr;
+        int cl, cr;
+        node_bounds(r0, r1, r2, r3, r4, r5, c.p, dl, dr, cl, cr);
+        const bool vl = dl < limit, vr = dr < limit, swap = dr < dl;
+        if (vl && vr) {
+          const uint2 e = make_uint2(static_cast<uint32_t>(swap ? cl : cr), __float_as_uint(swap ? dl : dr));
+          if (sp < kNearShared)
+            stack[sp * stride] = e;
+          else
+            deep[sp - kNearShared] = e;
+          ++sp;
+        }
+        have = vl || vr;
+        node = vl && !(vr && swap) ? cl : cr;
+      }
+    }
+    if constexpr (sizeof(T) == 8) {
+      if (flush || done) found |= cull_flush(g, p, c, best2, best_tri, cand, stride);
+    }
+    if (done) break;
+  }
   return found;
 }
 

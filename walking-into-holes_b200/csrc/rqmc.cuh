@@ -5,7 +5,8 @@
 //
 // One block per (site, batch), one thread per walk; all walks of the block
 // take their steps together.  At each step a thread answers its walk's
-// closest-point query (nearest_geo, stack in local memory); walks within
+// closest-point query (nearest_geo; at the first step, where all walks stand at
+// the site, warp 0 answers for all); walks within
 // epsilon stop and add the boundary data at their exit point; then, in
 // ARRAY mode, the block sorts (Hilbert key, thread) pairs with a bitonic
 // network in shared memory and the walk of rank i takes the Korobov lattice
@@ -71,9 +72,23 @@ template <typename T> __device__ __forceinline__ TermT<T> to_termT(const TermDev
 
 }  // namespace
 
-template <typename T> __global__ void __launch_bounds__(1024) rqmc_kernel(const RqmcLaunch R) {
-  extern __shared__ unsigned long long s_keys[];  // [walks] (key << 32 | thread), then ranks
-  uint32_t *s_rank = reinterpret_cast<uint32_t *>(s_keys + R.walks);
+// Shared-memory entries for the block's searches: a column per walk, or the
+// first step's warp search.
+template <typename T> __host__ __device__ inline uint32_t rqmc_near_entries(uint32_t walks) {
+  const uint32_t columns = near_entries<T>() * walks;
+  return columns > static_cast<uint32_t>(kWarpEntries) ? columns : static_cast<uint32_t>(kWarpEntries);
+}
+
+// BLOCK: most walks of an instantiation.  Up to 256 walks a thread has 80
+// registers (three blocks per SM); the 64 that 1,024 threads leave spill the
+// FP64 search.
+template <typename T, int BLOCK>
+__global__ void __launch_bounds__(BLOCK, BLOCK <= 256 ? 3 : 1) rqmc_kernel(const RqmcLaunch R) {
+  extern __shared__ unsigned long long s_keys[];  // [walks] (key << 32 | thread), search stacks, then ranks
+  uint2 *s_near = reinterpret_cast<uint2 *>(s_keys + R.walks);
+  uint32_t *s_rank = reinterpret_cast<uint32_t *>(s_near + rqmc_near_entries<T>(R.walks));
+  __shared__ T s_first;
+  __shared__ uint32_t s_first_tri;
   __shared__ TermT<T> s_terms[3 * TWOS_MAX_TERMS];
   __shared__ double s_red[32][2];
   // SOBOL: one step's scrambling (lower-triangular matrix rows and digital
@@ -89,14 +104,26 @@ template <typename T> __global__ void __launch_bounds__(1024) rqmc_kernel(const 
   bool active = true, cap = false;
   uint32_t steps = 0, err = 0;
   double vu = 0.0, vp = 0.0;
-  uint2 lstack[kStack + kCand];
+  uint2 *stack = s_near + tid;
   const uint32_t ctr3 = (batch << 16) | (R.repeat << 3);
   for (int k = 0; k < R.max_steps; ++k) {
     T r = T(0);
+    if (k == 0) {
+      if (tid < 32u) {
+        T best2 = static_cast<T>(CUDART_INF);
+        uint32_t tri = 0;
+        const bool found = warp_nearest(G, pos, best2, tri, s_near, err);
+        if (tid == 0) {
+          s_first = found ? best2 : T(-1);
+          s_first_tri = tri;
+        }
+      }
+      __syncthreads();
+    }
     if (active) {
-      T best2 = static_cast<T>(CUDART_INF);
-      uint32_t tri = 0;
-      if (!nearest_geo(G, pos, best2, tri, lstack, 1, err)) {
+      T best2 = k == 0 ? s_first : static_cast<T>(CUDART_INF);
+      uint32_t tri = k == 0 ? s_first_tri : 0;
+      if (k == 0 ? best2 < T(0) : !nearest_geo(G, pos, best2, tri, stack, n, err)) {
         err |= TWOS_DEVERR_QUERY;
         active = false;
       } else {
@@ -148,8 +175,9 @@ template <typename T> __global__ void __launch_bounds__(1024) rqmc_kernel(const 
       const double U1 = uniform<double>(sh.x, sh.y), U2 = uniform<double>(sh.z, sh.w);
       // Korobov point (i/n, a i/n, a^2 i/n) mod 1: its first coordinate is
       // the sorted rank itself; the other two drive the step.
-      double a1 = static_cast<double>((static_cast<uint64_t>(R.generator) * rank) % n) / n + U1;
-      double a2 = static_cast<double>((static_cast<uint64_t>(R.generator2) * rank) % n) / n + U2;
+      // (n is a power of two.)
+      double a1 = static_cast<double>((R.generator * rank) & (n - 1u)) / n + U1;
+      double a2 = static_cast<double>((R.generator2 * rank) & (n - 1u)) / n + U2;
       a1 -= floor(a1);
       a2 -= floor(a2);
       u1 = static_cast<T>(a1);
@@ -307,12 +335,19 @@ cudaError_t launch_rqmc(int precision, const RqmcLaunch &R, cudaStream_t s) {
   if ((R.walk_u == nullptr) != (R.walk_p == nullptr)) return cudaErrorInvalidValue;
   if (R.method == TWOS_RQMC_SOBOL && (!R.sobol_v || (1u << R.sobol_bits) != R.walks || R.sobol_bits > kSobolBits))
     return cudaErrorInvalidValue;
-  const size_t dyn = R.walks * (sizeof(unsigned long long) + sizeof(uint32_t));
-  if (precision == TWOS_PREC_MIXED)
-    rqmc_kernel<float><<<static_cast<unsigned>(blocks), R.walks, dyn, s>>>(R);
-  else
-    rqmc_kernel<double><<<static_cast<unsigned>(blocks), R.walks, dyn, s>>>(R);
-  return cudaGetLastError();
+  const bool mixed = precision == TWOS_PREC_MIXED;
+  const size_t dyn = R.walks * (sizeof(unsigned long long) + sizeof(uint32_t)) +
+                     (mixed ? rqmc_near_entries<float>(R.walks) : rqmc_near_entries<double>(R.walks)) * sizeof(uint2);
+  const bool small = R.walks <= 256;
+  const void *fn = mixed ? (small ? reinterpret_cast<const void *>(&rqmc_kernel<float, 256>)
+                                  : reinterpret_cast<const void *>(&rqmc_kernel<float, 1024>))
+                         : (small ? reinterpret_cast<const void *>(&rqmc_kernel<double, 256>)
+                                  : reinterpret_cast<const void *>(&rqmc_kernel<double, 1024>));
+  const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dyn));
+  if (e != cudaSuccess) return e;
+  RqmcLaunch copy = R;
+  void *args[] = {&copy};
+  return cudaLaunchKernel(fn, dim3(static_cast<unsigned>(blocks)), dim3(R.walks), args, dyn, s);
 }
 
 cudaError_t launch_rqmc_reuse(const RqmcLaunch &R, cudaStream_t s) {
