@@ -186,3 +186,42 @@ def test_first_queries_return_the_traversals_value(tb, shape):
     # u = r^2/6 * 6 of the first ball, evaluated in FP32 as the walk does.
     want = np.where(r > np.float32(1e-30), (r * r / np.float32(6)) * np.float32(6), np.float32(0))
     assert np.array_equal(got["u"][:, 0].astype(np.float32), want)
+
+
+@pytest.mark.parametrize("shape", ["tetra", "sphere4", "noise5", "fan5", "fan64", "sliver", "box"])
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_candidate_lists_change_no_walk(tb, shape, precision):
+    """Queries from the grid cells' candidate lists (the default) against
+    queries that traverse from the root (entry=0): the same walks, bit for
+    bit -- with cavities, in cells whose candidates are too many for a list
+    (around the apex of 64 triangles) and among needle triangles."""
+    if shape == "tetra":
+        V = np.array([[0.0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1]]) - 0.25
+        F = np.array([[0, 2, 1], [0, 1, 3], [0, 3, 2], [1, 2, 3]], dtype=np.uint32)
+    elif shape.startswith("sphere"):
+        V, F = tb.geometry.icosphere(int(shape[6:]))
+    elif shape.startswith("noise"):
+        V, F = tb.geometry.noise_sphere(int(shape[5:]), 2)
+    elif shape == "sliver":
+        V, F = tb.geometry.icosphere(4)
+        V = V * np.array([1.0, 0.05, 1.0])
+    elif shape == "box":
+        V, F, _ = tb.geometry.box_minus_cylinders(h=0.2)
+        V = V - V.mean(0)
+    else:
+        V, F = _fan(int(shape[3:]))
+    rng = np.random.default_rng(9)
+    mid = V[F.astype(np.int64)].mean(1)
+    P = mid[rng.integers(0, len(mid), 150)] * rng.uniform(0.05, 0.98, (150, 1))
+    cav = np.array([[0.05, 0.0, 0.02], [-0.1, 0.01, 0.0]])
+    with tb.Mesh(V, F) as m:
+        keep = m.inside(P)
+        P = P[keep][:60]
+        for c in (None, cav):
+            cfg = tb.Config(walks=500, precision=precision, seed=14, epsilon=1e-4, cavity_radius=0.01, max_steps=4096,
+                            source=tb.sources.affine())
+            rows = []
+            for entry in (1, 0):
+                m.set_tuning(**dict(m.get_tuning(), entry=entry))
+                rows.append(m.estimate(P, cfg, cavities=c)[0])
+            np.testing.assert_array_equal(rows[0], rows[1])

@@ -619,10 +619,46 @@ __device__ __forceinline__ bool grid_bounds(const GeoDesc &g, const Vec<float> &
   return true;
 }
 
+// A cell record's last word: an entry node (-1: none), or the start of the
+// cell's candidate list, whose first entry holds the entry node.
+__device__ __forceinline__ bool is_list(int word) { return word < -1; }
+__device__ __forceinline__ uint32_t list_start(int word) { return static_cast<uint32_t>(word) & 0x7fffffffu; }
+__device__ __forceinline__ int entry_of(const GeoDesc &g, int word) {
+  return is_list(word) ? static_cast<int>(__ldg(&g.lists[list_start(word)].x)) : word;
+}
+// The last word of the record of p's cell (p inside the grid).
+__device__ __forceinline__ int cell_word(const GeoDesc &g, const Vec<float> &p) {
+  const float x[3] = {p.x, p.y, p.z};
+  size_t cell = 0;
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+    cell = cell * (g.grid_n[a] - 1) +
+           min(static_cast<uint32_t>(fmaxf((x[a] - g.grid_lo[a]) * g.grid_inv_h, 0.f)), g.grid_n[a] - 2);
+  return static_cast<int>(__ldg(&g.grid[cell].w));
+}
+// Distance from p to the centre of its grid cell, from above.
+__device__ __forceinline__ float cell_offset(const GeoDesc &g, const Vec<float> &p) {
+  float d2 = 0.f;
+  const float x[3] = {p.x, p.y, p.z};
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const uint32_t i = min(static_cast<uint32_t>((x[a] - g.grid_lo[a]) * g.grid_inv_h), g.grid_n[a] - 2);
+    const float e = x[a] - __fmaf_rn(static_cast<float>(i) + 0.5f, g.grid_h, g.grid_lo[a]);
+    d2 = __fmaf_ru(e, e, d2);
+  }
+  return __fsqrt_ru(d2);
+}
+
 __device__ __forceinline__ bool grid_bound(const GeoDesc &g, const Vec<float> &p, float &bound) {
   float upper;
   int entry_node;
   return grid_bounds(g, p, bound, upper, entry_node);
+}
+
+// (sqrt(d2) + by)^2, rounded up.
+__device__ __forceinline__ float widen2(float d2, float by) {
+  const float t = __fadd_ru(__fsqrt_ru(d2), by);
+  return __fmul_ru(t, t);
 }
 
 // ---------------------------------------------------------------- FP64 queries
@@ -762,7 +798,7 @@ __device__ __forceinline__ void grid_start(const GeoDesc &g, const Vec<float> &p
     return;
   }
   upper = __fmaf_ru(6.f, g.delta, upper);
-  if (entry >= 0 && fminf(radius, upper) < g.entry_radius) node = entry;
+  if (fminf(radius, upper) < g.entry_radius) node = max(entry_of(g, entry), 0);
 }
 
 // nearest() over the FP64 nodes, for what the FP32 bounds cannot hold; out of
@@ -1129,6 +1165,13 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
   // Four-wide form: this query continues on the binary BVH (set when a
   // four-wide visit would overflow the stack).
   bool narrow = false;
+  // The query reads its cell's candidate list: node = the entry at hand (its
+  // triangle in tri_cur, the bits of its centre distance in tri_end), sp = the
+  // bits of the distance from the cell centre; FP32: have = a triangle, iter,
+  // improved best2, second = the smallest distance of another one.
+  constexpr bool LISTS = !WIDE;
+  bool list = false;
+  float second = CUDART_INF_F;
   bool resume = false;  // FP64 form: back to the traversal after the candidates' test
   bool tri_ok = false;    // best_tri belongs to this walk
   uint32_t tri_cur = 0, tri_end = 0, iter = 0;
@@ -1142,7 +1185,7 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
   // Squared bound that prunes a subtree.
   auto prune_limit = [&]() -> float {
     if constexpr (sizeof(T) == 4)
-      return best2;
+      return LISTS && list ? cull.limit : best2.v;
     else
       return cull.limit;
   };
@@ -1194,6 +1237,7 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
         return;
       }
     }
+    list = false;
     const float ubs = __fmaf_ru(6.f, G.delta, upper);
     // A cavity nearer than the mesh decides the step, so the search goes no
     // farther than the cavity, and with a mesh known to be beyond there is
@@ -1217,7 +1261,10 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
       }
     }
     if (in_grid) {
-      if (!WIDE && entry_node >= 0 && ubs < G.entry_radius) node = entry_node;
+      if constexpr (LISTS) {
+        list = is_list(entry_node);
+        if (!list && entry_node >= 0 && ubs < G.entry_radius) node = entry_node;
+      }
       if constexpr (sizeof(T) == 4) {
         best2 = fminf(best2, ubs * ubs);
       } else {
@@ -1226,6 +1273,28 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
       }
     }
     set_best2(best2);
+    iter = 0;
+    phase = kTraverse;
+    if (LISTS && list) {
+      // The candidates hold every triangle that can be nearest (or within 3
+      // delta of it) at a point of the cell, nearest to the cell's centre
+      // first.
+      const Vec<float> q = [&]() -> Vec<float> {
+        if constexpr (sizeof(T) == 4)
+          return pos;
+        else
+          return cull.p;
+      }();
+      sp = __float_as_int(__fmaf_ru(2.f, G.delta, cell_offset(G, q)));
+      node = static_cast<int>(list_start(entry_node)) + 1;
+      const uint2 e = __ldg(G.lists + node);
+      tri_cur = e.x;
+      tri_end = e.y;
+      have = false;
+      second = CUDART_INF_F;
+      if constexpr (sizeof(T) == 4) cull.limit = best2;
+      return;
+    }
     sp = 0;
     have = true;
     narrow = false;
@@ -1238,8 +1307,6 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
       tri_cur = best_tri;
       tri_end = tri_cur + 1;
     }
-    iter = 0;
-    phase = kTraverse;
   };
 
   for (;;) {
@@ -1608,9 +1675,44 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
       };
 #pragma unroll 1
       for (int unit = 0; unit < units; ++unit) {
+        if constexpr (LISTS) {
+          if (list) {
+            const float low = __uint_as_float(tri_end) - __int_as_float(sp);
+            if (tri_end == 0x7f800000u || (low > 0.f && !(low * low < prune_limit()))) {
+              // No later candidate is nearer.  FP32: with another triangle
+              // within rounding of the minimum, the value depends on the
+              // order of the tests, and the traversal's is the one to return.
+              list = false;
+              if (sizeof(T) == 8 || (found && !(have && second < cull.limit))) {
+                if (sizeof(T) == 4 && have) {
+                  best_tri = iter;
+                  tri_ok = true;
+                }
+                phase = kStep;
+                break;
+              }
+              if constexpr (sizeof(T) == 4) {
+                if (have) {
+                  best2 = cull.limit;
+                  found = false;
+                }
+                const int start = entry_of(G, cell_word(G, pos));
+                node = start >= 0 && sqrtf(best2) < G.entry_radius ? start : 0;
+                sp = 0;
+                have = true;
+                iter = 0;
+                tri_cur = tri_end = 0;
+                if (L.warm && tri_ok) {
+                  tri_cur = best_tri;
+                  tri_end = tri_cur + 1;
+                }
+              }
+            }
+          }
+        }
         // The unit's triangle or node: the leaf at hand, else the current
         // node or the next stack entry still closer than the current best.
-        if (tri_cur >= tri_end) {
+        if (!(LISTS && list) && tri_cur >= tri_end) {
           while (!have && sp > 0) {
             --sp;
             const uint2 e = sp < kShared ? stack[sp * BLOCK] : deep[sp - kShared];
@@ -1630,7 +1732,7 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
             have = false;
           }
         }
-        if (++iter > G.max_iter) {
+        if (!(LISTS && list) && ++iter > G.max_iter) {
           fail(TWOS_DEVERR_ITER);
           break;
         }
@@ -1676,28 +1778,39 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
         // One set of loads for either kind (64 bytes of a triangle or 96 of a
         // node): lanes on nodes and lanes on triangles wait for memory
         // together, once per unit, before the warp splits on the arithmetic.
-        const bool on_tri = tri_cur < tri_end;
+        const bool on_tri = (LISTS && list) || tri_cur < tri_end;
         const char *at = on_tri ? reinterpret_cast<const char *>(G.tris_f + tri_cur)
                                 : reinterpret_cast<const char *>(G.nodes_f + node);
         float4 r0, r1, r2, r3, r4{}, r5{};
         ldg32(at, r0, r1);
         ldg32(at + 32, r2, r3);
         ldg32_if(!on_tri, at + 64, r4, r5);
+        uint2 next = make_uint2(tri_cur + 1u, tri_end);
+        if (LISTS && list) next = __ldg(G.lists + node + 1);
         if (on_tri) {
           ++c_planes;
           if constexpr (sizeof(T) == 4) {
-            if (plane_gap2(r0, r1, pos) < best2) {
+            if (plane_gap2(r0, r1, pos) < prune_limit()) {
               ++c_tris;
               const float d2 = tri_dist2(pos, Vec<float>{r1.x, r1.y, r1.z}, Vec<float>{r2.x, r2.y, r2.z},
                                          Vec<float>{r3.x, r3.y, r3.z});
-              if (d2 < best2) {
-                best2 = d2;
-                found = true;
+              const bool nearer = d2 < best2;
+              if (LISTS && list) {
+                if (!nearer || have) second = fminf(second, nearer ? best2.v : d2);
+                if (nearer) {
+                  cull.limit = widen2(d2, 3.f * G.delta);
+                  iter = tri_cur;
+                  have = true;
+                }
+              } else if (nearer) {
                 best_tri = tri_cur;
                 tri_ok = true;
               }
+              if (nearer) {
+                best2 = d2;
+                found = true;
+              }
             }
-            ++tri_cur;
           } else {
             // A full candidate list is tested first; the triangle comes again.
             if (cull_tri(tri_cur, r0, r1, r2, r3, cull, stack + kShared * BLOCK, BLOCK, c_tris)) {
@@ -1705,8 +1818,10 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
               phase = kStep;
               break;
             }
-            ++tri_cur;
           }
+          tri_cur = next.x;
+          tri_end = next.y;
+          if (LISTS && list) ++node;
         } else {
           ++c_nodes;
           float dl, dr;
@@ -1847,10 +1962,6 @@ template <typename T> __device__ __forceinline__ void warp_best(T &best, uint32_
 // (node_first: a node's first triangle), which are few.
 constexpr int kContend = 256;
 constexpr int kWarpEntries = kWarpStack + kContend + 1;  // shared-memory entries per warp
-__device__ __forceinline__ float widen2(float d2, float by) {
-  const float t = __fadd_ru(__fsqrt_ru(d2), by);
-  return __fmul_ru(t, t);
-}
 __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<float> &p, float &best2, uint32_t &best_tri,
                                              uint2 *stack, uint32_t &err) {
   const unsigned full = 0xffffffffu, lane = threadIdx.x & 31u;
@@ -2811,6 +2922,142 @@ cudaError_t launch_grid_pack(const uint16_t *vertices, const uint32_t n[3], cons
   const int grid = static_cast<int>(std::min<uint64_t>((count + 255) / 256, 148ull * 64));
   grid_pack_kernel<<<grid, 256, 0, s>>>(vertices, n[0], n[1], n[2], table, shift, table ? entry_n[1] : 0,
                                         table ? entry_n[2] : 0, cells);
+  return cudaGetLastError();
+}
+
+// Candidate lists (GeoDesc::lists).  A cell whose centre lies within
+// kListReach spacings of the surface -- beyond, a mixed-form step takes its
+// radius from the grid -- lists every triangle that can be nearest, or within
+// 8 delta of it, at a point of the cell: with rho half the cell's diagonal
+// (grown by the 0.01 h of the point-to-cell rounding), those within
+// d(centre) + 2 rho of the centre.  At most kListMost triangles; denser cells
+// keep their entry node.
+constexpr float kListReach = 1.7f;
+constexpr int kListMost = 30;
+
+// The cells near the surface, in `cells` (cells[0 .. *count)).
+__global__ void __launch_bounds__(256) list_cells_kernel(const GeoDesc *geo, uint32_t *cells, uint32_t capacity,
+                                                         uint32_t *count) {
+  const GeoDesc G = *geo;
+  const uint64_t m1 = G.grid_n[1] - 1, m2 = G.grid_n[2] - 1, n = (G.grid_n[0] - 1) * m1 * m2;
+  const float most = (kListReach + 0.8661f) * 128.f + 1.f;  // corner values of such a cell are below
+  const unsigned lane = threadIdx.x & 31u;
+  const uint64_t threads = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+  for (uint64_t base = blockIdx.x * static_cast<uint64_t>(blockDim.x); base < n; base += threads) {
+    const uint64_t cell = base + threadIdx.x;
+    const bool take = cell < n && static_cast<float>(G.grid[cell].z & 0xffffu) <= most;
+    const unsigned m = __ballot_sync(0xffffffffu, take);
+    if (m == 0u) continue;
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(count, static_cast<uint32_t>(__popc(m)));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+    if (take && cells && at < capacity) cells[at] = static_cast<uint32_t>(cell);
+  }
+}
+
+// FILL 0: adds the entries of all lists to *cursor; 1: writes the lists at
+// positions taken from *cursor and points the records at them.
+template <int FILL>
+__global__ void __launch_bounds__(kWosBlock) list_build_kernel(const GeoDesc *geo, const uint32_t *cells, uint32_t n,
+                                                               uint4 *grid, uint2 *lists, uint32_t *cursor,
+                                                               uint32_t *error) {
+  __shared__ uint2 s_stack[near_entries<double>() * kWosBlock];
+  const GeoDesc G = *geo;
+  const uint64_t m1 = G.grid_n[1] - 1, m2 = G.grid_n[2] - 1;
+  uint32_t err = 0;
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    const uint64_t cell = cells[t];
+    const float h = G.grid_h;
+    const Vec<float> c{__fmaf_rn(static_cast<float>(cell / (m1 * m2)) + 0.5f, h, G.grid_lo[0]),
+                       __fmaf_rn(static_cast<float>(cell / m2 % m1) + 0.5f, h, G.grid_lo[1]),
+                       __fmaf_rn(static_cast<float>(cell % m2) + 0.5f, h, G.grid_lo[2])};
+    // The centre's FP64 distance, and lower bounds for the triangles that hold
+    // however degenerate they are.
+    double best2 = CUDART_INF;
+    uint32_t tri = 0;
+    const Vec<double> c64{static_cast<double>(c.x) + G.center[0], static_cast<double>(c.y) + G.center[1],
+                          static_cast<double>(c.z) + G.center[2]};
+    if (!nearest_geo(G, c64, best2, tri, s_stack + threadIdx.x, kWosBlock, err)) continue;
+    const float d = __double2float_ru(sqrt(best2));
+    if (!(d <= kListReach * h)) continue;
+    const float radius = d + 1.7668f * h + 8.f * G.delta;  // 2 rho = sqrt(3) * 1.02 h
+    const float limit = radius * radius;
+    uint32_t id[kListMost];
+    float dist[kListMost];
+    int held = 0;
+    uint2 stack[kStack];
+    int sp = 0, node = 0;
+    uint32_t iter = 0;
+    bool fits = true;
+    for (bool have = true; have && fits;) {
+      if (++iter > G.max_iter) {
+        fits = false;
+        break;
+      }
+      if (node < 0) {
+        const uint32_t enc = ~static_cast<uint32_t>(node);
+        for (uint32_t i = enc >> 3, e = (enc >> 3) + (enc & 7u); i < e && fits; ++i) {
+          if (!(tri_plane_gap2(G.tris_f, i, c) < limit)) continue;
+          Vec<float> ta, tb, tc;
+          load_tri(G.tris_f, i, ta, tb, tc);
+          const Vec<float> ap = sub(c, ta), bp = sub(c, tb), cp = sub(c, tc);
+          const Vec<float> w = tri_point(ap, bp, cp, sub(tb, ta), sub(tc, ta));
+          const float d2 = support2(w, ap, bp, cp, dot3(w, w));
+          if (!(d2 < limit)) continue;
+          if (held == kListMost) {
+            fits = false;
+          } else if (FILL) {
+            const float dd = sqrtf(d2);
+            int k = held;
+            for (; k > 0 && (dist[k - 1] > dd || (dist[k - 1] == dd && id[k - 1] > i)); --k) {
+              dist[k] = dist[k - 1];
+              id[k] = id[k - 1];
+            }
+            dist[k] = dd;
+            id[k] = i;
+          }
+          ++held;
+        }
+      } else {
+        float dl, dr;
+        int cl, cr;
+        node_dist2(G.nodes_f, node, c, dl, dr, cl, cr);
+        if (dl < limit || dr < limit) {
+          if (dl < limit && dr < limit) stack[sp++] = make_uint2(static_cast<uint32_t>(cr), 0u);
+          node = dl < limit ? cl : cr;
+          continue;
+        }
+      }
+      have = sp > 0;
+      if (have) node = static_cast<int>(stack[--sp].x);
+    }
+    if (!fits) continue;
+    // Header (entry node), the triangles, a terminator.
+    const uint32_t at = atomicAdd(cursor, static_cast<uint32_t>(held + 2));
+    if (FILL) {
+      uint2 *out = lists + at;
+      out[0] = make_uint2(grid[cell].w, 0u);
+      for (int k = 0; k < held; ++k) out[1 + k] = make_uint2(id[k], __float_as_uint(dist[k]));
+      out[1 + held] = make_uint2(0u, 0x7f800000u);
+      grid[cell].w = 0x80000000u | at;
+    }
+  }
+  if (err) atomicOr(error, err);
+}
+
+cudaError_t launch_list_cells(const GeoDesc *geo_dev, uint32_t *cells, uint32_t capacity, uint32_t *count,
+                              cudaStream_t s) {
+  list_cells_kernel<<<148 * 8, 256, 0, s>>>(geo_dev, cells, capacity, count);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_list_build(const GeoDesc *geo_dev, const uint32_t *cells, uint32_t n, uint4 *grid, uint2 *lists,
+                              uint32_t *cursor, uint32_t *error, cudaStream_t s) {
+  const int blocks = static_cast<int>(std::min<uint32_t>((n + kWosBlock - 1) / kWosBlock, 148u * 32));
+  if (lists)
+    list_build_kernel<1><<<blocks, kWosBlock, 0, s>>>(geo_dev, cells, n, grid, lists, cursor, error);
+  else
+    list_build_kernel<0><<<blocks, kWosBlock, 0, s>>>(geo_dev, cells, n, grid, lists, cursor, error);
   return cudaGetLastError();
 }
 

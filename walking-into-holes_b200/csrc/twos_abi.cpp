@@ -67,6 +67,46 @@ double seconds_since(std::chrono::steady_clock::time_point t0) {
 // covering the FP32 query and the vertex placement), in steps of h/128.
 std::vector<int32_t> build_entry_table(twos_mesh *m);
 
+// Candidate lists of the grid cells near the surface (a few hundred MB for
+// the 4 GB grid of the 327,680-triangle noise sphere, built on the device).
+// A grid whose lists would take more than 2 GB keeps its entry nodes.
+void build_candidate_lists(twos_mesh *m) {
+  GeoDesc &g = m->geo_host;
+  const uint64_t cells = static_cast<uint64_t>(g.grid_n[0] - 1) * (g.grid_n[1] - 1) * (g.grid_n[2] - 1);
+  if (cells > 0xffffffffull || !(g.cull_margin > 0.f)) return;
+  check(cudaMemcpy(m->geo.ptr, &g, sizeof(GeoDesc), cudaMemcpyHostToDevice), "upload");
+  unsigned long long *tot = m->totals.as<unsigned long long>();
+  uint32_t *word = reinterpret_cast<uint32_t *>(tot);  // [0] cells, [1] entries, [2] write cursor, [4] errors
+  check(cudaMemset(tot, 0, 24), "memset");
+  const GeoDesc *geo = m->geo.as<GeoDesc>();
+  auto read = [&](int i) {
+    uint32_t v = 0;
+    check(cudaMemcpy(&v, word + i, sizeof(v), cudaMemcpyDeviceToHost), "candidate lists");
+    return v;
+  };
+  check(launch_list_cells(geo, nullptr, 0, word, nullptr), "list cells");
+  const uint32_t near = read(0);
+  if (near == 0 || near > (1u << 26)) return;  // at most 32 entries a cell: their count fits 32 bits
+  DevBuf ids;
+  struct Release {
+    DevBuf &b;
+    ~Release() { b.release(); }
+  } release_ids{ids};
+  ids.reserve(near * sizeof(uint32_t));
+  check(cudaMemset(word, 0, sizeof(uint32_t)), "memset");
+  check(launch_list_cells(geo, ids.as<uint32_t>(), near, word, nullptr), "list cells");
+  check(launch_list_build(geo, ids.as<uint32_t>(), near, nullptr, nullptr, word + 1, word + 4, nullptr), "list sizes");
+  const uint32_t entries = read(1);
+  if (entries == 0 || entries > (1u << 28) || read(4) != 0) return;
+  m->lists.reserve(entries * sizeof(uint2));
+  check(launch_list_build(geo, ids.as<uint32_t>(), near, m->grid.as<uint4>(), m->lists.as<uint2>(), word + 2, word + 4,
+                          nullptr),
+        "candidate lists");
+  check(cudaDeviceSynchronize(), "candidate lists");
+  g.lists = m->lists.as<uint2>();
+  m->resident_bytes += entries * sizeof(uint2);
+}
+
 void build_distance_grid(twos_mesh *m, size_t n_tris) {
   GeoDesc &g = m->geo_host;
   g.grid = nullptr;
@@ -138,6 +178,7 @@ void build_distance_grid(twos_mesh *m, size_t n_tris) {
   check(cudaDeviceSynchronize(), "grid pack");
   g.grid = m->grid.as<uint4>();
   m->resident_bytes += cells * sizeof(uint4);
+  build_candidate_lists(m);
 }
 
 // The entry-node table over the distance grid: cells of 2^s grid spacings
@@ -672,7 +713,7 @@ void twos_mesh_close(twos_mesh *m) {
   if (m->stream) cudaStreamSynchronize(m->stream);
   for (DevBuf *b : {&m->nodes_f, &m->tris_f, &m->nodes_d, &m->tris_d, &m->geo, &m->jobs, &m->geos, &m->terms, &m->cavities,
                     &m->sites, &m->out, &m->u, &m->p, &m->steps, &m->first, &m->counter, &m->totals, &m->points, &m->dist,
-                    &m->closest, &m->topk, &m->grid, &m->grad, &m->nodes4_f, &m->wf, &m->node_first})
+                    &m->closest, &m->topk, &m->grid, &m->grad, &m->nodes4_f, &m->wf, &m->node_first, &m->lists})
     b->release();
   m->scratch.release();
   if (m->ev0) cudaEventDestroy(m->ev0);

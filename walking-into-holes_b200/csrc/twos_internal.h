@@ -145,9 +145,13 @@ struct GeoDesc {
   // .y (corners 4-7), corner = a * 4 + b * 2 + c, each corner's D minus that
   // base (255: saturated or too far above the base -- the base alone is used
   // and the corner gives no upper bound), and in .w the cell's entry node
-  // (-1: none).  D varies by at most sqrt(3) h / grid_q + 1 < 224 over a
+  // (-1: none) or, with the top bit set, the start of its candidate list.  D varies by at most sqrt(3) h / grid_q + 1 < 224 over a
   // cell, so the bytes hold every unsaturated corner exactly.
   const uint4 *grid;
+  // Candidate lists of the cells near the surface: (entry node, 0), then
+  // (triangle, distance from the cell's centre) by that distance, then
+  // (0, infinity).  A query at a point of the cell needs no other triangle.
+  const uint2 *lists;
   float grid_lo[3];
   float grid_h, grid_inv_h, grid_q;
   uint32_t grid_n[3];
@@ -474,6 +478,13 @@ cudaError_t launch_grid_build(const GeoDesc *geo_dev, uint64_t n, double margin,
 // records of GeoDesc::grid.
 cudaError_t launch_grid_pack(const uint16_t *vertices, const uint32_t n[3], const int32_t *table, uint32_t shift,
                              const uint32_t entry_n[3], uint4 *cells, cudaStream_t s);
+// Candidate lists: the cells near the surface (count only without `cells`),
+// then the entries of their lists added to *cursor (without `lists`) or the
+// lists themselves, the records in `grid` pointed at them.
+cudaError_t launch_list_cells(const GeoDesc *geo_dev, uint32_t *cells, uint32_t capacity, uint32_t *count,
+                              cudaStream_t s);
+cudaError_t launch_list_build(const GeoDesc *geo_dev, const uint32_t *cells, uint32_t n, uint4 *grid, uint2 *lists,
+                              uint32_t *cursor, uint32_t *error, cudaStream_t s);
 // The walk step's grid bound at each point (original coordinates); NaN
 // outside the grid.
 cudaError_t launch_grid_bound(const GeoDesc *geo_dev, const double *pts, uint64_t n, double *out, cudaStream_t s);

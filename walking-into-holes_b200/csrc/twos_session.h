@@ -98,6 +98,7 @@ struct twos_mesh {
   twos::DevBuf nodes_f, tris_f, nodes_d, tris_d;
   twos::DevBuf grid;   // distance-bound grid (16-byte corner record per cell), may be empty
   twos::DevBuf nodes4_f;  // the four-wide BVH (mixed form, bvh_width 4)
+  twos::DevBuf lists;       // candidate lists of the grid cells near the surface
   twos::DevBuf node_first;  // first triangle of each node
   twos::DevBuf geo;  // one GeoDesc
   twos::GeoDesc geo_host{};

@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(kCertBlock, 6) cert_walk_kernel(const Validate
           }
           if (!(low >= far)) {
             low = 0.0;
-            node = entry >= 0 && ub < G.entry_radius ? entry : 0;
+            node = ub < G.entry_radius ? max(entry_of(G, entry), 0) : 0;
             const float reach = __fmaf_ru(2.f, c.margin, fminf(ub, __double2float_ru(far)));
             c.limit = __fmul_ru(reach, reach);
             sp = 0;

@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(kWfStepBlock) wf_step_kernel(const WosLaunch L
         found = true;
         ++c_grid;
       } else {
-        if (!(in_grid && L.entry)) entry_node = -1;
+        entry_node = in_grid && L.entry ? entry_of(G, entry_node) : -1;
         if (L.warm && tri_ok) {
           Vec<float> ta, tb, tc;
           load_tri(G.tris_f, best_tri, ta, tb, tc);
