@@ -58,6 +58,27 @@ __device__ __forceinline__ Philox4 philox(uint32_t k0, uint32_t k1, uint32_t c0,
   return {c0, c1, c2, c3};
 }
 
+// Blocks c3, c3 + 1, .. c3 + N - 1 of one counter together, round by round: a
+// step that draws several blocks spends a tenth of the instructions' bytes
+// (the walk kernels' stalls on instruction fetch) and has N independent chains.
+template <int N>
+__device__ __forceinline__ void philox_blocks(uint32_t k0, uint32_t k1, uint32_t c0, uint32_t c1, uint32_t c2,
+                                              uint32_t c3, Philox4 (&q)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) q[i] = {c0, c1, c2, c3 + static_cast<uint32_t>(i)};
+#pragma unroll 1
+  for (int r = 0; r < 10; ++r) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const uint32_t lo0 = 0xD2511F53u * q[i].x, hi0 = __umulhi(0xD2511F53u, q[i].x);
+      const uint32_t lo1 = 0xCD9E8D57u * q[i].z, hi1 = __umulhi(0xCD9E8D57u, q[i].z);
+      q[i] = {hi1 ^ q[i].y ^ k0, lo1, hi0 ^ q[i].w ^ k1, lo0};
+    }
+    k0 += 0x9E3779B9u;
+    k1 += 0xBB67AE85u;
+  }
+}
+
 // Uniforms in [0,1): FP64 takes the top 53 bits of (hi:lo); FP32 takes the
 // top 24, i.e. the FP64 value truncated, so both forms share samples.
 template <typename T> __device__ __forceinline__ T uniform(uint32_t hi, uint32_t lo);
@@ -491,10 +512,29 @@ template <typename T> __device__ __forceinline__ T term_value(const TermT<T> &t,
 
 template <typename T>
 __device__ __forceinline__ T source_value(const TermT<T> *terms, uint32_t begin, uint32_t n, const Vec<T> &x) {
-  if (n == 0) return T(0);
-  T s = term_value(terms[begin], x);
-  for (uint32_t i = 1; i < n; ++i) s = s + term_value(terms[begin + i], x);
+  T s = T(0);
+#pragma unroll 1
+  for (uint32_t i = 0; i < n; ++i) {
+    const T v = term_value(terms[begin + i], x);
+    s = i == 0 ? v : s + v;
+  }
   return s;
+}
+
+// Two sources at one point, through one copy of the terms' code.
+template <typename T>
+__device__ __forceinline__ void source_values(const TermT<T> *terms, uint32_t begin0, uint32_t n0, uint32_t begin1,
+                                              uint32_t n1, const Vec<T> &x, T &s0, T &s1) {
+  s0 = s1 = T(0);
+#pragma unroll 1
+  for (uint32_t i = 0; i < n0 + n1; ++i) {
+    const bool second = i >= n0;
+    const T v = term_value(terms[second ? begin1 + (i - n0) : begin0 + i], x);
+    if (second)
+      s1 = i == n0 ? v : s1 + v;
+    else
+      s0 = i == 0 ? v : s0 + v;
+  }
 }
 
 }  // namespace twos
@@ -1454,12 +1494,15 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
           if (!done) {
             const uint32_t ctr3 = J.repeat << 3;
             const uint32_t step = steps, wk = walk, key = J.site_offset + site;
-            const Philox4 q0 = philox(J.k0, J.k1, step, wk, key, ctr3 | 0u);
+            Philox4 q0;
             Vec<T> a = pos;
-            if (GREEN) {
-              const Philox4 q1 = philox(J.k0, J.k1, step, wk, key, ctr3 | 1u);
-              const Philox4 q2 = philox(J.k0, J.k1, step, wk, key, ctr3 | 2u);
-              const Philox4 q3 = philox(J.k0, J.k1, step, wk, key, ctr3 | 3u);
+            if constexpr (!GREEN) {
+              q0 = philox(J.k0, J.k1, step, wk, key, ctr3 | 0u);
+            } else {
+              Philox4 q[4];
+              philox_blocks(J.k0, J.k1, step, wk, key, ctr3, q);
+              q0 = q[0];
+              const Philox4 q1 = q[1], q2 = q[2], q3 = q[3];
               const T beta = median3(uniform<T>(q2.x, q2.y), uniform<T>(q2.z, q2.w), uniform<T>(q3.x, q3.y));
               const Vec<T> g = direction<T>(uniform<T>(q1.x, q1.y), uniform<T>(q1.z, q1.w));
               a = add_scaled(pos, g, r * beta);
@@ -1469,15 +1512,18 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
               if (PAIRED) pv = exact_source(static_cast<T>(pv), s_terms, J.adj_begin, J.n_adj, pos, r, err);
             } else {
               const T w = r * r / T(6);
-              if (MODE != kModeBoundary) {
-                const T du = w * source_value(s_terms, J.src_begin, J.n_src, a);
+              if constexpr (PAIRED) {
+                T su, sp;
+                source_values(s_terms, J.src_begin, J.n_src, J.adj_begin, J.n_adj, a, su, sp);
+                const T du = w * su, dp = w * sp;
                 u = u + du;
-                if (GRAD && step == 0) g_u0 = du;
-              }
-              if (PAIRED) {
-                const T dp = w * source_value(s_terms, J.adj_begin, J.n_adj, a);
                 pv = pv + dp;
-                if (GRAD && step == 0) g_p0 = dp;
+                if (GRAD && step == 0) {
+                  g_u0 = du;
+                  g_p0 = dp;
+                }
+              } else if (MODE != kModeBoundary) {
+                u = u + w * source_value(s_terms, J.src_begin, J.n_src, a);
               }
             }
             const Vec<T> dir = direction<T>(uniform<T>(q0.x, q0.y), uniform<T>(q0.z, q0.w));
@@ -1485,14 +1531,16 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
               // First ball: the sphere term's radius and direction, and one draw
               // (blocks 4-5) for the ball source term of the gradient,
               // R (1 - t^3) f(x + t R w') w' with t ~ U(0,1), w' uniform.
-              const Philox4 q4 = philox(J.k0, J.k1, 0u, wk, key, ctr3 | 4u);
-              const Philox4 q5 = philox(J.k0, J.k1, 0u, wk, key, ctr3 | 5u);
+              Philox4 qb[2];
+              philox_blocks(J.k0, J.k1, 0u, wk, key, ctr3 | 4u, qb);
+              const Philox4 q4 = qb[0], q5 = qb[1];
               const T t = uniform<T>(q4.x, q4.y);
               const Vec<T> wp = direction<T>(uniform<T>(q4.z, q4.w), uniform<T>(q5.x, q5.y));
               const Vec<T> z = add_scaled(pos, wp, t * r);
               const T wt = r * (T(1) - t * t * t);
-              const T fs = wt * source_value(s_terms, J.src_begin, J.n_src, z);
-              const T fq = wt * source_value(s_terms, J.adj_begin, J.n_adj, z);
+              T su, sq;
+              source_values(s_terms, J.src_begin, J.n_src, J.adj_begin, J.n_adj, z, su, sq);
+              const T fs = wt * su, fq = wt * sq;
               g_su[0] = wp.x * fs;
               g_su[1] = wp.y * fs;
               g_su[2] = wp.z * fs;
@@ -1732,7 +1780,7 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
             have = false;
           }
         }
-        if (!(LISTS && list) && ++iter > G.max_iter) {
+        if ((sizeof(T) == 8 || !(LISTS && list)) && ++iter > G.max_iter) {
           fail(TWOS_DEVERR_ITER);
           break;
         }
