@@ -618,47 +618,85 @@ __device__ __forceinline__ Vec<float> grid_vertex(const GeoDesc &g, uint32_t i, 
           __fadd_rn(g.grid_lo[2], __fmul_rn(static_cast<float>(k), g.grid_h))};
 }
 
-// The grid's bounds of the mesh distance at `p` (FP32 frame).  Lower: the
-// largest D(v) - |p - v| over the eight corners v of p's cell (the distance
-// is 1-Lipschitz, so each is a bound).  Upper (before the FP32 allowance
-// the caller adds): the smallest (D(v) + 1) q + |p - v| over the corners
-// whose value is held exactly -- a vertex stores floor((d_FP32 - 2 delta)/q),
-// so its distance is below (D + 1) q + 3 delta.  `entry_node` is the cell's
-// entry node (-1: none).  False when p lies outside the grid (or is NaN).
-// One 16-byte record per cell (GeoDesc::grid).
-__device__ __forceinline__ bool grid_bounds(const GeoDesc &g, const Vec<float> &p, float &bound, float &upper,
-                                            int &entry_node) {
+// An integer below 2^23 as a float, exactly: one integer and one float
+// operation instead of a conversion, which has a sixteenth of their rate.
+__device__ __forceinline__ float small_float(uint32_t v) { return __uint_as_float(0x4B000000u | v) - 8388608.f; }
+
+// The grid cell of `p` (FP32 frame): its lower corner (clamped so the cell
+// lies inside the grid) and record; false when p lies outside the grid (or is
+// NaN).  A grid has fewer than 2^32 cells.
+__device__ __forceinline__ bool grid_cell(const GeoDesc &g, const Vec<float> &p, uint32_t (&c)[3], uint32_t &cell) {
   const float fx = (p.x - g.grid_lo[0]) * g.grid_inv_h;
   const float fy = (p.y - g.grid_lo[1]) * g.grid_inv_h;
   const float fz = (p.z - g.grid_lo[2]) * g.grid_inv_h;
-  if (!(fx >= 0.f && fy >= 0.f && fz >= 0.f && fx <= static_cast<float>(g.grid_n[0] - 1) &&
-        fy <= static_cast<float>(g.grid_n[1] - 1) && fz <= static_cast<float>(g.grid_n[2] - 1)))
+  if (!(fx >= 0.f && fy >= 0.f && fz >= 0.f && fx <= g.grid_top[0] && fy <= g.grid_top[1] && fz <= g.grid_top[2]))
     return false;
-  // The cell's lower corner (clamped so the cell lies inside the grid), then
-  // the best of its eight corners' bounds.
-  const uint32_t i0 = min(static_cast<uint32_t>(fx), g.grid_n[0] - 2);
-  const uint32_t j0 = min(static_cast<uint32_t>(fy), g.grid_n[1] - 2);
-  const uint32_t k0 = min(static_cast<uint32_t>(fz), g.grid_n[2] - 2);
-  float best = -CUDART_INF_F, up = CUDART_INF_F;
-  const uint4 rec = __ldg(g.grid + (static_cast<size_t>(i0) * (g.grid_n[1] - 1) + j0) * (g.grid_n[2] - 1) + k0);
-  const uint32_t base = rec.z & 0xffffu;
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    const uint32_t i = i0 + (c >> 2), j = j0 + ((c >> 1) & 1), k = k0 + (c & 1);
-    const Vec<float> v = grid_vertex(g, i, j, k);
-    const Vec<float> dv = sub(p, v);
-    const uint32_t off = ((c < 4 ? rec.x : rec.y) >> (8 * (c & 3))) & 0xffu;
-    const float dist = sqrt_up(dot3(dv, dv));
-    const float dq = static_cast<float>(off == 0xffu ? base : base + off) * g.grid_q;
-    best = fmaxf(best, dq - dist);
-    if (off != 0xffu) up = fminf(up, dq + g.grid_q + dist);
-  }
-  bound = best;
-  upper = up;
-  entry_node = static_cast<int>(rec.w);
+  c[0] = min(static_cast<uint32_t>(fx), g.grid_n[0] - 2);
+  c[1] = min(static_cast<uint32_t>(fy), g.grid_n[1] - 2);
+  c[2] = min(static_cast<uint32_t>(fz), g.grid_n[2] - 2);
+  cell = (c[0] * (g.grid_n[1] - 1) + c[1]) * (g.grid_n[2] - 1) + c[2];
   return true;
 }
 
+// The grid's bounds of the mesh distance at `p`.  Lower: the
+// largest D(v) - |p - v| over the eight corners v of p's cell (the distance
+// is 1-Lipschitz, so each is a bound).  Upper (with UPPER; before the FP32
+// allowance the caller adds): the smallest (D(v) + 1) q + |p - v| over the
+// corners whose value is held exactly -- a vertex stores
+// floor((d_FP32 - 2 delta)/q), so its distance is below (D + 1) q + 3 delta.
+// `word` is the record's last word (entry_of).  False when p lies outside the
+// grid.  One 16-byte record per cell (GeoDesc::grid).
+template <bool UPPER>
+__device__ __forceinline__ bool grid_bounds(const GeoDesc &g, const Vec<float> &p, float &bound, float &upper,
+                                            int &word) {
+  uint32_t c0[3], cell;
+  if (!grid_cell(g, p, c0, cell)) return false;
+  float best = -CUDART_INF_F, up = CUDART_INF_F;
+  const uint4 rec = __ldg(g.grid + cell);
+  const uint32_t base = rec.z & 0xffffu;
+  // The vertices' coordinates, rounded as grid_vertex rounds them.
+  float d[3][2];
+  const float x[3] = {p.x, p.y, p.z};
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const float f = small_float(c0[a]);
+    d[a][0] = x[a] - __fadd_rn(g.grid_lo[a], __fmul_rn(f, g.grid_h));
+    d[a][1] = x[a] - __fadd_rn(g.grid_lo[a], __fmul_rn(f + 1.f, g.grid_h));
+  }
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const Vec<float> dv{d[0][c >> 2], d[1][(c >> 1) & 1], d[2][c & 1]};
+    const uint32_t off = ((c < 4 ? rec.x : rec.y) >> (8 * (c & 3))) & 0xffu;
+    const float dist = sqrt_up(dot3(dv, dv));
+    const float dq = small_float(off == 0xffu ? base : base + off) * g.grid_q;
+    best = fmaxf(best, dq - dist);
+    if (UPPER && off != 0xffu) up = fminf(up, dq + g.grid_q + dist);
+  }
+  bound = best;
+  if (UPPER) upper = up;
+  word = static_cast<int>(rec.w);
+  return true;
+}
+
+// The upper bound alone, at a point of the grid (a rolled loop: the mixed
+// form's walk steps seldom need it).
+__device__ __forceinline__ float grid_upper(const GeoDesc &g, const Vec<float> &p) {
+  uint32_t c0[3], cell;
+  float up = CUDART_INF_F;
+  if (!grid_cell(g, p, c0, cell)) return up;
+  const uint4 rec = __ldg(g.grid + cell);
+  const uint32_t base = rec.z & 0xffffu;
+#pragma unroll 1
+  for (uint32_t c = 0; c < 8; ++c) {
+    const uint32_t off = ((c < 4 ? rec.x : rec.y) >> (8 * (c & 3))) & 0xffu;
+    if (off == 0xffu) continue;
+    const Vec<float> dv = sub(p, grid_vertex(g, c0[0] + (c >> 2), c0[1] + ((c >> 1) & 1u), c0[2] + (c & 1u)));
+    up = fminf(up, small_float(base + off) * g.grid_q + g.grid_q + sqrt_up(dot3(dv, dv)));
+  }
+  return up;
+}
+
+constexpr float kListReach = 1.7f;  // spacings from the surface up to which cells have lists
 // A cell record's last word: an entry node (-1: none), or the start of the
 // cell's candidate list, whose first entry holds the entry node.
 __device__ __forceinline__ bool is_list(int word) { return word < -1; }
@@ -668,22 +706,18 @@ __device__ __forceinline__ int entry_of(const GeoDesc &g, int word) {
 }
 // The last word of the record of p's cell (p inside the grid).
 __device__ __forceinline__ int cell_word(const GeoDesc &g, const Vec<float> &p) {
-  const float x[3] = {p.x, p.y, p.z};
-  size_t cell = 0;
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-    cell = cell * (g.grid_n[a] - 1) +
-           min(static_cast<uint32_t>(fmaxf((x[a] - g.grid_lo[a]) * g.grid_inv_h, 0.f)), g.grid_n[a] - 2);
-  return static_cast<int>(__ldg(&g.grid[cell].w));
+  uint32_t c[3], cell = 0;
+  return grid_cell(g, p, c, cell) ? static_cast<int>(__ldg(&g.grid[cell].w)) : -1;
 }
-// Distance from p to the centre of its grid cell, from above.
+// Distance from p to the centre of its grid cell (p inside the grid), from above.
 __device__ __forceinline__ float cell_offset(const GeoDesc &g, const Vec<float> &p) {
+  uint32_t c[3] = {0u, 0u, 0u}, cell;
+  grid_cell(g, p, c, cell);
   float d2 = 0.f;
   const float x[3] = {p.x, p.y, p.z};
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    const uint32_t i = min(static_cast<uint32_t>((x[a] - g.grid_lo[a]) * g.grid_inv_h), g.grid_n[a] - 2);
-    const float e = x[a] - __fmaf_rn(static_cast<float>(i) + 0.5f, g.grid_h, g.grid_lo[a]);
+    const float e = x[a] - __fmaf_rn(small_float(c[a]) + 0.5f, g.grid_h, g.grid_lo[a]);
     d2 = __fmaf_ru(e, e, d2);
   }
   return __fsqrt_ru(d2);
@@ -692,7 +726,7 @@ __device__ __forceinline__ float cell_offset(const GeoDesc &g, const Vec<float> 
 __device__ __forceinline__ bool grid_bound(const GeoDesc &g, const Vec<float> &p, float &bound) {
   float upper;
   int entry_node;
-  return grid_bounds(g, p, bound, upper, entry_node);
+  return grid_bounds<false>(g, p, bound, upper, entry_node);
 }
 
 // (sqrt(d2) + by)^2, rounded up.
@@ -833,7 +867,7 @@ __device__ __forceinline__ void grid_start(const GeoDesc &g, const Vec<float> &p
   int entry = -1;
   upper = CUDART_INF_F;
   node = 0;
-  if (!g.grid || !grid_bounds(g, p, bound, upper, entry)) {
+  if (!g.grid || !grid_bounds<true>(g, p, bound, upper, entry)) {
     upper = CUDART_INF_F;
     return;
   }
@@ -1243,14 +1277,15 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
       }
     }
   };
-  // The grid's bounds and entry node at pos.
+  // The grid's bounds and record word at pos (the mixed form's upper bound
+  // comes later: begin_query).
   auto walk_grid = [&](const GeoDesc &G, const Vec<T> &pos, float &bound, float &upper, int &entry_node) {
     if (!G.grid) return false;
     if constexpr (sizeof(T) == 4) {
-      return grid_bounds(G, pos, bound, upper, entry_node);
+      return grid_bounds<false>(G, pos, bound, upper, entry_node);
     } else {
       const double p3[3] = {pos.x, pos.y, pos.z};
-      return grid_bounds(G, to_frame<float>(p3, G), bound, upper, entry_node);
+      return grid_bounds<true>(G, to_frame<float>(p3, G), bound, upper, entry_node);
     }
   };
   // Starts the query at pos; `in_grid`: with the grid's upper bound and entry
@@ -1278,6 +1313,11 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
       }
     }
     list = false;
+    if constexpr (sizeof(T) == 4) {
+      // A point of a cell with a list is at most kListReach spacings and half
+      // a cell's diagonal from the surface: bound enough for its short search.
+      if (in_grid) upper = LISTS && is_list(entry_node) ? (kListReach + 0.9f) * G.grid_h : grid_upper(G, pos);
+    }
     const float ubs = __fmaf_ru(6.f, G.delta, upper);
     // A cavity nearer than the mesh decides the step, so the search goes no
     // farther than the cavity, and with a mesh known to be beyond there is
@@ -1356,8 +1396,9 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
       const uint64_t id = wid;
       job = find_job(s_jobs, L.n_jobs, id);
       const JobDesc &J = s_jobs[job];
+      // (A 64-bit division takes four times as long as a 32-bit one.)
       const uint64_t local = id - J.walk_begin;
-      const uint32_t at = static_cast<uint32_t>(local / J.walks);
+      const uint32_t at = local >> 32 ? static_cast<uint32_t>(local / J.walks) : static_cast<uint32_t>(local) / J.walks;
       site = at;
       walk = static_cast<uint32_t>(local - static_cast<uint64_t>(at) * J.walks);
       const GeoDesc &G = s_geos[J.geo];
@@ -1497,7 +1538,9 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
             Philox4 q0;
             Vec<T> a = pos;
             if constexpr (!GREEN) {
-              q0 = philox(J.k0, J.k1, step, wk, key, ctr3 | 0u);
+              Philox4 q[1];
+              philox_blocks(J.k0, J.k1, step, wk, key, ctr3, q);
+              q0 = q[0];
             } else {
               Philox4 q[4];
               philox_blocks(J.k0, J.k1, step, wk, key, ctr3, q);
@@ -2980,7 +3023,6 @@ cudaError_t launch_grid_pack(const uint16_t *vertices, const uint32_t n[3], cons
 // (grown by the 0.01 h of the point-to-cell rounding), those within
 // d(centre) + 2 rho of the centre.  At most kListMost triangles; denser cells
 // keep their entry node.
-constexpr float kListReach = 1.7f;
 constexpr int kListMost = 30;
 
 // The cells near the surface, in `cells` (cells[0 .. *count)).

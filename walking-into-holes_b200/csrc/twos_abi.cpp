@@ -134,6 +134,7 @@ void build_distance_grid(twos_mesh *m, size_t n_tris) {
   for (int a = 0; a < 3; ++a) {
     g.grid_lo[a] = static_cast<float>(m->bmin[a] - h - m->center[a]);
     g.grid_n[a] = static_cast<uint32_t>(n[a]);
+    g.grid_top[a] = static_cast<float>(n[a] - 1);
   }
   g.grid_h = static_cast<float>(h);
   g.grid_inv_h = 1.0f / g.grid_h;

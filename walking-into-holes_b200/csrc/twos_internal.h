@@ -155,6 +155,7 @@ struct GeoDesc {
   float grid_lo[3];
   float grid_h, grid_inv_h, grid_q;
   uint32_t grid_n[3];
+  float grid_top[3];  // grid_n - 1
   // Entry nodes (in the grid's records): the BVH node a query may start
   // from at a point of the cell when its initial bound is below
   // entry_radius (every triangle outside that node's subtree is farther).

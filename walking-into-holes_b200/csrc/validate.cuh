@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(kCertBlock, 6) cert_walk_kernel(const Validate
           best = CUDART_INF;
           float bound, upper;
           int entry = -1;
-          if (G.grid && grid_bounds(G, c.p, bound, upper, entry)) {
+          if (G.grid && grid_bounds<true>(G, c.p, bound, upper, entry)) {
             ub = fminf(ub, __fmaf_ru(6.f, G.delta, upper));
             low = fmax(low, static_cast<double>(bound - G.box_extent - 2.f * c.margin));
           }

@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(kWfStepBlock) wf_step_kernel(const WosLaunch L
       found = false;
       float bound, upper = CUDART_INF_F;
       int entry_node = -1;
-      const bool in_grid = (L.grid_tau > 0.f || L.entry) && G.grid && grid_bounds(G, pos, bound, upper, entry_node);
+      const bool in_grid = (L.grid_tau > 0.f || L.entry) && G.grid && grid_bounds<true>(G, pos, bound, upper, entry_node);
       if (in_grid && L.grid_tau > 0.f && bound >= L.grid_tau * G.grid_h && bound > 2.f * (eps + G.delta) &&
           bound * bound < best2) {
         best2 = bound * bound;
