@@ -1056,10 +1056,10 @@ template <typename T> __host__ __device__ constexpr int wos_stack_entries() {
 }
 
 // A walk's state that its traversal does not touch (position, sums, ids).
-// The mixed form keeps it in registers; the FP64 form, whose state is twice as
-// wide, in shared memory (one word per thread and field, consecutive threads
-// on consecutive words), so the traversal runs without spills: with them, the
-// local memory of 768 threads took the L1 from the BVH's nodes.
+// Its ids are in shared memory (one word per thread and field, consecutive
+// threads on consecutive words), and so is the rest in the FP64 form, whose
+// state is twice as wide; the mixed form keeps what every step changes in
+// registers.
 template <typename V, bool SHARED> struct Cell {
   V v;
   __device__ __forceinline__ operator V() const { return v; }
@@ -1070,10 +1070,10 @@ template <typename V> struct Cell<V, true> {
   __device__ __forceinline__ operator V() const { return *p; }
   __device__ __forceinline__ void operator=(V x) { *p = x; }
 };
-// Shared-memory bytes of that state per thread (both forms: the nearest
+// Shared-memory bytes of that state per thread (both forms: ids, the nearest
 // cavity's distance and index).
 template <typename T> __host__ __device__ constexpr int wos_cold_bytes(bool gradient) {
-  return sizeof(T) == 4 ? 8 : 88 + (gradient ? 96 : 0);
+  return sizeof(T) == 4 ? 24 : 88 + (gradient ? 96 : 0);
 }
 
 enum : int { kIdle = 0, kTraverse = 1, kStep = 2, kBegin = 3, kFirst = 4 };
@@ -1105,13 +1105,17 @@ enum : int { kIdle = 0, kTraverse = 1, kStep = 2, kBegin = 3, kFirst = 4 };
 // ms); and few stack entries in shared memory, which leaves it to the L1
 // (FP64 52 -> 47 ms, mixed 204 -> 201).
 // Residency: the FP32 form with the centre-point source fits 64 registers, so
-// 1024 threads (8 blocks of 128) stay resident per SM; the others take up to
-// 80 (768 threads, 6 blocks of 128; the FP64 form with 64: 50 ms for 47).
+// 1024 threads (8 blocks of 128) stay resident per SM; the other FP32 forms
+// take up to 80 (768 threads), the FP64 form 128 (512 threads: it spills below,
+// and its local memory then shares the L1 with the BVH; 2,000 x 512 walks on
+// 81,920 triangles 39 ms with 80 registers and 32 with 120, the gradient form
+// 4.2 and 2.7).
 template <typename T, int MODE, int SRC>
 constexpr int wos_min_blocks(int block) {
-  return sizeof(T) == 4 && SRC == TWOS_SOURCE_CENTER && MODE != kModeGradient ? 1024 / block
-         : block >= 768                                                      ? 1
-                                                                              : 768 / block;
+  const int threads = sizeof(T) == 8                                      ? 512
+                      : SRC == TWOS_SOURCE_CENTER && MODE != kModeGradient ? 1024
+                                                                           : 768;
+  return threads / block > 1 ? threads / block : 1;
 }
 
 // Walks a lane claims from the work queue at once.
@@ -1182,15 +1186,21 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
   const int units = L.units > 0 ? L.units : 1;
   // Walk state.
   constexpr bool COLD = sizeof(T) == 8;
-  auto cell = [&](auto &c, int word) {  // 8-byte words of the thread's column
+  auto word8 = [&](auto &c, int word) {  // 8-byte words of the thread's column
+    c.p = reinterpret_cast<decltype(c.p)>(s_cold + (word * BLOCK + threadIdx.x) * 8);
+  };
+  auto word4 = [&](auto &c, int word, int h) {  // 4-byte halves of a word, in separate rows
+    c.p = reinterpret_cast<decltype(c.p)>(s_cold + word * BLOCK * 8 + (h * BLOCK + threadIdx.x) * 4);
+  };
+  auto cell = [&](auto &c, int word) {
     if constexpr (COLD)
-      c.p = reinterpret_cast<decltype(c.p)>(s_cold + (word * BLOCK + threadIdx.x) * 8);
+      word8(c, word);
     else
       c.v = 0;
   };
-  auto half = [&](auto &c, int word, int h) {  // 4-byte halves of a word, in separate rows
+  auto half = [&](auto &c, int word, int h) {
     if constexpr (COLD)
-      c.p = reinterpret_cast<decltype(c.p)>(s_cold + word * BLOCK * 8 + (h * BLOCK + threadIdx.x) * 4);
+      word4(c, word, h);
     else
       c.v = 0;
   };
@@ -1204,17 +1214,18 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
 
   uint32_t job = 0;
   Cell<T, COLD> px, py, pz, u, pv, best2;
-  Cell<uint64_t, COLD> wid;
-  Cell<uint32_t, COLD> site, walk, steps, best_tri;  // best_tri: leaf-order index of the walk's nearest triangle
+  Cell<uint64_t, true> wid;
+  Cell<uint32_t, true> site, walk;
+  Cell<uint32_t, COLD> steps, best_tri;  // best_tri: leaf-order index of the walk's nearest triangle
   cell(px, 0);
   cell(py, 1);
   cell(pz, 2);
   cell(u, 3);
   cell(pv, 4);
   cell(best2, 5);
-  cell(wid, 6);
-  half(site, 7, 0);
-  half(walk, 7, 1);
+  word8(wid, COLD ? 6 : 1);
+  word4(site, COLD ? 7 : 2, 0);
+  word4(walk, COLD ? 7 : 2, 1);
   half(steps, 8, 0);
   half(best_tri, 8, 1);
   // Gradient mode: first-ball radius, payoff increments and direction, and
