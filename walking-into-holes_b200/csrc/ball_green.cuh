@@ -101,8 +101,10 @@ __device__ __forceinline__ DD potential_primitive(DD x, DD R, DD A) {
 // The exact ball integral for a bump at distance d from the ball centre;
 // sets `negative` when the difference is below -1e-11 max(1, |N(d)|)
 // (study.cpp:74, which throws there).
-__device__ double exact_bump_green(double d_, double r_, double R_, double A_, bool &negative) {
-  if (d_ >= r_ + R_) return 0.0;
+// Out of line and by value: inlined into both payoffs' term loops, its
+// double-double code made the walk kernels stall on instruction fetch and spill.
+// A negative result beyond round-off comes back as NaN.
+__device__ __noinline__ double exact_bump_green_value(double d_, double r_, double R_, double A_) {
   const DD d = dd(d_), r = dd(r_), R = dd(R_), A = dd(A_);
   const DD at_center = bump_potential(d, R, A);
   DD mean;
@@ -114,8 +116,16 @@ __device__ double exact_bump_green(double d_, double r_, double R_, double A_, b
     mean = (potential_primitive(two_sum(d_, r_), R, A) - potential_primitive(ddabs(two_sum(d_, -r_)), R, A)) /
            (dd(2.0) * d * r);
   const DD value = at_center - mean;
-  if (value.hi < -1e-11 * fmax(1.0, fabs(at_center.hi))) negative = true;
+  if (value.hi < -1e-11 * fmax(1.0, fabs(at_center.hi))) return CUDART_NAN;
   return fmax(0.0, value.hi + value.lo);
+}
+
+__device__ __forceinline__ double exact_bump_green(double d, double r, double R, double A, bool &negative) {
+  if (d >= r + R) return 0.0;
+  const double v = exact_bump_green_value(d, r, R, A);
+  // (fmax above never returns NaN, so NaN marks the negative case alone.)
+  if (isnan(v)) negative = true;
+  return isnan(v) ? 0.0 : v;
 }
 
 }  // namespace twos

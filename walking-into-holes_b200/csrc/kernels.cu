@@ -1106,13 +1106,13 @@ enum : int { kIdle = 0, kTraverse = 1, kStep = 2, kBegin = 3, kFirst = 4 };
 // (FP64 52 -> 47 ms, mixed 204 -> 201).
 // Residency: the FP32 form with the centre-point source fits 64 registers, so
 // 1024 threads (8 blocks of 128) stay resident per SM; the other FP32 forms
-// take up to 80 (768 threads), the FP64 form 128 (512 threads: it spills below,
-// and its local memory then shares the L1 with the BVH; 2,000 x 512 walks on
-// 81,920 triangles 39 ms with 80 registers and 32 with 120, the gradient form
-// 4.2 and 2.7).
+// take up to 80 (768 threads), the FP64 form and the exact ball integrals
+// (double-double) 128 (512 threads: they spill below, and their local memory
+// then shares the L1 with the BVH; 2,000 x 512 FP64 walks on 81,920 triangles
+// 39 ms with 80 registers and 32 with 120, the gradient form 4.2 and 2.7).
 template <typename T, int MODE, int SRC>
 constexpr int wos_min_blocks(int block) {
-  const int threads = sizeof(T) == 8                                      ? 512
+  const int threads = sizeof(T) == 8 || SRC == TWOS_SOURCE_EXACT           ? 512
                       : SRC == TWOS_SOURCE_CENTER && MODE != kModeGradient ? 1024
                                                                            : 768;
   return threads / block > 1 ? threads / block : 1;
