@@ -213,9 +213,11 @@ const char *twos_last_error(void);
  * it, up to 2^30; 0 builds none) holding at each vertex v a lower bound of
  * the distance from v to the surface (the FP32 distance minus twice the
  * mixed form's error bound, rounded down to 1/128 of the spacing h, 16
- * bits), stored as one 16-byte record per cell with the cell's entry node
- * (about 16 bytes per vertex: 4 GB at 2^28 vertices, built in a few
- * seconds).  The distance function is 1-Lipschitz, so D(v) - |x - v| bounds
+ * bits), stored as one 16-byte record per cell with the cell's entry node or
+ * candidate list (about 16 bytes per vertex: 4 GB at 2^28 vertices, and 8
+ * bytes per list entry: up to 2 GB, built in a few seconds).  FP64 queries
+ * start from its upper bound too and prune in FP32; the distances stay the
+ * FP64 minima.  The distance function is 1-Lipschitz, so D(v) - |x - v| bounds
  * the distance at any x from below: a mixed-form step may take that as its
  * ball radius -- the ball still lies in the domain, so the walk stays an
  * unbiased walk-on-spheres -- and skip the closest-point query.  Replaces
@@ -259,10 +261,12 @@ typedef struct twos_tuning {
   int32_t units;         /* traversal units (node visits or triangle tests) a
                             lane runs back to back before its warp returns to
                             the refill and step ballots (1..64).  Default 8. */
-  int32_t entry;         /* mixed form: 1 lets a closest-point query whose
-                            initial bound is below one entry cell start at
-                            the entry-node table's node instead of the root
-                            (same result, fewer node visits); 0 = root. */
+  int32_t entry;         /* 1 lets a closest-point query start from the
+                            distance grid: its upper bound prunes, and near
+                            the surface the search reads its cell's candidate
+                            list, or starts at the cell's entry node (same
+                            result, fewer visits); 0 = unbounded from the
+                            root. */
   int32_t grid_fp64;     /* 1: the FP64 compliance form (centre source) also
                             takes the distance grid's steps and entry nodes,
                             for comparing precision alone; 0 (default): the

@@ -6,16 +6,19 @@
 //                    lengths do not idle a warp.  Replaces the OpenMP site loop
 //                    + evaluate_site/paired_site + walk of the reference
 //                    (wih_twos.cpp:635-717, 1825-1841; adjoint.cpp:18-42).
-//   nearest()        BVH closest-point query used by every step: 16-byte node
-//                    and triangle loads, nearest-child-first order, a traversal
-//                    stack in shared memory, pruning on push and pop.  Replaces
-//                    rtcPointQuery + point_query_callback (wih_twos.cpp:339-359,
-//                    416-430).
+//   nearest()        plain BVH closest-point query: nearest-child-first order,
+//                    pruning on push and pop.  Replaces rtcPointQuery +
+//                    point_query_callback (wih_twos.cpp:339-359, 416-430).
+//                    nearest_geo() and the walk kernel run the same search in
+//                    units with one set of loads for nodes and triangles;
+//                    warp_search() takes one query with a whole warp.
 //   finalize_kernel  one warp per site: FP64 U-statistic, means and the
 //                    leave-one-out jackknife SE over the per-walk samples with
 //                    warp-shuffle reductions in a fixed order (wih_twos.cpp:
 //                    691-715; adjoint.cpp:36-41).
-//   closest_kernel   batched closest point (tests and the queries/s figure).
+//   closest_kernel   batched closest point, a lane (or closest_warp_kernel: a
+//                    warp) per point.
+//   list_*_kernel    the candidate lists of the grid cells near the surface.
 //   grid_build_kernel / grid_bound_kernel
 //                    the mixed form's distance-bound grid: one FP32 closest-
 //                    point query per grid vertex at mesh open, and the bound

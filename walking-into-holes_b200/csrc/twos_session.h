@@ -118,7 +118,7 @@ struct twos_mesh {
   int units = 8;           // traversal units per lane per warp-loop iteration
   int lane_walks = 1;      // walks a lane claims from the queue at once
   uint32_t wavefront = 0;  // > 0: mixed centre-source walks run in the wavefront form with this many slots
-  int entry_start = 1;     // 1: mixed-form queries start at the entry-node table's node
+  int entry_start = 1;     // 1: queries start from the grid's bound, candidate list or entry node
   int grid_fp64 = 0;       // 1: the FP64 compliance form uses the grid and entry nodes too
   int bvh_width = 2;       // mixed form: 2 (binary) or 4 (four-wide) BVH traversal
 };

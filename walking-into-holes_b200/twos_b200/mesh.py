@@ -136,7 +136,8 @@ class Mesh:
         distance-grid bound (in grid spacings) above which a step skips its
         closest-point query, 0 to query every step; units is the number of
         traversal units a lane runs per warp-loop iteration; entry 1 starts
-        qualifying mixed-form queries at the entry-node table's node;
+        queries from the distance grid (its bound, candidate list or entry
+        node);
         grid_fp64 1 gives the FP64 compliance form the grid and entry nodes
         too (a like-for-like comparison of precision); bvh_width 2 or 4 picks
         the mixed form's binary or four-wide BVH traversal; lane_walks is the
