@@ -69,7 +69,8 @@ std::vector<int32_t> build_entry_table(twos_mesh *m);
 
 // Candidate lists of the grid cells near the surface (a few hundred MB for
 // the 4 GB grid of the 327,680-triangle noise sphere, built on the device).
-// A grid whose lists would take more than 2 GB keeps its entry nodes.
+// A grid whose lists would take more than 2 GB, or more than the device has
+// left, keeps its entry nodes: a mesh opens where it did without lists.
 void build_candidate_lists(twos_mesh *m) {
   GeoDesc &g = m->geo_host;
   const uint64_t cells = static_cast<uint64_t>(g.grid_n[0] - 1) * (g.grid_n[1] - 1) * (g.grid_n[2] - 1);
@@ -87,18 +88,27 @@ void build_candidate_lists(twos_mesh *m) {
   check(launch_list_cells(geo, nullptr, 0, word, nullptr), "list cells");
   const uint32_t near = read(0);
   if (near == 0 || near > (1u << 26)) return;  // at most 32 entries a cell: their count fits 32 bits
+  auto room = [](DevBuf &b, size_t bytes) {
+    if (cudaMalloc(&b.ptr, bytes) == cudaSuccess) {
+      b.bytes = bytes;
+      return true;
+    }
+    b.ptr = nullptr;
+    cudaGetLastError();
+    return false;
+  };
   DevBuf ids;
   struct Release {
     DevBuf &b;
     ~Release() { b.release(); }
   } release_ids{ids};
-  ids.reserve(near * sizeof(uint32_t));
+  if (!room(ids, near * sizeof(uint32_t))) return;
   check(cudaMemset(word, 0, sizeof(uint32_t)), "memset");
   check(launch_list_cells(geo, ids.as<uint32_t>(), near, word, nullptr), "list cells");
   check(launch_list_build(geo, ids.as<uint32_t>(), near, nullptr, nullptr, word + 1, word + 4, nullptr), "list sizes");
   const uint32_t entries = read(1);
   if (entries == 0 || entries > (1u << 28) || read(4) != 0) return;
-  m->lists.reserve(entries * sizeof(uint2));
+  if (!room(m->lists, entries * sizeof(uint2))) return;
   check(launch_list_build(geo, ids.as<uint32_t>(), near, m->grid.as<uint4>(), m->lists.as<uint2>(), word + 2, word + 4,
                           nullptr),
         "candidate lists");
