@@ -73,11 +73,11 @@ REF_SUBSET_SEED = 1234
 NCU_WALK_KERNEL = {
     "case": "bench.py --walks 256 --grid 24 --steps 1 --warmup 1 --no-cpu --no-fp64 --no-ablation --no-accuracy "
             "--no-autotune",
-    "lts__throughput_pct": 13.3,
-    "smsp__thread_inst_executed_per_inst_executed": 7.90,
-    "smsp__issue_active_pct": 70.3,
-    "sm__warps_active_pct": 48.2,
-    "lts__t_sector_hit_rate_pct": 73.6,
+    "lts__throughput_pct": 9.6,
+    "smsp__thread_inst_executed_per_inst_executed": 10.41,
+    "smsp__issue_active_pct": 75.5,
+    "sm__warps_active_pct": 48.0,
+    "lts__t_sector_hit_rate_pct": 40.6,
     "wavefront_split": {"step_kernel_threads_per_inst": 24.1, "query_kernel_threads_per_inst": 8.4,
                         "issue_active_pct": 38},
 }
@@ -86,12 +86,12 @@ NCU_WALK_KERNEL = {
 def dram_traffic_per_launch(walks: int) -> float:
     """DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one walk-
     kernel launch, from one single-pass ncu capture of the full workload
-    (default launch tuning): 691.7 GB read + 8.1 GB written for 502,403,072
-    walks, 1,393 B per walk.  With the 2^28-vertex grid (4 GB of cell
+    (default launch tuning): 812.7 GB read + 8.1 GB written for 502,128,640
+    walks, 1,635 B per walk.  With the 2^28-vertex grid (4 GB of cell
     records, entry nodes included) the touched cells no longer fit the 126 MB
-    L2: the reads are grid records; the writes are the per-walk samples.
-    Scaled to the walks of the launch."""
-    return 1392.83 * walks
+    L2: the reads are grid records and candidate lists; the writes are the
+    per-walk samples.  Scaled to the walks of the launch."""
+    return 1634.81 * walks
 
 
 EPSILON = 1e-4
@@ -486,15 +486,14 @@ def run_ours(args):
         tris = np.mean([s["triangle_tests"] for s in s_mixed])
         walks_launch = n * args.walks
         # Bytes the walk kernel must fetch: 96 B per node visit (two child
-        # boxes + normal slabs + child words; 192 B for a four-wide node),
-        # 32 B per triangle plane test
-        # (plane slab + first vertex), 32 B more per full closest-point test
-        # (the other two vertices), counted on the device; four 32 B sectors
-        # per distance-grid lookup (the cell's eight corners lie in four
-        # (i, j) rows; one lookup after every step).
+        # boxes + normal slabs + child words; 192 B for a four-wide node) and
+        # 64 B per triangle (plane slab and vertices; loaded together before
+        # the plane test decides), counted on the device; one 32 B sector per
+        # distance-grid lookup (the cell's 16-byte record; one lookup after
+        # every step).  The 8-byte candidate-list words are left out.
         grid_lookups = steps if info["grid_dims"][0] else 0.0
         node_bytes = 192.0 if tuning.get("bvh_width", 2) == 4 else 96.0
-        fetched = node_bytes * nodes + 32.0 * planes + 32.0 * tris + 32.0 * grid_lookups
+        fetched = node_bytes * nodes + 64.0 * planes + 32.0 * grid_lookups
         bvh_queries = queries - grid_steps
         hbm_peak, hbm_kind = measured_peaks()
         l2_peak = tb.l2_read_gbs(local)
@@ -505,14 +504,14 @@ def run_ours(args):
                 "peak_source": "measured in this run: twos_l2_read_gbs, 32-byte loads from every SM over a "
                                "64 MiB L2-resident buffer (the walk kernel's load form)",
                 "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one full-workload walk-kernel "
-                                  "launch, 1,393 B per walk (grid records read from HBM, per-walk samples "
+                                  "launch, 1,635 B per walk (grid records read from HBM, per-walk samples "
                                   "written), scaled to this launch's walks",
                 "hbm": {"peak": hbm_peak, "peak_source": hbm_kind + " hbm_gbs",
                         "traffic_gbs": traffic / walk_s / 1e9, "frac": traffic / walk_s / 1e9 / hbm_peak},
                 "ncu_walk_kernel": NCU_WALK_KERNEL,
                 "bytes_per_walk": float(fetched / walks_launch),
-                "bytes_definition": "device-counted: 96 B/node visit (192 B four-wide) + 32 B/plane test + 32 B/full "
-                                    "triangle test + 32 B/distance-grid lookup (one 16-byte cell record, one sector; "
+                "bytes_definition": "device-counted: 96 B/node visit (192 B four-wide) + 64 B/triangle reached "
+                                    "+ 32 B/distance-grid lookup (one 16-byte cell record, one sector; "
                                     "one per step)",
                 "distance_evaluations_per_launch": float(queries), "grid_steps_per_launch": float(grid_steps),
                 "bvh_queries_per_launch": float(bvh_queries), "walk_kernel_seconds": walk_s,
@@ -524,7 +523,7 @@ def run_ours(args):
                 "canonical": {"bytes_per_query": CANONICAL_BYTES_PER_QUERY, "source": CANONICAL_SOURCE,
                               "effective_gbs": CANONICAL_BYTES_PER_QUERY * bvh_queries / walk_s / 1e9,
                               "note": "bytes of a plain binary-SAH traversal per BVH query; this traversal "
-                                      "fetches ~18x fewer and the grid skips most queries, so it is not a roof"}}
+                                      "fetches ~200x fewer and the grid skips most queries, so it is not a roof"}}
         accuracy = {}
         if rows64 is not None:
             accuracy["mixed_vs_fp64_z"] = mixed_vs_fp64(rows_mixed, rows64)
