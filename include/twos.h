@@ -234,6 +234,14 @@ void twos_mesh_close(twos_mesh *mesh);
 
 int twos_mesh_get_info(const twos_mesh *mesh, twos_mesh_info *info);
 
+/* The distance grid's candidate lists: cells near the surface that may have
+ * one, cells that do (the others start their queries at an entry node) and
+ * the entries of all lists.  All zero without a grid; no cell has a list where
+ * they would not fit (more than 2 GB, or than the device has left).  No
+ * reference counterpart. */
+int twos_mesh_candidate_lists(const twos_mesh *mesh, uint64_t *near_cells, uint64_t *listed_cells,
+                              uint64_t *entries);
+
 /* Issue the session's work on `stream` (a cudaStream_t of the session's
  * device) instead of its own stream; NULL restores the session's stream.
  * Lets a caller time the kernels with events on its own stream.  No

@@ -1,0 +1,45 @@
+"""Where a closest-point query's bounds are tight: candidate lists that do and
+do not fit, and the limits of the searches."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def tb(lib_built):
+    import twos_b200
+    return twos_b200
+
+
+def _fan(n):
+    """A closed double cone: n triangles meet at each apex."""
+    t = 2 * np.pi * np.arange(n) / n
+    V = np.concatenate([np.c_[np.cos(t), np.sin(t), np.zeros(n)], [[0, 0, 0.5], [0, 0, -0.5]]])
+    i = np.arange(n)
+    j = (i + 1) % n
+    return V, np.concatenate([np.c_[i, j, np.full(n, n)], np.c_[j, i, np.full(n, n + 1)]]).astype(np.uint32)
+
+
+@pytest.mark.parametrize("shape", ["fan4", "sphere3", "noise5", "sliver", "fan64"])
+def test_cells_near_the_surface_have_candidate_lists(tb, monkeypatch, shape):
+    """The grid's cells near the surface have candidate lists -- a list holds
+    its entry node, one triangle at least and its end, 32 entries at most --
+    except where the candidates are too many (around the apex of 64
+    triangles), and a session without a grid has none."""
+    if shape.startswith("fan"):
+        V, F = _fan(int(shape[3:]))
+    elif shape == "sliver":
+        V, F = tb.geometry.icosphere(4)
+        V = V * np.array([1.0, 0.05, 1.0])
+    else:
+        V, F = tb.geometry.icosphere(3) if shape == "sphere3" else tb.geometry.noise_sphere(5, 2)
+    with tb.Mesh(V, F) as m:
+        n = m.candidate_lists()
+    assert 0 < n["listed_cells"] <= n["near_cells"]
+    assert 3 * n["listed_cells"] <= n["entries"] <= 32 * n["listed_cells"]
+    if shape == "fan64":
+        assert n["listed_cells"] < n["near_cells"]
+    monkeypatch.setenv("TWOS_GRID_VERTICES", "0")
+    with tb.Mesh(V, F) as m:
+        assert set(m.candidate_lists().values()) == {0}

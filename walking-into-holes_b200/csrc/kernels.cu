@@ -3060,11 +3060,12 @@ __global__ void __launch_bounds__(256) list_cells_kernel(const GeoDesc *geo, uin
 }
 
 // FILL 0: adds the entries of all lists to *cursor; 1: writes the lists at
-// positions taken from *cursor and points the records at them.
+// positions taken from *cursor, points the records at them and counts them in
+// *listed.
 template <int FILL>
 __global__ void __launch_bounds__(kWosBlock) list_build_kernel(const GeoDesc *geo, const uint32_t *cells, uint32_t n,
                                                                uint4 *grid, uint2 *lists, uint32_t *cursor,
-                                                               uint32_t *error) {
+                                                               uint32_t *listed, uint32_t *error) {
   __shared__ uint2 s_stack[near_entries<double>() * kWosBlock];
   const GeoDesc G = *geo;
   const uint64_t m1 = G.grid_n[1] - 1, m2 = G.grid_n[2] - 1;
@@ -3144,6 +3145,7 @@ __global__ void __launch_bounds__(kWosBlock) list_build_kernel(const GeoDesc *ge
       for (int k = 0; k < held; ++k) out[1 + k] = make_uint2(id[k], __float_as_uint(dist[k]));
       out[1 + held] = make_uint2(0u, 0x7f800000u);
       grid[cell].w = 0x80000000u | at;
+      atomicAdd(listed, 1u);
     }
   }
   if (err) atomicOr(error, err);
@@ -3156,12 +3158,12 @@ cudaError_t launch_list_cells(const GeoDesc *geo_dev, uint32_t *cells, uint32_t 
 }
 
 cudaError_t launch_list_build(const GeoDesc *geo_dev, const uint32_t *cells, uint32_t n, uint4 *grid, uint2 *lists,
-                              uint32_t *cursor, uint32_t *error, cudaStream_t s) {
+                              uint32_t *cursor, uint32_t *listed, uint32_t *error, cudaStream_t s) {
   const int blocks = static_cast<int>(std::min<uint32_t>((n + kWosBlock - 1) / kWosBlock, 148u * 32));
   if (lists)
-    list_build_kernel<1><<<blocks, kWosBlock, 0, s>>>(geo_dev, cells, n, grid, lists, cursor, error);
+    list_build_kernel<1><<<blocks, kWosBlock, 0, s>>>(geo_dev, cells, n, grid, lists, cursor, listed, error);
   else
-    list_build_kernel<0><<<blocks, kWosBlock, 0, s>>>(geo_dev, cells, n, grid, lists, cursor, error);
+    list_build_kernel<0><<<blocks, kWosBlock, 0, s>>>(geo_dev, cells, n, grid, lists, cursor, listed, error);
   return cudaGetLastError();
 }
 

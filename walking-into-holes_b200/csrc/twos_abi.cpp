@@ -77,7 +77,7 @@ void build_candidate_lists(twos_mesh *m) {
   if (cells > 0xffffffffull || !(g.cull_margin > 0.f)) return;
   check(cudaMemcpy(m->geo.ptr, &g, sizeof(GeoDesc), cudaMemcpyHostToDevice), "upload");
   unsigned long long *tot = m->totals.as<unsigned long long>();
-  uint32_t *word = reinterpret_cast<uint32_t *>(tot);  // [0] cells, [1] entries, [2] write cursor, [4] errors
+  uint32_t *word = reinterpret_cast<uint32_t *>(tot);  // [0] cells, [1] entries, [2] write cursor, [3] lists, [4] errors
   check(cudaMemset(tot, 0, 24), "memset");
   const GeoDesc *geo = m->geo.as<GeoDesc>();
   auto read = [&](int i) {
@@ -87,6 +87,7 @@ void build_candidate_lists(twos_mesh *m) {
   };
   check(launch_list_cells(geo, nullptr, 0, word, nullptr), "list cells");
   const uint32_t near = read(0);
+  m->near_cells = near;
   if (near == 0 || near > (1u << 26)) return;  // at most 32 entries a cell: their count fits 32 bits
   auto room = [](DevBuf &b, size_t bytes) {
     if (cudaMalloc(&b.ptr, bytes) == cudaSuccess) {
@@ -105,15 +106,18 @@ void build_candidate_lists(twos_mesh *m) {
   if (!room(ids, near * sizeof(uint32_t))) return;
   check(cudaMemset(word, 0, sizeof(uint32_t)), "memset");
   check(launch_list_cells(geo, ids.as<uint32_t>(), near, word, nullptr), "list cells");
-  check(launch_list_build(geo, ids.as<uint32_t>(), near, nullptr, nullptr, word + 1, word + 4, nullptr), "list sizes");
+  check(launch_list_build(geo, ids.as<uint32_t>(), near, nullptr, nullptr, word + 1, nullptr, word + 4, nullptr),
+        "list sizes");
   const uint32_t entries = read(1);
   if (entries == 0 || entries > (1u << 28) || read(4) != 0) return;
   if (!room(m->lists, entries * sizeof(uint2))) return;
-  check(launch_list_build(geo, ids.as<uint32_t>(), near, m->grid.as<uint4>(), m->lists.as<uint2>(), word + 2, word + 4,
-                          nullptr),
+  check(launch_list_build(geo, ids.as<uint32_t>(), near, m->grid.as<uint4>(), m->lists.as<uint2>(), word + 2, word + 3,
+                          word + 4, nullptr),
         "candidate lists");
   check(cudaDeviceSynchronize(), "candidate lists");
   g.lists = m->lists.as<uint2>();
+  m->listed_cells = read(3);
+  m->list_entries = entries;
   m->resident_bytes += entries * sizeof(uint2);
 }
 
@@ -800,6 +804,14 @@ int twos_mesh_get_info(const twos_mesh *m, twos_mesh_info *info) {
   for (int a = 0; a < 3; ++a) info->grid_dims[a] = m->geo_host.grid ? m->geo_host.grid_n[a] : 0u;
   info->grid_pad = 0;
   info->grid_spacing = m->geo_host.grid ? static_cast<double>(m->geo_host.grid_h) : 0.0;
+  return TWOS_OK;
+}
+
+int twos_mesh_candidate_lists(const twos_mesh *m, uint64_t *near_cells, uint64_t *listed_cells, uint64_t *entries) {
+  if (!m || !near_cells || !listed_cells || !entries) return fail(TWOS_ERR_USAGE, "null argument");
+  *near_cells = m->near_cells;
+  *listed_cells = m->listed_cells;
+  *entries = m->list_entries;
   return TWOS_OK;
 }
 

@@ -103,6 +103,7 @@ struct twos_mesh {
   twos::DevBuf geo;  // one GeoDesc
   twos::GeoDesc geo_host{};
   uint64_t resident_bytes = 0;
+  uint32_t near_cells = 0, listed_cells = 0, list_entries = 0;  // of the candidate lists
   // Scratch, grown on demand.
   twos::DevBuf jobs, geos, terms, cavities, sites, out, u, p, grad, steps, first, counter, totals, points, dist, closest,
       topk, wf;

@@ -29,7 +29,7 @@ EXPORTED = [
     "twos_estimate_batch", "twos_design_loop", "twos_walk_samples", "twos_inside", "twos_topk_device",
     "twos_estimate_noalloc", "twos_mesh_set_tuning", "twos_mesh_get_tuning", "twos_diffwos",
     "twos_ball_green_integral", "twos_validate", "twos_estimate_gradient", "twos_rqmc", "twos_finalize_samples",
-    "twos_l2_read_gbs", "twos_trace_grid_steps", "twos_sobol_directions",
+    "twos_l2_read_gbs", "twos_trace_grid_steps", "twos_sobol_directions", "twos_mesh_candidate_lists",
 ]
 RQMC_MC, RQMC_ARRAY, RQMC_NEIGHBOUR, RQMC_SOBOL = 0, 1, 2, 3
 
@@ -170,6 +170,7 @@ def load(path: Path | str | None = None):
     L.twos_mesh_close.restype = None
     L.twos_mesh_get_info.argtypes = [vp, ctypes.POINTER(MeshInfo)]
     L.twos_mesh_set_stream.argtypes = [vp, vp]
+    L.twos_mesh_candidate_lists.argtypes = [vp, ctypes.POINTER(u64), ctypes.POINTER(u64), ctypes.POINTER(u64)]
     L.twos_closest_point.argtypes = [vp, i32, vp, u64, dbl, vp, vp]
     L.twos_mesh_distance_bound.argtypes = [vp, vp, u64, vp]
     L.twos_estimate.argtypes = [vp, ctypes.POINTER(Request), vp, u32, vp, u32, vp, ctypes.POINTER(Summary)]

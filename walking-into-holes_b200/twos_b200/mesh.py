@@ -166,6 +166,13 @@ class Mesh:
                 "center": list(i.center), "mixed_delta": i.mixed_delta, "build_seconds": i.build_seconds,
                 "device_bytes": i.device_bytes, "grid_dims": list(i.grid_dims), "grid_spacing": i.grid_spacing}
 
+    def candidate_lists(self) -> dict:
+        """The distance grid's candidate lists: cells near the surface, cells
+        with a list, entries of all lists."""
+        n = [ctypes.c_uint64() for _ in range(3)]
+        check(_abi.load().twos_mesh_candidate_lists(self._h, *(ctypes.byref(x) for x in n)))
+        return dict(zip(("near_cells", "listed_cells", "entries"), (x.value for x in n)))
+
     # ------------------------------------------------------------------ queries
     def closest_point(self, points, precision="fp64", query_radius=0.0, with_points=True):
         pts = np.ascontiguousarray(points, dtype=np.float64).reshape(-1, 3)
