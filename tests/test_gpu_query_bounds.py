@@ -43,3 +43,20 @@ def test_cells_near_the_surface_have_candidate_lists(tb, monkeypatch, shape):
     monkeypatch.setenv("TWOS_GRID_VERTICES", "0")
     with tb.Mesh(V, F) as m:
         assert set(m.candidate_lists().values()) == {0}
+
+
+def test_every_open_builds_the_same_lists(tb):
+    """The lists' places in memory are taken in any order; their number and
+    the walks that read them are the same at every open, and those of queries
+    that start at the root."""
+    V, F = tb.geometry.noise_sphere(5, 2)
+    P = tb.geometry.uniform_ball(60, 0.7, seed=3)
+    cfg = tb.Config(walks=200, precision="mixed", seed=5, epsilon=1e-4, max_steps=4096, source=tb.sources.affine())
+    seen = []
+    for entry in (1, 1, 0):
+        with tb.Mesh(V, F) as m:
+            m.set_tuning(**dict(m.get_tuning(), entry=entry))
+            seen.append((m.candidate_lists(), m.estimate(P, cfg)[0]))
+    for n, rows in seen[1:]:
+        assert n == seen[0][0]
+        np.testing.assert_array_equal(rows, seen[0][1])

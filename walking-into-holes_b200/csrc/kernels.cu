@@ -3060,18 +3060,20 @@ __global__ void __launch_bounds__(256) list_cells_kernel(const GeoDesc *geo, uin
 }
 
 // FILL 0: adds the entries of all lists to *cursor; 1: writes the lists at
-// positions taken from *cursor, points the records at them and counts them in
-// *listed.
+// positions taken from *cursor, each list's cell in its first entry and its
+// position in place of the cell in `cells` (kNoList: none).  The records are
+// pointed at the lists by list_point_kernel: this kernel's searches read them.
+constexpr uint32_t kNoList = 0xffffffffu;
 template <int FILL>
-__global__ void __launch_bounds__(kWosBlock) list_build_kernel(const GeoDesc *geo, const uint32_t *cells, uint32_t n,
-                                                               uint4 *grid, uint2 *lists, uint32_t *cursor,
-                                                               uint32_t *listed, uint32_t *error) {
+__global__ void __launch_bounds__(kWosBlock) list_build_kernel(const GeoDesc *geo, uint32_t *cells, uint32_t n,
+                                                               uint2 *lists, uint32_t *cursor, uint32_t *error) {
   __shared__ uint2 s_stack[near_entries<double>() * kWosBlock];
   const GeoDesc G = *geo;
   const uint64_t m1 = G.grid_n[1] - 1, m2 = G.grid_n[2] - 1;
   uint32_t err = 0;
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     const uint64_t cell = cells[t];
+    if (FILL) cells[t] = kNoList;
     const float h = G.grid_h;
     const Vec<float> c{__fmaf_rn(static_cast<float>(cell / (m1 * m2)) + 0.5f, h, G.grid_lo[0]),
                        __fmaf_rn(static_cast<float>(cell / m2 % m1) + 0.5f, h, G.grid_lo[1]),
@@ -3141,14 +3143,28 @@ __global__ void __launch_bounds__(kWosBlock) list_build_kernel(const GeoDesc *ge
     const uint32_t at = atomicAdd(cursor, static_cast<uint32_t>(held + 2));
     if (FILL) {
       uint2 *out = lists + at;
-      out[0] = make_uint2(grid[cell].w, 0u);
+      out[0] = make_uint2(G.grid[cell].w, static_cast<uint32_t>(cell));
       for (int k = 0; k < held; ++k) out[1 + k] = make_uint2(id[k], __float_as_uint(dist[k]));
       out[1 + held] = make_uint2(0u, 0x7f800000u);
-      grid[cell].w = 0x80000000u | at;
-      atomicAdd(listed, 1u);
+      cells[t] = at;
     }
   }
   if (err) atomicOr(error, err);
+}
+
+// Points the records of the cells with lists (positions in `at`) at them and
+// counts them in *listed.
+__global__ void __launch_bounds__(256) list_point_kernel(const uint32_t *at, uint32_t n, uint2 *lists, uint4 *grid,
+                                                         uint32_t *listed) {
+  uint32_t count = 0;
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    if (at[t] == kNoList) continue;
+    uint2 *head = lists + at[t];
+    grid[head->y].w = 0x80000000u | at[t];
+    head->y = 0u;
+    ++count;
+  }
+  if (count) atomicAdd(listed, count);
 }
 
 cudaError_t launch_list_cells(const GeoDesc *geo_dev, uint32_t *cells, uint32_t capacity, uint32_t *count,
@@ -3157,13 +3173,18 @@ cudaError_t launch_list_cells(const GeoDesc *geo_dev, uint32_t *cells, uint32_t 
   return cudaGetLastError();
 }
 
-cudaError_t launch_list_build(const GeoDesc *geo_dev, const uint32_t *cells, uint32_t n, uint4 *grid, uint2 *lists,
+cudaError_t launch_list_build(const GeoDesc *geo_dev, uint32_t *cells, uint32_t n, uint4 *grid, uint2 *lists,
                               uint32_t *cursor, uint32_t *listed, uint32_t *error, cudaStream_t s) {
   const int blocks = static_cast<int>(std::min<uint32_t>((n + kWosBlock - 1) / kWosBlock, 148u * 32));
-  if (lists)
-    list_build_kernel<1><<<blocks, kWosBlock, 0, s>>>(geo_dev, cells, n, grid, lists, cursor, listed, error);
-  else
-    list_build_kernel<0><<<blocks, kWosBlock, 0, s>>>(geo_dev, cells, n, grid, lists, cursor, listed, error);
+  if (!lists) {
+    list_build_kernel<0><<<blocks, kWosBlock, 0, s>>>(geo_dev, cells, n, nullptr, cursor, error);
+    return cudaGetLastError();
+  }
+  list_build_kernel<1><<<blocks, kWosBlock, 0, s>>>(geo_dev, cells, n, lists, cursor, error);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  list_point_kernel<<<static_cast<int>(std::min<uint32_t>((n + 255) / 256, 148u * 8)), 256, 0, s>>>(cells, n, lists,
+                                                                                                 grid, listed);
   return cudaGetLastError();
 }
 

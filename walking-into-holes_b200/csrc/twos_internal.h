@@ -482,10 +482,10 @@ cudaError_t launch_grid_pack(const uint16_t *vertices, const uint32_t n[3], cons
 // Candidate lists: the cells near the surface (count only without `cells`),
 // then the entries of their lists added to *cursor (without `lists`) or the
 // lists themselves, the records in `grid` pointed at them and their number
-// added to *listed.
+// added to *listed (`cells` then holds the lists' positions).
 cudaError_t launch_list_cells(const GeoDesc *geo_dev, uint32_t *cells, uint32_t capacity, uint32_t *count,
                               cudaStream_t s);
-cudaError_t launch_list_build(const GeoDesc *geo_dev, const uint32_t *cells, uint32_t n, uint4 *grid, uint2 *lists,
+cudaError_t launch_list_build(const GeoDesc *geo_dev, uint32_t *cells, uint32_t n, uint4 *grid, uint2 *lists,
                               uint32_t *cursor, uint32_t *listed, uint32_t *error, cudaStream_t s);
 // The walk step's grid bound at each point (original coordinates); NaN
 // outside the grid.
