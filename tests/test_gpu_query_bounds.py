@@ -60,3 +60,23 @@ def test_every_open_builds_the_same_lists(tb):
     for n, rows in seen[1:]:
         assert n == seen[0][0]
         np.testing.assert_array_equal(rows, seen[0][1])
+
+
+@pytest.mark.parametrize("level,jitter", [(1, 0.0), (3, 0.0), (4, 1e-9), (5, 0.0)])
+def test_many_nearly_equidistant_triangles_at_once(tb, level, jitter):
+    """Points at and beside the centre of a sphere, among others: the number of
+    triangles within rounding of the minimum goes from one to far beyond what
+    a warp replays, from point to point of one warp.  Every point gets what a
+    lane's traversal gives it, alone and among others."""
+    V, F = tb.geometry.icosphere(level)
+    rng = np.random.default_rng(level)
+    P = rng.uniform(-0.3, 0.3, (12000, 3))
+    P[::3] = jitter * rng.normal(size=(4000, 3))
+    with tb.Mesh(V, F) as m:
+        d, q = m.closest_point(np.tile(P, (2, 1)), precision="mixed")  # a lane per point
+        dw, qw = m.closest_point(P, precision="mixed")  # a warp per point
+        one = [m.closest_point(P[i:i + 1], precision="mixed") for i in (0, 1, 3)]
+    assert np.array_equal(d[: len(P)], d[len(P):]) and np.array_equal(d[: len(P)], dw)
+    assert np.array_equal(q[: len(P)], qw)
+    for i, (di, qi) in zip((0, 1, 3), one):
+        assert di[0] == dw[i] and np.array_equal(qi[0], qw[i])

@@ -2076,6 +2076,7 @@ __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<float> 
   int root;
   grid_start(g, p, sqrtf(best2), upper, root);
   float limit = fminf(best2, upper * upper), mine = CUDART_INF_F;
+  __syncwarp();  // the previous call's reads of the list are done
   if (lane == 0) *count = 0u;
   warp_search<true>(g, p, root, limit, stack, err, [&](uint32_t i, const float4 *r, float lim) {
     if (!(plane_gap2(r[0], r[1], p) < lim)) return lim;
@@ -2106,9 +2107,16 @@ __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<float> 
     }
   }
   if (n > kContend || held > 32u) {
-    // Too many to replay: the traversal itself, below the cut.
-    best2 = cut;
-    return nearest<float>(g.nodes_f, g.tris_f, g.max_iter, p, best2, best_tri, stack, 1, err, root);
+    // Too many to replay: the traversal itself, below the cut, by one lane
+    // (its stack in the warp's memory).
+    float b = cut;
+    uint32_t t = best_tri, e = 0;
+    bool hit = false;
+    if (lane == 0) hit = nearest<float>(g.nodes_f, g.tris_f, g.max_iter, p, b, t, stack, 1, e, root);
+    best2 = __shfl_sync(full, b, 0);
+    best_tri = __shfl_sync(full, t, 0);
+    err |= __shfl_sync(full, e, 0);
+    return __shfl_sync(full, static_cast<int>(hit), 0) != 0;
   }
   uint32_t tri = 0xffffffffu;
   float d2 = CUDART_INF_F, plane2 = CUDART_INF_F;
@@ -2123,7 +2131,8 @@ __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<float> 
     return true;
   }
   // Replay, by all lanes alike; entries: (node, bound) and the end of the
-  // node's triangle range.
+  // node's triangle range.  The lanes share the stack, so none stores an entry
+  // before all have read the last one there, or reads it before it is stored.
   float r = cut;
   int sp = 0, node = root;
   uint32_t end = 0xffffffffu;
@@ -2155,8 +2164,10 @@ __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<float> 
         const bool swap = dr < dl;
         if (vl && vr) {
           const int far = swap ? cl : cr;
+          __syncwarp();
           stack[2 * sp] = make_uint2(static_cast<uint32_t>(far), __float_as_uint(swap ? dl : dr));
           stack[2 * sp + 1].x = swap ? mid : end;
+          __syncwarp();
           ++sp;
         }
         const bool left = vl && !(vr && swap);
