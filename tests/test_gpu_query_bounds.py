@@ -80,3 +80,61 @@ def test_many_nearly_equidistant_triangles_at_once(tb, level, jitter):
     assert np.array_equal(q[: len(P)], qw)
     for i, (di, qi) in zip((0, 1, 3), one):
         assert di[0] == dw[i] and np.array_equal(qi[0], qw[i])
+
+
+def _cube(n):
+    """A rotated cube of half extent about 1, each face n x n squares of two triangles."""
+    g = np.linspace(-1.0, 1.0, n + 1)
+    i, j = np.meshgrid(np.arange(n), np.arange(n), indexing="ij")
+    a = (i * (n + 1) + j).ravel()
+    quads = np.stack([a, a + n + 1, a + n + 2, a + 1], 1)
+    V, F = [], []
+    for axis in range(3):
+        for side in (-1.0, 1.0):
+            P = np.zeros((n + 1, n + 1, 3))
+            P[..., axis] = side
+            P[..., (axis + 1) % 3], P[..., (axis + 2) % 3] = g[:, None], g[None, :]
+            q = quads if side > 0 else quads[:, ::-1]
+            F.append(np.concatenate([q[:, [0, 1, 2]], q[:, [0, 2, 3]]]) + sum(len(v) for v in V))
+            V.append(P.reshape(-1, 3))
+    R = np.linalg.qr(np.array([[0.8, 0.3, 0.5], [-0.4, 0.9, 0.1], [-0.4, -0.2, 0.9]]))[0]
+    return np.concatenate(V) @ R.T * 0.6, np.concatenate(F).astype(np.uint32)
+
+
+@pytest.mark.parametrize("shape", ["cube8", "cube60", "sphere4", "graded"])
+@pytest.mark.parametrize("query_radius", [0.0, 300.0])
+def test_mixed_queries_far_from_the_mesh(tb, shape, query_radius):
+    """FP32 bounds lose more to rounding the farther the point is: what a warp
+    returns for a point (a small call, a site's first query) stays what a
+    lane's traversal returns, from the surface to 10^4 half extents away."""
+    if shape.startswith("cube"):
+        V, F = _cube(int(shape[4:]))
+    else:
+        V, F = tb.geometry.icosphere(4)
+        if shape == "graded":  # triangles down to 1e-6 of the extent, in a plane
+            V = V * 10.0 ** np.clip(6.0 * (V[:, 2:] - 1.0) / 2.0, -6.0, 0.0)
+    rng = np.random.default_rng(6)
+    out = rng.normal(size=(6000, 3))
+    out /= np.linalg.norm(out, axis=1)[:, None]
+    on = V[F[rng.integers(0, len(F), 6000)].astype(np.int64)].mean(1)  # far along the faces' own normals, too
+    n = np.cross(V[F[:, 1]] - V[F[:, 0]], V[F[:, 2]] - V[F[:, 0]])
+    n = n[rng.integers(0, len(n), 6000)]
+    n /= np.linalg.norm(n, axis=1)[:, None]
+    far = 10.0 ** rng.uniform(-1.0, 4.0, (6000, 1))
+    P = np.concatenate([out * far, on + n * far, out * 2.0 ** rng.integers(0, 14, (6000, 1))])
+    with tb.Mesh(V, F) as m:
+        d, q = m.closest_point(P, precision="mixed", query_radius=query_radius)  # a lane per point
+        parts = [m.closest_point(p, precision="mixed", query_radius=query_radius) for p in np.split(P, 6)]
+        delta = np.float32(m.info()["mixed_delta"])
+        cfg = tb.Config(walks=2, precision="mixed", seed=3, epsilon=1e-30, max_steps=1, query_radius=None,
+                        source=tb.sources.constant(6.0))
+        got = m.walk_samples(P, cfg)["u"][:, 0].astype(np.float32) if query_radius == 0.0 else None
+    dw, qw = (np.concatenate(x) for x in zip(*parts))  # a warp per point
+    if query_radius == 0.0:
+        assert np.all(np.isfinite(d)) and np.all(np.isfinite(q))
+    np.testing.assert_array_equal(dw, d)
+    np.testing.assert_array_equal(qw, q)
+    if got is not None:
+        r = d.astype(np.float32) - delta
+        want = np.where(r > np.float32(1e-30), (r * r / np.float32(6)) * np.float32(6), np.float32(0))
+        np.testing.assert_array_equal(got, want)

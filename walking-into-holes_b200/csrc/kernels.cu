@@ -2061,21 +2061,28 @@ template <typename T> __device__ __forceinline__ void warp_best(T &best, uint32_
 // traversal returns depends on its order, because a node bound can exceed a
 // contained triangle's distance by rounding.  A site's first distance moves
 // all its walks, so the warp's search returns the very value: it collects
-// the triangles within 3 delta of the minimum (bounds are off by less than
-// delta / 2, so no other one can change the outcome), and if there are
-// several, replays the lane's traversal on the nodes that hold them
-// (node_first: a node's first triangle), which are few.
+// the triangles within 3 delta of the minimum, and if there are several,
+// replays the lane's traversal on the nodes that hold them (node_first: a
+// node's first triangle), which are few.  No other triangle can change the
+// outcome while a node bound and a triangle's distance are together off by
+// less than 3 delta, that is 96 * 2^-24 of the mesh's half extent.  Each is off
+// by some 4 * 2^-24 (|p|_1 + half the box's diagonal), so points within eight
+// half extents (|p|_1 <= 2^22 delta) are searched this way and one lane takes
+// the others.  (A cube of 768 triangles and this search at any distance:
+// another triangle, or none, from 48 half extents on.)  Distances to triangles
+// so small beside their distance that FP32 cannot resolve them can be off by
+// more: where the replay then ends without a triangle, the traversal follows.
 constexpr int kContend = 256;
 constexpr int kWarpEntries = kWarpStack + kContend + 1;  // shared-memory entries per warp
-__device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<float> &p, float &best2, uint32_t &best_tri,
-                                             uint2 *stack, uint32_t &err) {
+// The search and the replay: 1 with the nearest triangle, 0 with none below
+// sqrt(from), -1 where the traversal has to decide, below sqrt(cut) if that
+// finds a triangle.
+__device__ __forceinline__ int warp_contenders(const GeoDesc &g, const Vec<float> &p, int root, float from, float &cut,
+                                               float &best2, uint32_t &best_tri, uint2 *stack, uint32_t &err) {
   const unsigned full = 0xffffffffu, lane = threadIdx.x & 31u;
   uint2 *list = stack + kWarpStack;
   uint32_t *count = &list[kContend].x;
-  float upper;
-  int root;
-  grid_start(g, p, sqrtf(best2), upper, root);
-  float limit = fminf(best2, upper * upper), mine = CUDART_INF_F;
+  float limit = from, mine = CUDART_INF_F;
   __syncwarp();  // the previous call's reads of the list are done
   if (lane == 0) *count = 0u;
   warp_search<true>(g, p, root, limit, stack, err, [&](uint32_t i, const float4 *r, float lim) {
@@ -2089,9 +2096,9 @@ __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<float> 
     return widen2(d2, 4.f * g.delta);
   });
   mine = __uint_as_float(__reduce_min_sync(full, __float_as_uint(mine)));
-  if (!(mine < best2)) return false;
+  if (!(mine < best2)) return 0;
   // The contenders, one per lane.
-  const float cut = fminf(best2, widen2(mine, 3.f * g.delta));
+  cut = fminf(best2, widen2(mine, 3.f * g.delta));
   const uint32_t n = *count;
   uint32_t held = 0;
   if (n <= kContend) {
@@ -2106,18 +2113,7 @@ __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<float> 
       __syncwarp();
     }
   }
-  if (n > kContend || held > 32u) {
-    // Too many to replay: the traversal itself, below the cut, by one lane
-    // (its stack in the warp's memory).
-    float b = cut;
-    uint32_t t = best_tri, e = 0;
-    bool hit = false;
-    if (lane == 0) hit = nearest<float>(g.nodes_f, g.tris_f, g.max_iter, p, b, t, stack, 1, e, root);
-    best2 = __shfl_sync(full, b, 0);
-    best_tri = __shfl_sync(full, t, 0);
-    err |= __shfl_sync(full, e, 0);
-    return __shfl_sync(full, static_cast<int>(hit), 0) != 0;
-  }
+  if (n > kContend || held > 32u) return -1;  // too many to replay
   uint32_t tri = 0xffffffffu;
   float d2 = CUDART_INF_F, plane2 = CUDART_INF_F;
   if (lane < held) {
@@ -2125,15 +2121,16 @@ __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<float> 
     d2 = __uint_as_float(list[lane].y);
     plane2 = tri_plane_gap2(g.tris_f, tri, p);
   }
-  best2 = mine;
   if (held == 1u) {
+    best2 = mine;
     best_tri = __shfl_sync(full, tri, 0);
-    return true;
+    return 1;
   }
   // Replay, by all lanes alike; entries: (node, bound) and the end of the
   // node's triangle range.  The lanes share the stack, so none stores an entry
   // before all have read the last one there, or reads it before it is stored.
   float r = cut;
+  bool found = false;
   int sp = 0, node = root;
   uint32_t end = 0xffffffffu;
   for (bool have = true; have;) {
@@ -2147,6 +2144,7 @@ __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<float> 
         if (pg < r && dd < r) {
           r = dd;
           best_tri = i;
+          found = true;
         }
       }
     } else {
@@ -2188,8 +2186,43 @@ __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<float> 
       }
     }
   }
+  if (!found) {
+    cut = from;
+    return -1;
+  }
   best2 = r;
-  return true;
+  return 1;
+}
+
+__device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<float> &p, float &best2, uint32_t &best_tri,
+                                             uint2 *stack, uint32_t &err) {
+  const unsigned full = 0xffffffffu;
+  float upper;
+  int root;
+  grid_start(g, p, sqrtf(best2), upper, root);
+  const float from = fminf(best2, upper * upper);
+  float cut = from;
+  int state = -1;
+  if ((fabsf(p.x) + fabsf(p.y) + fabsf(p.z)) * 0x1.0p-22f <= g.delta)
+    state = warp_contenders(g, p, root, from, cut, best2, best_tri, stack, err);
+  if (state >= 0) return state > 0;
+  // The traversal itself, by one lane (its stack in the warp's memory).
+  uint32_t bits = 0;
+  bool found = false;
+  __syncwarp();
+  if ((threadIdx.x & 31u) == 0u) {
+#pragma unroll 1
+    for (;;) {
+      best2 = cut;
+      found = nearest<float>(g.nodes_f, g.tris_f, g.max_iter, p, best2, best_tri, stack, 1, bits, root);
+      if (found || bits != 0u || !(cut < from)) break;
+      cut = from;
+    }
+  }
+  best2 = __shfl_sync(full, best2, 0);
+  best_tri = __shfl_sync(full, best_tri, 0);
+  err |= __shfl_sync(full, bits, 0);
+  return __shfl_sync(full, static_cast<int>(found), 0) != 0;
 }
 
 __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<double> &p, double &best2,
