@@ -138,3 +138,61 @@ def test_mixed_queries_far_from_the_mesh(tb, shape, query_radius):
         r = d.astype(np.float32) - delta
         want = np.where(r > np.float32(1e-30), (r * r / np.float32(6)) * np.float32(6), np.float32(0))
         np.testing.assert_array_equal(got, want)
+
+
+@pytest.fixture(scope="module")
+def deep():
+    """A closed cone whose rings shrink by a constant factor towards the apex:
+    a BVH of the deepest level the builder allows, 24, all of whose levels hold
+    a stack entry when an unbounded search reaches the leaf nearest to many
+    points (0.2 of those below the apex, 0.1 of those in the cone)."""
+    S, R = 32, 800
+    r = 1e-8 ** (np.arange(R + 1) / R)
+    t = 2 * np.pi * np.arange(S) / S
+    V = np.concatenate([np.c_[x * np.cos(t), x * np.sin(t), np.full(S, x)] for x in r] + [[[0, 0, 1], [0, 0, r[-1]]]])
+    a = (np.arange(R)[:, None] * S + np.arange(S)).ravel()
+    b = (np.arange(R)[:, None] * S + (np.arange(S) + 1) % S).ravel()
+    i, j = np.arange(S), (np.arange(S) + 1) % S
+    F = [np.c_[a, b, b + S], np.c_[a, b + S, a + S], np.c_[np.full(S, (R + 1) * S), j, i],
+         np.c_[np.full(S, (R + 1) * S + 1), R * S + i, R * S + j]]
+    rng = np.random.default_rng(1)
+    z = 10.0 ** rng.uniform(-8.0, 0.0, (10000, 1))
+    inner = np.c_[rng.uniform(-0.6, 0.6, (10000, 2)) * z, z]
+    z = 10.0 ** rng.uniform(-3.0, 1.0, (10000, 1))
+    outer = np.c_[rng.uniform(-0.5, 0.5, (10000, 2)) * z, -z]
+    return V, np.concatenate(F).astype(np.uint32), inner, outer
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("grid", [True, False])
+def test_searches_of_the_deepest_hierarchy(tb, deep, monkeypatch, precision, grid):
+    """A leaf at depth 24 with an entry held at every level is within the stack:
+    closest points (a lane per point against a warp per point) and RQMC, with
+    and without the grid's bounds."""
+    V, F, inner, outer = deep
+    if not grid:
+        monkeypatch.setenv("TWOS_GRID_VERTICES", "0")
+    cfg = tb.Config(walks=64, precision=precision, seed=2, epsilon=1e-5 if precision == "mixed" else 1e-12,
+                    max_steps=4096, source=tb.sources.constant(1.0))
+    with tb.Mesh(V, F) as m:
+        assert m.info()["bvh_depth"] == 24
+        P = np.concatenate([inner, outer])
+        d = m.closest_point(P, precision=precision, with_points=False)
+        assert np.array_equal(d, np.concatenate([m.closest_point(p, precision=precision, with_points=False)
+                                                 for p in np.split(P, 2)]))
+        bu, _, _, _ = m.rqmc(inner[:200], cfg, tb.sources.constant(0.0), tb.sources.constant(0.0), method="mc", batches=2)
+        assert np.all(np.isfinite(bu))
+
+
+@pytest.mark.parametrize("grid", [True, False])
+def test_certified_searches_of_the_deepest_hierarchy(tb, deep, monkeypatch, grid):
+    """Certified walks in the same cone, with and without the grid's bounds."""
+    V, F, inner, _ = deep
+    if not grid:
+        monkeypatch.setenv("TWOS_GRID_VERTICES", "0")
+    cfg = tb.Config(walks=64, precision="fp64", seed=2, epsilon=1e-9, max_steps=8, source=tb.sources.constant(1.0))
+    with tb.Mesh(V, F) as m:
+        sites = inner[m.inside(inner)][:64]
+        s, st, _ = m.validate(sites, cfg, radius_cap=1e3, value_cap=1e9, strict=False)
+    assert len(sites) == 64 and np.all(s["contained"] == 1)
+    assert np.all(s["steps"][st["center_clearance_lower"][:, 0] > 1e-9] > 0)

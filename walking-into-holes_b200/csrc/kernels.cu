@@ -899,7 +899,10 @@ __device__ __noinline__ Plain64 nearest_plain64(const GeoDesc *g, double x, doub
 // grid's bound and entry node; the FP64 form searches in FP32.  A loop of
 // units with one set of loads for nodes and triangles, as the walk kernel's.
 // `stack`: this thread's column of kNearShared traversal entries and, in the
-// FP64 form, kCand candidates; deeper entries are local.
+// FP64 form, kCand candidates; deeper entries are local.  A leaf may be reached
+// with kStack entries held, so an overrun is one entry more, which there is
+// room for until the next unit notices it (likewise in closest_kernel and
+// cert_walk_kernel).
 constexpr int kNearShared = 8;
 template <typename T> __host__ __device__ constexpr int near_entries() {
   return kNearShared + (sizeof(T) == 8 ? kCand : 0);
@@ -909,7 +912,7 @@ __device__ __forceinline__ bool nearest_geo(const GeoDesc &g, const Vec<T> &p, T
                                             uint2 *stack, int stride, uint32_t &err) {
   Cull c{{0.f, 0.f, 0.f}, 0.f, 0.f, 0};
   uint2 *cand = stack + kNearShared * stride;
-  uint2 deep[kStack - kNearShared];
+  uint2 deep[kStack + 1 - kNearShared];
   float upper;
   int node, sp = 0;
   bool found = false, have = true;
@@ -957,8 +960,8 @@ __device__ __forceinline__ bool nearest_geo(const GeoDesc &g, const Vec<T> &p, T
         have = false;
       }
     }
-    if (!done && (++iter > g.max_iter || sp >= kStack)) {
-      err |= sp >= kStack ? TWOS_DEVERR_STACK : TWOS_DEVERR_ITER;
+    if (!done && (++iter > g.max_iter || sp > kStack)) {
+      err |= sp > kStack ? TWOS_DEVERR_STACK : TWOS_DEVERR_ITER;
       done = true;
     }
     if (!done) {
@@ -2776,7 +2779,7 @@ __global__ void __launch_bounds__(kWosBlock) closest_kernel(const GeoDesc *geo, 
   if (threadIdx.x == 0) G = *geo;
   __syncthreads();
   uint2 *stack = s_stack + threadIdx.x, *cand = stack + kLaneStack * kWosBlock;
-  uint2 deep[kStack - kLaneStack];
+  uint2 deep[kStack + 1 - kLaneStack];
   const unsigned lane = threadIdx.x & 31u, full = 0xffffffffu;
   uint32_t err = 0;
   uint64_t i = 0;
@@ -2874,8 +2877,8 @@ __global__ void __launch_bounds__(kWosBlock) closest_kernel(const GeoDesc *geo, 
           have = false;
         }
       }
-      if (++iter > G.max_iter || sp >= kStack) {
-        err |= sp >= kStack ? TWOS_DEVERR_STACK : TWOS_DEVERR_ITER;
+      if (++iter > G.max_iter || sp > kStack) {
+        err |= sp > kStack ? TWOS_DEVERR_STACK : TWOS_DEVERR_ITER;
         have = false;
         sp = 0;
         tri_cur = tri_end;

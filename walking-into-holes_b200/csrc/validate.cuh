@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(kCertBlock, 6) cert_walk_kernel(const Validate
   if (threadIdx.x == 0) G = *V.geo;
   __syncthreads();
   uint2 *stack = s_stack + threadIdx.x, *cand = stack + kCertStack * kCertBlock;
-  uint2 deep[kStack - kCertStack];
+  uint2 deep[kStack + 1 - kCertStack];
   const unsigned lane = threadIdx.x & 31u, full = 0xffffffffu;
   const bool on = static_cast<int>(lane) < lanes;
   const unsigned on_mask = __ballot_sync(full, on);
@@ -349,8 +349,8 @@ __global__ void __launch_bounds__(kCertBlock, 6) cert_walk_kernel(const Validate
           have = false;
         }
       }
-      if (++iter > G.max_iter || sp >= kStack) {
-        err |= sp >= kStack ? TWOS_DEVERR_STACK : TWOS_DEVERR_ITER;
+      if (++iter > G.max_iter || sp > kStack) {
+        err |= sp > kStack ? TWOS_DEVERR_STACK : TWOS_DEVERR_ITER;
         best = 0.0;  // fail closed: a zero distance ends the walk
         c.count = 0;
         phase = kStep;
