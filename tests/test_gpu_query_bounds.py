@@ -1,5 +1,7 @@
 """Where a closest-point query's bounds are tight: candidate lists that do and
 do not fit, and the limits of the searches."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -196,3 +198,25 @@ def test_certified_searches_of_the_deepest_hierarchy(tb, deep, monkeypatch, grid
         s, st, _ = m.validate(sites, cfg, radius_cap=1e3, value_cap=1e9, strict=False)
     assert len(sites) == 64 and np.all(s["contained"] == 1)
     assert np.all(s["steps"][st["center_clearance_lower"][:, 0] > 1e-9] > 0)
+
+
+def test_a_certified_first_distance_that_overruns_is_zero(tb, monkeypatch):
+    """A search that gives up certifies nothing: a site whose first distance
+    overruns the iteration bound (the centre of a sphere, equidistant to all of
+    it; the bound lowered to a hundredth of the visits) has clearance 0, its
+    walks take no step, and the call reports the overrun."""
+    V, F = tb.geometry.icosphere(5)
+    monkeypatch.setenv("TWOS_MAX_ITERATIONS", "200")
+    req = tb.Config(walks=64, precision="fp64", seed=2, epsilon=1e-6, max_steps=32,
+                    source=tb.sources.constant(1.0)).to_request()
+    site = np.zeros((1, 3))
+    abi = tb._abi
+    samples = np.zeros((1, 64), dtype=abi.CERT_SAMPLE_DTYPE)
+    stages = np.zeros((1, abi.VALIDATE_MAX_STAGES), dtype=abi.VALIDATE_STAGE_DTYPE)
+    params, n, summ = abi.ValidateParams(0.1, 10.0), ctypes.c_uint32(), abi.Summary()
+    with tb.Mesh(V, F) as m:
+        rc = abi.load().twos_validate(m._h, ctypes.byref(req), ctypes.byref(params), site.ctypes.data, 1, None, 0,
+                                      samples.ctypes.data, stages.ctypes.data, ctypes.byref(n), ctypes.byref(summ))
+    assert rc != abi.OK and summ.error_flags & abi.DEVERR_ITER
+    assert n.value >= 1 and stages["center_clearance_lower"][0, 0] == 0.0
+    assert np.all(samples["steps"] == 0) and np.all(samples["value"] == 0.0)

@@ -334,6 +334,10 @@ int open_impl(std::vector<double> &&v, std::vector<uint32_t> &&f, int device, tw
     m->counter.reserve(16);
     m->totals.reserve(64);
     build_distance_grid(m.get(), tf.size());
+    // A smaller bound for the session's searches: how an overrun is reported
+    // can be seen.
+    if (const char *e = std::getenv("TWOS_MAX_ITERATIONS"))
+      g.max_iter = static_cast<uint32_t>(std::min<uint64_t>(g.max_iter, std::max<uint64_t>(1, std::strtoull(e, nullptr, 10))));
     check(cudaMemcpy(m->geo.ptr, &g, sizeof(GeoDesc), cudaMemcpyHostToDevice), "upload");
     m->build_seconds = seconds_since(t0);
     if (const char *e = std::getenv("TWOS_MAX_LAUNCH_WALKS")) m->max_launch_walks = std::strtoull(e, nullptr, 10);

@@ -493,7 +493,8 @@ __global__ void __launch_bounds__(kWosBlock) validate_center_kernel(const Valida
     if (cull_begin(G, v, best2, c)) {
       // Boxes contain their triangles: the exact distance bounds this one.
       float limit = c.limit;
-      warp_search<false>(G, c.p, 0, limit, stack, err, [&](uint32_t i, const float4 *r, float lim) {
+      uint32_t overrun = 0;
+      warp_search<false>(G, c.p, 0, limit, stack, overrun, [&](uint32_t i, const float4 *r, float lim) {
         const float gx = gap(fminf(fminf(r[1].x, r[2].x), r[3].x), fmaxf(fmaxf(r[1].x, r[2].x), r[3].x), c.p.x);
         const float gy = gap(fminf(fminf(r[1].y, r[2].y), r[3].y), fmaxf(fmaxf(r[1].y, r[2].y), r[3].y), c.p.y);
         const float gz = gap(fminf(fminf(r[1].z, r[2].z), r[3].z), fmaxf(fmaxf(r[1].z, r[2].z), r[3].z), c.p.z);
@@ -502,6 +503,8 @@ __global__ void __launch_bounds__(kWosBlock) validate_center_kernel(const Valida
         return cull_limit(dm * dm, c.margin);
       });
       warp_best(dm, tri);
+      err |= overrun;
+      if (overrun) dm = 0.0;  // fail closed, as cv_mesh_distance: the site's walks end at once
     } else {
       dm = cv_mesh_distance(G, p, err);
     }
