@@ -220,3 +220,22 @@ def test_a_certified_first_distance_that_overruns_is_zero(tb, monkeypatch):
     assert rc != abi.OK and summ.error_flags & abi.DEVERR_ITER
     assert n.value >= 1 and stages["center_clearance_lower"][0, 0] == 0.0
     assert np.all(samples["steps"] == 0) and np.all(samples["value"] == 0.0)
+
+
+@pytest.mark.parametrize("radius_cap", [0.02, 0.3])
+def test_certified_walks_among_more_boxes_than_a_query_holds(tb, oracle_mod, radius_cap):
+    """Around an apex where 64 triangles meet, a query's candidates are tested
+    several times before it ends: the oracle's steps and flags exactly, its
+    values to the parity tests' 1e-10."""
+    V, F = _fan(64)
+    sites = np.array([[0.0, 0.0, 0.45], [0.01, 0.0, -0.4], [0.02, -0.03, 0.2]])
+    common = dict(walks=200, seed=9, epsilon=1e-6, max_steps=96, cavity_radius=0.05)
+    cfg = tb.Config(precision="fp64", green=True, source=tb.sources.constant(1.0), **common)
+    with tb.Mesh(V, F) as m:
+        s, st, _ = m.validate(sites, cfg, radius_cap=radius_cap, value_cap=0.2, strict=False)
+    o = oracle_mod.OracleMesh(V, F).validate(sites, radius_cap, 0.2, rng=oracle_mod.RNG_COUNTER, green=True,
+                                             source=[oracle_mod.term(oracle_mod.TERM_CONST, 1.0)], **common)
+    for k in ("steps", "capped", "clipped", "contained"):
+        assert np.array_equal(s[k].astype(o[k].dtype), o[k]), k
+    np.testing.assert_allclose(s["value"], o["value"], rtol=1e-10, atol=0)
+    assert np.array_equal(st["center_clearance_lower"][:, 0], o["clearance"])

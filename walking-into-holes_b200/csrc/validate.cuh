@@ -232,12 +232,12 @@ __global__ void __launch_bounds__(kCertBlock, 6) cert_walk_kernel(const Validate
         if (__uint_as_float(e.y) < c.limit) best = fmin(best, cv_tri_box(G, e.x, pt));
       }
       c.count = 0;
-      low = fmax(low, fmin(best, far));
       if (resume && best > 0.0) {
         resume = false;
-        phase = kTraverse;
+        phase = kTraverse;  // `best` is the smallest so far: no bound from below yet
       } else {
         resume = false;
+        low = fmax(low, fmin(best, far));
         double d = fmin(best, fmax(low, far));
         for (uint32_t i = 0; i < V.n_cav; ++i)
           d = fmin(d, cv_dn(cv_point_distance(pt, V.cavities + 3 * i, false) - V.cavity_radius));
