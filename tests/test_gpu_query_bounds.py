@@ -239,3 +239,32 @@ def test_certified_walks_among_more_boxes_than_a_query_holds(tb, oracle_mod, rad
         assert np.array_equal(s[k].astype(o[k].dtype), o[k]), k
     np.testing.assert_allclose(s["value"], o["value"], rtol=1e-10, atol=0)
     assert np.array_equal(st["center_clearance_lower"][:, 0], o["clearance"])
+
+
+@pytest.mark.parametrize("k", [30, 34, 37])
+@pytest.mark.parametrize("level", [1, 4])
+def test_a_scaled_mesh_gives_scaled_results(tb, monkeypatch, level, k):
+    """A power of two times every length is a power of two times every FP64
+    distance and estimate, bit for bit, and leaves the steps alone, also where
+    FP32 has no room for the products of the closest-point arithmetic.  The
+    mixed form's distances there are those of a session without a grid."""
+    V, F = tb.geometry.icosphere(level)
+    rng = np.random.default_rng(level)
+    P = rng.uniform(-0.9, 0.9, (20000, 3))
+    sites = 0.5 * rng.uniform(-1, 1, (24, 3))
+    cav = np.array([[0.3, 0.1, 0.0], [-0.4, 0.2, 0.1]])
+    got = []
+    for a in (1.0, 2.0 ** k):
+        cfg = tb.Config(walks=100, precision="fp64", seed=7, epsilon=1e-4 * a, max_steps=4096, cavity_radius=0.1 * a,
+                        query_radius=None, source=tb.sources.constant(1.0))
+        with tb.Mesh(V * a, F) as m:
+            d = [m.closest_point(p * a, precision="fp64", with_points=False) / a for p in (P, P[:500])]
+            rows, _ = m.estimate(sites * a, cfg, cavities=cav * a)
+            f = [m.closest_point(p * a, precision="mixed", with_points=False) for p in (P, P[:500])]
+        got.append((*d, rows["u"] / a**2, rows["steps"]))
+    for x, y in zip(*got):
+        np.testing.assert_array_equal(x, y)
+    monkeypatch.setenv("TWOS_GRID_VERTICES", "0")
+    with tb.Mesh(V * a, F) as m:
+        for x, p in zip(f, (P, P[:500])):
+            np.testing.assert_array_equal(x, m.closest_point(p * a, precision="mixed", with_points=False))

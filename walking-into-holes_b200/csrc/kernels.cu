@@ -766,7 +766,9 @@ __device__ __forceinline__ float cull_limit(double best2, float margin) {
 
 // Sets up the search at p for distances below sqrt(best2); false when FP32
 // cannot hold the geometry or the point (cull_margin 0: see open_impl; a
-// coordinate beyond 2^50, whose square would overflow, or NaN), and the
+// coordinate beyond 2^50, whose square would overflow, or NaN; a distance
+// whose product with an edge may be beyond 2^60, where the squares of such
+// products overflow: cull_margin is at least 2^-19 half extents), and the
 // caller takes the FP64 nodes.
 __device__ __forceinline__ bool cull_begin(const GeoDesc &g, const Vec<double> &p, double best2, Cull &c) {
   const double xyz[3] = {p.x, p.y, p.z};
@@ -775,7 +777,7 @@ __device__ __forceinline__ bool cull_begin(const GeoDesc &g, const Vec<double> &
   c.margin = __fmaf_ru(norm1, 0x1.0p-20f, g.cull_margin);
   c.limit = cull_limit(best2, c.margin);
   c.count = 0;
-  return g.cull_margin > 0.f && norm1 < 0x1.0p50f;
+  return g.cull_margin > 0.f && norm1 < 0x1.0p50f && (norm1 + 0x1.0p20f * g.cull_margin) * g.box_extent < 0x1.0p60f;
 }
 
 // A point of the triangle at (nearly) its closest to p: Ericson's regions as
@@ -863,14 +865,16 @@ __device__ __forceinline__ bool cull_tri(uint32_t i, const float4 &P, const floa
 // bound plus 6 delta (its 3 delta and the query's own error, with room) is
 // above the distance, so the traversal may prune with it before any triangle
 // is found; when the initial bound is below one entry cell, it starts at the
-// cell's entry node (every triangle outside that subtree is farther).
+// cell's entry node (every triangle outside that subtree is farther).  A
+// geometry FP32 cannot hold (cull_margin 0) has no bounds: its FP32 distances
+// overflow for some triangles, at a grid vertex for others than at p.
 __device__ __forceinline__ void grid_start(const GeoDesc &g, const Vec<float> &p, float radius, float &upper,
                                            int &node) {
   float bound;
   int entry = -1;
   upper = CUDART_INF_F;
   node = 0;
-  if (!g.grid || !grid_bounds<true>(g, p, bound, upper, entry)) {
+  if (!g.grid || !(g.cull_margin > 0.f) || !grid_bounds<true>(g, p, bound, upper, entry)) {
     upper = CUDART_INF_F;
     return;
   }

@@ -327,6 +327,11 @@ int open_impl(std::vector<double> &&v, std::vector<uint32_t> &&f, int device, tw
       extent2 = std::max(extent2, d2);
     }
     g.box_extent = static_cast<float>(1.0001 * std::sqrt(extent2));
+    // The closest-point arithmetic multiplies products of an edge and a
+    // vertex's distance from the point: beyond 2^60 for a point of the padded
+    // box (at most 8 half extents from any vertex), FP32 has no room for their
+    // squares, and the distance grid's values are no bounds.
+    if (!(8.0 * reach * std::sqrt(extent2) < 0x1p60)) g.cull_margin = 0.f;
     // A query visits each node and tests each triangle at most once.
     g.max_iter = static_cast<uint32_t>(
         std::min<uint64_t>(2ull * (m->bvh.nodes.size() + m->faces.size() / 3) + 16, 0xffffffffull));
