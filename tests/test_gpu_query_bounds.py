@@ -268,3 +268,59 @@ def test_a_scaled_mesh_gives_scaled_results(tb, monkeypatch, level, k):
     with tb.Mesh(V * a, F) as m:
         for x, p in zip(f, (P, P[:500])):
             np.testing.assert_array_equal(x, m.closest_point(p * a, precision="mixed", with_points=False))
+
+
+@pytest.mark.parametrize("k", [-38, -34, -32, -28])
+@pytest.mark.parametrize("level", [1, 3])
+def test_a_small_mesh_gives_scaled_results(tb, level, k):
+    """The same where the products of the closest-point arithmetic are below
+    FP32's normal numbers and the grid's values far off: searches that find
+    nothing below its bound are made without it."""
+    V, F = tb.geometry.icosphere(level)
+    rng = np.random.default_rng(level)
+    P = rng.uniform(-0.9, 0.9, (20000, 3))
+    sites = 0.5 * rng.uniform(-1, 1, (24, 3))
+    got = []
+    for a in (1.0, 2.0 ** k):
+        cfg = tb.Config(walks=100, precision="fp64", seed=7, epsilon=1e-4 * a, max_steps=4096, query_radius=None,
+                        source=tb.sources.constant(1.0))
+        with tb.Mesh(V * a, F) as m:
+            d = [m.closest_point(p * a, precision="fp64", with_points=False) / a for p in (P, P[:500])]
+            rows, _ = m.estimate(sites * a, cfg)
+        got.append((*d, rows["u"] / a**2, rows["steps"]))
+    for x, y in zip(*got):
+        np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_walks_between_needles(tb, monkeypatch, precision):
+    """A cylinder of 3,000 segments: triangles a thousand times longer than
+    high, whose FP32 distances at the grid's vertices can be below those at
+    the points of a walk.  Every query is answered; the FP64 samples, and all
+    closest points, are those without the grid.  (Without it a mixed walk can
+    run out of the solid on such triangles.)"""
+    n = 3000
+    t = 2 * np.pi * np.arange(n) / n
+    V = np.concatenate([np.c_[np.cos(t), np.sin(t), np.full(n, -1.0)], np.c_[np.cos(t), np.sin(t), np.full(n, 1.0)],
+                        [[0, 0, -1], [0, 0, 1]]])
+    i, j = np.arange(n), (np.arange(n) + 1) % n
+    F = np.concatenate([np.c_[i, j, j + n], np.c_[i, j + n, i + n], np.c_[j, i, np.full(n, 2 * n)],
+                        np.c_[i + n, j + n, np.full(n, 2 * n + 1)]]).astype(np.uint32)
+    R = np.linalg.qr(np.random.default_rng(3).normal(size=(3, 3)))[0]
+    rng = np.random.default_rng(6)
+    S, P = rng.uniform(-0.5, 0.5, (200, 3)) @ R.T, rng.uniform(-1.3, 1.3, (20000, 3)) @ R.T
+    cfg = tb.Config(epsilon=1e-4, max_steps=2000, query_radius=None, walks=64, precision=precision, seed=7,
+                    source=tb.sources.constant(1.0))
+    got = []
+    for grid in (True, False):
+        if not grid:
+            monkeypatch.setenv("TWOS_GRID_VERTICES", "0")
+        with tb.Mesh(V @ R.T, F) as m:
+            got.append((m.closest_point(P, precision=precision, with_points=False),
+                        m.closest_point(P[:4000], precision=precision, with_points=False),
+                        m.walk_samples(S, cfg) if grid or precision == "fp64" else None))
+    for x, y in zip(got[0][:2], got[1][:2]):
+        np.testing.assert_array_equal(x, y)
+    if precision == "fp64":
+        for key in got[0][2]:
+            np.testing.assert_array_equal(got[0][2][key], got[1][2][key])

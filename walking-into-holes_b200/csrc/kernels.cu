@@ -868,6 +868,13 @@ __device__ __forceinline__ bool cull_tri(uint32_t i, const float4 &P, const floa
 // cell's entry node (every triangle outside that subtree is farther).  A
 // geometry FP32 cannot hold (cull_margin 0) has no bounds: its FP32 distances
 // overflow for some triangles, at a grid vertex for others than at p.
+//
+// The grid's upper bound comes from FP32 distances at its vertices.  Where FP32
+// cannot evaluate a triangle (edges a thousand times longer than its height;
+// products below the smallest normal number) its interior point is anywhere
+// in its plane, and the bound can be below the distance.  So a search takes
+// the bound as a distance to be found below, and one that finds none below it
+// is made again without it.
 __device__ __forceinline__ void grid_start(const GeoDesc &g, const Vec<float> &p, float radius, float &upper,
                                            int &node) {
   float bound;
@@ -899,6 +906,17 @@ __device__ __noinline__ Plain64 nearest_plain64(const GeoDesc *g, double x, doub
   return r;
 }
 
+// The same, as nearest_geo().
+__device__ __forceinline__ bool nearest_plain(const GeoDesc &g, const Vec<double> &p, double &best2,
+                                              uint32_t &best_tri, uint32_t &err) {
+  const Plain64 r = nearest_plain64(&g, p.x, p.y, p.z, best2);
+  err |= r.flags & 0x7fffffffu;
+  if (!(r.flags >> 31)) return false;
+  best2 = r.best2;
+  best_tri = r.tri;
+  return true;
+}
+
 // Closest-point query outside the walk kernel, as nearest(), from the distance
 // grid's bound and entry node; the FP64 form searches in FP32.  A loop of
 // units with one set of loads for nodes and triangles, as the walk kernel's.
@@ -920,22 +938,17 @@ __device__ __forceinline__ bool nearest_geo(const GeoDesc &g, const Vec<T> &p, T
   float upper;
   int node, sp = 0;
   bool found = false, have = true;
+  const T from = best2;
   if constexpr (sizeof(T) == 4) {
     c.p = p;
     grid_start(g, c.p, sqrtf(best2), upper, node);
     best2 = fminf(best2, upper * upper);
   } else {
-    if (!cull_begin(g, p, best2, c)) {
-      const Plain64 r = nearest_plain64(&g, p.x, p.y, p.z, best2);
-      err |= r.flags & 0x7fffffffu;
-      if (!(r.flags >> 31)) return false;
-      best2 = r.best2;
-      best_tri = r.tri;
-      return true;
-    }
+    if (!cull_begin(g, p, best2, c)) return nearest_plain(g, p, best2, best_tri, err);
     grid_start(g, c.p, sqrtf(c.limit), upper, node);
-    const float reach = __fadd_ru(upper, c.margin);
-    c.limit = fminf(c.limit, __fmul_ru(reach, reach));
+    const float reach = __fadd_ru(upper, c.margin), reach2 = __fmul_ru(reach, reach);
+    c.limit = fminf(c.limit, reach2);
+    best2 = fmin(best2, static_cast<double>(reach2));
   }
   uint32_t tri_cur = 0, tri_end = 0, iter = 0;
 #pragma unroll 1
@@ -967,6 +980,7 @@ __device__ __forceinline__ bool nearest_geo(const GeoDesc &g, const Vec<T> &p, T
     if (!done && (++iter > g.max_iter || sp > kStack)) {
       err |= sp > kStack ? TWOS_DEVERR_STACK : TWOS_DEVERR_ITER;
       done = true;
+      best2 = fmax(best2, from);  // no second search
     }
     if (!done) {
       const bool on_tri = tri_cur < tri_end;
@@ -1014,7 +1028,15 @@ __device__ __forceinline__ bool nearest_geo(const GeoDesc &g, const Vec<T> &p, T
     if constexpr (sizeof(T) == 8) {
       if (flush || done) found |= cull_flush(g, p, c, best2, best_tri, cand, stride);
     }
-    if (done) break;
+    if (done) {
+      if (found || !(best2 < from)) break;
+      // None below the grid's bound (grid_start): without it, from the root.
+      best2 = from;
+      if constexpr (sizeof(T) == 8) c.limit = cull_limit(from, c.margin);
+      node = sp = 0;
+      have = true;
+      tri_cur = tri_end = iter = 0;
+    }
   }
   return found;
 }
@@ -1086,7 +1108,7 @@ template <typename T> __host__ __device__ constexpr int wos_cold_bytes(bool grad
   return sizeof(T) == 4 ? 24 : 88 + (gradient ? 96 : 0);
 }
 
-enum : int { kIdle = 0, kTraverse = 1, kStep = 2, kBegin = 3, kFirst = 4 };
+enum : int { kIdle = 0, kTraverse = 1, kStep = 2, kBegin = 3, kFirst = 4, kAgain = 5 };
 
 // Persistent walk-on-spheres kernel as a per-lane state machine.  Each loop
 // iteration every traversing lane runs up to `units` units of work back to
@@ -1366,11 +1388,16 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
         list = is_list(entry_node);
         if (!list && entry_node >= 0 && ubs < G.entry_radius) node = entry_node;
       }
+      // A triangle is to be found below the bound (see the step).
       if constexpr (sizeof(T) == 4) {
         best2 = fminf(best2, ubs * ubs);
       } else {
-        const float reach = __fadd_ru(ubs, cull.margin);
-        cull.limit = fminf(cull.limit, __fmul_ru(reach, reach));
+        const float reach = __fadd_ru(ubs, cull.margin), reach2 = __fmul_ru(reach, reach);
+        cull.limit = fminf(cull.limit, reach2);
+        if (static_cast<double>(reach2) < best2) {
+          best2 = static_cast<double>(reach2);
+          found = false;
+        }
       }
     }
     set_best2(best2);
@@ -1537,6 +1564,17 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
             phase = kTraverse;
             break;
           }
+          if (!found && static_cast<T>(best2) < static_cast<T>(J.query_radius2)) {
+            // None below the grid's bound (grid_start).  Where a mixed
+            // search has gone on from the previous triangle and an entry node,
+            // the bound is the distance; else the search is made without it.
+            if (sizeof(T) == 4 && L.warm && tri_ok && sqrtf(static_cast<float>(best2)) < G.entry_radius)
+              found = true;
+            else
+              phase = kAgain;
+          }
+        }
+        if (phase == kStep) {
           T d = sqrt(static_cast<T>(best2));
           if (!found) {
             err |= TWOS_DEVERR_QUERY;
@@ -1747,7 +1785,7 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
             break;
           }
         }
-        begin_query(J, G, pos, in_grid && L.entry, bound, upper, entry_node, dc);
+        begin_query(J, G, pos, in_grid && L.entry && phase != kAgain, bound, upper, entry_node, dc);
       } while (false);
     }
 
@@ -1781,6 +1819,7 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
       auto fail = [&](uint32_t bit) {
         err |= bit;
         found = false;
+        set_best2(static_cast<T>(CUDART_INF_F));
         cull.count = 0;
         resume = false;
         phase = kStep;
@@ -2207,12 +2246,16 @@ __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<float> 
   float upper;
   int root;
   grid_start(g, p, sqrtf(best2), upper, root);
-  const float from = fminf(best2, upper * upper);
+  const float given = best2, from = fminf(given, upper * upper);
   float cut = from;
   int state = -1;
   if ((fabsf(p.x) + fabsf(p.y) + fabsf(p.z)) * 0x1.0p-22f <= g.delta)
     state = warp_contenders(g, p, root, from, cut, best2, best_tri, stack, err);
-  if (state >= 0) return state > 0;
+  if (state > 0 || (state == 0 && !(from < given))) return state > 0;
+  if (state == 0) {  // none below the grid's bound: without it, from the root
+    cut = given;
+    root = 0;
+  }
   // The traversal itself, by one lane (its stack in the warp's memory).
   uint32_t bits = 0;
   bool found = false;
@@ -2222,8 +2265,9 @@ __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<float> 
     for (;;) {
       best2 = cut;
       found = nearest<float>(g.nodes_f, g.tris_f, g.max_iter, p, best2, best_tri, stack, 1, bits, root);
-      if (found || bits != 0u || !(cut < from)) break;
-      cut = from;
+      if (found || bits != 0u || !(cut < given)) break;
+      if (!(cut < from)) root = 0;
+      cut = cut < from ? from : given;
     }
   }
   best2 = __shfl_sync(full, best2, 0);
@@ -2235,22 +2279,15 @@ __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<float> 
 __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<double> &p, double &best2,
                                              uint32_t &best_tri, uint2 *stack, uint32_t &err) {
   Cull c;
-  if (!cull_begin(g, p, best2, c)) {
-    const Plain64 r = nearest_plain64(&g, p.x, p.y, p.z, best2);
-    err |= r.flags & 0x7fffffffu;
-    if (!(r.flags >> 31)) return false;
-    best2 = r.best2;
-    best_tri = r.tri;
-    return true;
-  }
+  if (!cull_begin(g, p, best2, c)) return nearest_plain(g, p, best2, best_tri, err);
   float upper;
   int node;
   grid_start(g, c.p, sqrtf(c.limit), upper, node);
-  const float reach = __fadd_ru(upper, c.margin);
-  float limit = fminf(c.limit, __fmul_ru(reach, reach));
-  double mine = best2;
-  uint32_t tri = 0xffffffffu;
-  warp_search<true>(g, c.p, node, limit, stack, err, [&](uint32_t i, const float4 *r, float lim) {
+  const float reach = __fadd_ru(upper, c.margin), reach2 = __fmul_ru(reach, reach);
+  float limit = fminf(c.limit, reach2);
+  double mine = fmin(best2, static_cast<double>(reach2));
+  uint32_t tri = 0xffffffffu, overrun = 0;
+  warp_search<true>(g, c.p, node, limit, stack, overrun, [&](uint32_t i, const float4 *r, float lim) {
     if (!(plane_gap2(r[0], r[1], c.p) < lim)) return lim;
     Vec<double> ta, tb, tc;
     load_tri(g.tris_d, i, ta, tb, tc);
@@ -2261,7 +2298,9 @@ __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<double>
     return cull_limit(d2, c.margin);
   });
   warp_best(mine, tri);
-  if (tri == 0xffffffffu) return false;
+  err |= overrun;
+  if (tri == 0xffffffffu)
+    return overrun == 0u && reach2 < best2 && nearest_plain(g, p, best2, best_tri, err);
   best2 = mine;
   best_tri = tri;
   return true;
@@ -2800,8 +2839,18 @@ __global__ void __launch_bounds__(kWosBlock) closest_kernel(const GeoDesc *geo, 
       if (have || tri_cur < tri_end || sp > 0) {
         phase = kTraverse;  // the candidate list was full: the search goes on
       } else {
-        closest_store(G, p, found, best2, best_tri, i, dist, closest);
-        phase = kIdle;
+        if (!found && best2 < static_cast<T>(query_radius2)) {
+          // None below the grid's bound (grid_start): without it, from the root.
+          best2 = static_cast<T>(query_radius2);
+          if constexpr (sizeof(T) == 8) c.limit = cull_limit(best2, c.margin);
+          node = 0;
+          have = true;
+          iter = 0;
+          phase = kTraverse;
+        } else {
+          closest_store(G, p, found, best2, best_tri, i, dist, closest);
+          phase = kIdle;
+        }
       }
     }
     const unsigned idle = __ballot_sync(full, phase == kIdle);
@@ -2824,11 +2873,7 @@ __global__ void __launch_bounds__(kWosBlock) closest_kernel(const GeoDesc *geo, 
           c.p = p;
         } else {
           if (!cull_begin(G, p, best2, c)) {
-            const Plain64 r = nearest_plain64(&G, p.x, p.y, p.z, best2);
-            err |= r.flags & 0x7fffffffu;
-            found = r.flags >> 31;
-            best2 = r.best2;
-            best_tri = r.tri;
+            found = nearest_plain(G, p, best2, best_tri, err);
             have = search = false;
             phase = kStep;
           }
@@ -2840,8 +2885,9 @@ __global__ void __launch_bounds__(kWosBlock) closest_kernel(const GeoDesc *geo, 
             best2 = fminf(best2, upper * upper);
           } else {
             grid_start(G, c.p, sqrtf(c.limit), upper, node);
-            const float reach = __fadd_ru(upper, c.margin);
-            c.limit = fminf(c.limit, __fmul_ru(reach, reach));
+            const float reach = __fadd_ru(upper, c.margin), reach2 = __fmul_ru(reach, reach);
+            c.limit = fminf(c.limit, reach2);
+            best2 = fmin(best2, static_cast<double>(reach2));
           }
           have = true;
           phase = kTraverse;
@@ -2883,6 +2929,7 @@ __global__ void __launch_bounds__(kWosBlock) closest_kernel(const GeoDesc *geo, 
       }
       if (++iter > G.max_iter || sp > kStack) {
         err |= sp > kStack ? TWOS_DEVERR_STACK : TWOS_DEVERR_ITER;
+        best2 = static_cast<T>(CUDART_INF_F);  // no second search
         have = false;
         sp = 0;
         tri_cur = tri_end;

@@ -203,6 +203,7 @@ __global__ void __launch_bounds__(kCertBlock, 6) cert_walk_kernel(const Validate
   int node = 0, sp = 0;
   bool have = false;
   uint32_t tri_cur = 0, tri_end = 0, iter = 0;
+  float within = CUDART_INF_F;  // the grid's upper bound, where the query relies on it
   for (;;) {
     const unsigned idle = __ballot_sync(full, on && phase == kIdle);
     if (!exhausted && idle != 0u) {
@@ -235,6 +236,16 @@ __global__ void __launch_bounds__(kCertBlock, 6) cert_walk_kernel(const Validate
       if (resume && best > 0.0) {
         resume = false;
         phase = kTraverse;  // `best` is the smallest so far: no bound from below yet
+      } else if (best > within) {
+        // None within the grid's bound (grid_start): without it, from the root.
+        resume = false;
+        within = CUDART_INF_F;
+        const float reach = __fmaf_ru(2.f, c.margin, __double2float_ru(far));
+        c.limit = __fmul_ru(reach, reach);
+        node = sp = 0;
+        have = true;
+        tri_cur = tri_end = iter = 0;
+        phase = kTraverse;
       } else {
         resume = false;
         low = fmax(low, fmin(best, far));
@@ -302,13 +313,18 @@ __global__ void __launch_bounds__(kCertBlock, 6) cert_walk_kernel(const Validate
           float ub = __fadd_ru(__double2float_ru(best), __double2float_ru(s));
           low -= s * (1.0 + 0x1.0p-40);
           best = CUDART_INF;
+          within = CUDART_INF_F;
           float bound, upper;
           int entry = -1;
           if (G.grid && grid_bounds<true>(G, c.p, bound, upper, entry)) {
-            ub = fminf(ub, __fmaf_ru(6.f, G.delta, upper));
+            upper = __fmaf_ru(6.f, G.delta, upper);
+            if (upper < ub && upper < far) within = upper;
+            ub = fminf(ub, upper);
             low = fmax(low, static_cast<double>(bound - G.box_extent - 2.f * c.margin));
           }
-          if (!(low >= far)) {
+          if (low >= far) {
+            within = CUDART_INF_F;
+          } else {
             low = 0.0;
             node = ub < G.entry_radius ? max(entry_of(G, entry), 0) : 0;
             const float reach = __fmaf_ru(2.f, c.margin, fminf(ub, __double2float_ru(far)));
