@@ -272,21 +272,23 @@ def test_a_scaled_mesh_gives_scaled_results(tb, monkeypatch, level, k):
 
 @pytest.mark.parametrize("k", [-38, -34, -32, -28])
 @pytest.mark.parametrize("level", [1, 3])
-def test_a_small_mesh_gives_scaled_results(tb, level, k):
+@pytest.mark.parametrize("cavities", [False, True])
+def test_a_small_mesh_gives_scaled_results(tb, level, k, cavities):
     """The same where the products of the closest-point arithmetic are below
-    FP32's normal numbers and the grid's values far off: searches that find
-    nothing below its bound are made without it."""
+    FP32's normal numbers and the grid's values far off: no search depends
+    on its upper bound, and no cavity is taken for nearer than the surface."""
     V, F = tb.geometry.icosphere(level)
     rng = np.random.default_rng(level)
     P = rng.uniform(-0.9, 0.9, (20000, 3))
-    sites = 0.5 * rng.uniform(-1, 1, (24, 3))
+    sites = 0.5 * rng.uniform(-1, 1, (200, 3))
+    cav = np.array([[0.3, 0.1, 0.0], [-0.4, 0.2, 0.1], [0.7, 0.1, 0.1], [-0.1, -0.75, 0.0]]) if cavities else np.zeros((0, 3))
     got = []
     for a in (1.0, 2.0 ** k):
         cfg = tb.Config(walks=100, precision="fp64", seed=7, epsilon=1e-4 * a, max_steps=4096, query_radius=None,
-                        source=tb.sources.constant(1.0))
+                        cavity_radius=0.1 * a, source=tb.sources.constant(1.0))
         with tb.Mesh(V * a, F) as m:
             d = [m.closest_point(p * a, precision="fp64", with_points=False) / a for p in (P, P[:500])]
-            rows, _ = m.estimate(sites * a, cfg)
+            rows, _ = m.estimate(sites * a, cfg, cavities=cav * a)
         got.append((*d, rows["u"] / a**2, rows["steps"]))
     for x, y in zip(*got):
         np.testing.assert_array_equal(x, y)

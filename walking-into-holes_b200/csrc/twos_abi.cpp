@@ -314,7 +314,7 @@ int open_impl(std::vector<double> &&v, std::vector<uint32_t> &&f, int device, tw
     g.cull_margin = reach >= 1e-12 && reach <= 1e12 && far <= 1e6 * reach
                         ? static_cast<float>(1.0001 * (m->delta + std::ldexp(far, -46)))
                         : 0.f;
-    double extent2 = 0.0;
+    double extent2 = 0.0, small2 = 0.0;
     for (size_t f = 0; f < m->faces.size(); f += 3) {
       double d2 = 0.0;
       for (int a = 0; a < 3; ++a) {
@@ -325,6 +325,7 @@ int open_impl(std::vector<double> &&v, std::vector<uint32_t> &&f, int device, tw
         d2 += e * e;
       }
       extent2 = std::max(extent2, d2);
+      if (d2 < 0x1p-56) small2 += d2;
     }
     g.box_extent = static_cast<float>(1.0001 * std::sqrt(extent2));
     // The closest-point arithmetic multiplies products of an edge and a
@@ -332,6 +333,12 @@ int open_impl(std::vector<double> &&v, std::vector<uint32_t> &&f, int device, tw
     // box (at most 8 half extents from any vertex), FP32 has no room for their
     // squares, and the distance grid's values are no bounds.
     if (!(8.0 * reach * std::sqrt(extent2) < 0x1p60)) g.cull_margin = 0.f;
+    // The same products of triangles below 2^-28 lose digits to FP32's smallest
+    // normal number, and the grid's values where such triangles cover more than
+    // the error bound (a small mesh, not the tip of a graded one): without
+    // this, FP64 walks among cavities of an 80-triangle sphere of 2^-32 left
+    // it, since the grid put its surface beyond the cavities.
+    if (std::sqrt(small2) > 0.25 * m->delta) g.cull_margin = 0.f;
     // A query visits each node and tests each triangle at most once.
     g.max_iter = static_cast<uint32_t>(
         std::min<uint64_t>(2ull * (m->bvh.nodes.size() + m->faces.size() / 3) + 16, 0xffffffffull));
