@@ -326,3 +326,33 @@ def test_walks_between_needles(tb, monkeypatch, precision):
     if precision == "fp64":
         for key in got[0][2]:
             np.testing.assert_array_equal(got[0][2][key], got[1][2][key])
+
+
+@pytest.mark.parametrize("shape", ["cube1", "cube8", "sphere3", "noise4"])
+def test_of_equidistant_triangles_the_same_one_is_met(tb, shape):
+    """Points of a lattice (on planes of symmetry and edges' normals) and at
+    random: the FP64 closest point is the one of a search of the FP64 nodes,
+    which a mesh beyond FP32's range takes -- to the bit in a call with few
+    points, but for the rounding of points on a common edge in a bulk call."""
+    if shape.startswith("cube"):
+        n = int(shape[4:])
+        V, F = _cube(n)  # its triangles, on the axes again
+        g = np.linspace(-1.0, 1.0, n + 1)
+        u, v = np.meshgrid(g, g, indexing="ij")
+        V = np.concatenate([np.roll(np.stack([np.full_like(u, side), u, v], -1).reshape(-1, 3), axis, axis=1)
+                            for axis in range(3) for side in (-1.0, 1.0)])
+    else:
+        V, F = tb.geometry.icosphere(3) if shape == "sphere3" else tb.geometry.noise_sphere(4, 1)
+    t = np.linspace(-1.5, 1.5, 25)
+    P = np.stack(np.meshgrid(t, t, t), -1).reshape(-1, 3)
+    P = np.concatenate([P, np.random.default_rng(1).uniform(-1.5, 1.5, (4000, 3))])
+    a = 2.0 ** 41
+    with tb.Mesh(V, F) as m, tb.Mesh(V * a, F) as far:
+        d, q = far.closest_point(P * a, precision="fp64")
+        small = [m.closest_point(p, precision="fp64") for p in np.array_split(P, 2)]
+        bulk = m.closest_point(P, precision="fp64")
+    assert len(P) > 16384
+    np.testing.assert_array_equal(np.concatenate([x[0] for x in small]), d / a)
+    np.testing.assert_array_equal(np.concatenate([x[1] for x in small]), q / a)
+    np.testing.assert_array_equal(bulk[0], d / a)
+    np.testing.assert_allclose(bulk[1], q / a, rtol=0, atol=2.0 ** -47)

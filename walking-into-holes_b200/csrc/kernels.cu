@@ -805,20 +805,82 @@ __device__ __forceinline__ Vec<float> tri_point(const Vec<float> &ap, const Vec<
   return add_scaled(add_scaled(ap, ab, -v), ac, -w);
 }
 
-// FP64 closest-point test of the held candidates.
+// Of two triangles at the same FP64 distance from p, the one that a search of
+// the FP64 nodes, nearer child first, meets first: it decides the closest point
+// returned, and the two points can be far apart.  Where the points are the same
+// (a common vertex: most ties; within `near` of their size) i stands for both,
+// which `ties` notes (kTieSame); a triangle with another point cannot then be
+// compared with i alone, and kTieOpen leaves the decision to the search itself
+// (first_of_tied).  Out of line: ties are few.
+constexpr uint32_t kTieSame = 1u, kTieOpen = 2u;
+struct Tied {
+  uint32_t tri, ties;
+};
+__device__ __noinline__ Tied first_met(const GeoDesc *g, double x, double y, double z, uint32_t i, uint32_t j,
+                                       double near, uint32_t ties) {
+  const Vec<double> p{x, y, z};
+  Vec<double> a, b, c;
+  load_tri(g->tris_d, i, a, b, c);
+  const Vec<double> q = tri_closest(p, a, b, c);
+  load_tri(g->tris_d, j, a, b, c);
+  const Vec<double> r = tri_closest(p, a, b, c);
+  const double apart = fmax(fabs(q.x - r.x), fmax(fabs(q.y - r.y), fabs(q.z - r.z)));
+  if (apart <= near * (fabs(q.x) + fabs(q.y) + fabs(q.z))) return {i, ties | kTieSame};
+  if (ties & kTieSame) return {i, ties | kTieOpen};
+  const uint32_t lo = min(i, j), hi = max(i, j);
+  int node = 0;
+  for (int depth = 0; node >= 0 && depth <= kMaxDepth; ++depth) {
+    const int4 ch = __ldg(&g->nodes_d[node].child);
+    const uint32_t right = ~static_cast<uint32_t>(ch.y);  // of a leaf: first triangle and count
+    const uint32_t mid = ch.y >= 0 ? __ldg(g->node_first + ch.y) : (right & 7u) ? right >> 3 : 0xffffffffu;
+    if (lo < mid && hi >= mid) {  // the subtree where they part
+      double dl, dr;
+      int cl, cr;
+      node_dist2(g->nodes_d, node, p, dl, dr, cl, cr);
+      return {dr < dl ? hi : lo, ties};
+    }
+    node = hi < mid ? ch.x : ch.y;
+  }
+  return {lo, ties};
+}
+
+// The same for points that are the same but for rounding, nearly always.
+__device__ __forceinline__ float point_mark(const Vec<double> &q) {
+  return static_cast<float>(q.x + 0.7548776662466927 * q.y + 0.5698402909980532 * q.z);
+}
+
+// FP64 closest-point test of the held candidates (TIES: the triangle of several
+// at the same distance as first_met, its notes in *ties, the mark of its point
+// in *mark).  A lane's search of the FP32 nodes meets the same one first but for
+// symmetric points, so points that differ by rounding count as the same (bulk
+// call of 122,591 points: 1.88 ms without a look at ties, 1.95 so, 2.11 with
+// every rounding looked at).
+template <bool TIES = false>
 __device__ __forceinline__ bool cull_flush(const GeoDesc &g, const Vec<double> &p, Cull &c, double &best2,
-                                           uint32_t &best_tri, const uint2 *cand, int stride) {
+                                           uint32_t &best_tri, const uint2 *cand, int stride,
+                                           uint32_t *ties = nullptr, float *mark = nullptr) {
   bool found = false;
   for (int k = 0; k < c.count; ++k) {
     const uint2 e = cand[k * stride];
     if (!(__uint_as_float(e.y) < c.limit)) continue;  // the limit fell below its bound since
     Vec<double> ta, tb, tc;
     load_tri(g.tris_d, e.x, ta, tb, tc);
-    const double d2 = tri_dist2(p, ta, tb, tc);
+    const Vec<double> q = tri_closest(p, ta, tb, tc), dv = sub(p, q);
+    const double d2 = dot3(dv, dv);
     if (d2 < best2) {
       best2 = d2;
       best_tri = e.x;
       found = true;
+      if (TIES) *ties = 0u, *mark = point_mark(q);
+    } else if (TIES && d2 == best2) {
+      if (point_mark(q) == *mark) {
+        *ties |= kTieSame;
+      } else {
+        const Tied t = first_met(&g, p.x, p.y, p.z, best_tri, e.x, 0x1.0p-48, *ties);
+        if (t.tri == e.x) *mark = point_mark(q);
+        best_tri = t.tri;
+        *ties = t.ties;
+      }
     }
   }
   c.count = 0;
@@ -904,6 +966,13 @@ __device__ __noinline__ Plain64 nearest_plain64(const GeoDesc *g, double x, doub
                                      1, err);
   r.flags = err | (found ? 0x80000000u : 0u);
   return r;
+}
+
+// The triangle at the smallest FP64 distance best2 that the search of the FP64
+// nodes meets first (`tri`, one of them, should it meet none).
+__device__ __forceinline__ uint32_t first_of_tied(const GeoDesc &g, const Vec<double> &p, double best2, uint32_t tri) {
+  const Plain64 r = nearest_plain64(&g, p.x, p.y, p.z, best2 * (1.0 + 0x1.0p-40) + 0x1.0p-1000);
+  return r.flags >> 31 && r.best2 == best2 ? r.tri : tri;
 }
 
 // The same, as nearest_geo().
@@ -2241,7 +2310,7 @@ __device__ __forceinline__ int warp_contenders(const GeoDesc &g, const Vec<float
 }
 
 __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<float> &p, float &best2, uint32_t &best_tri,
-                                             uint2 *stack, uint32_t &err) {
+                                             uint2 *stack, uint32_t &err, bool = true) {
   const unsigned full = 0xffffffffu;
   float upper;
   int root;
@@ -2276,8 +2345,9 @@ __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<float> 
   return __shfl_sync(full, static_cast<int>(found), 0) != 0;
 }
 
+// `which`: of several triangles at the distance, the one of first_met is wanted.
 __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<double> &p, double &best2,
-                                             uint32_t &best_tri, uint2 *stack, uint32_t &err) {
+                                             uint32_t &best_tri, uint2 *stack, uint32_t &err, bool which = true) {
   Cull c;
   if (!cull_begin(g, p, best2, c)) return nearest_plain(g, p, best2, best_tri, err);
   float upper;
@@ -2286,21 +2356,42 @@ __device__ __forceinline__ bool warp_nearest(const GeoDesc &g, const Vec<double>
   const float reach = __fadd_ru(upper, c.margin), reach2 = __fmul_ru(reach, reach);
   float limit = fminf(c.limit, reach2);
   double mine = fmin(best2, static_cast<double>(reach2));
-  uint32_t tri = 0xffffffffu, overrun = 0;
+  uint32_t tri = 0xffffffffu, overrun = 0, ties = 0;
   warp_search<true>(g, c.p, node, limit, stack, overrun, [&](uint32_t i, const float4 *r, float lim) {
     if (!(plane_gap2(r[0], r[1], c.p) < lim)) return lim;
     Vec<double> ta, tb, tc;
     load_tri(g.tris_d, i, ta, tb, tc);
     const double d2 = tri_dist2(p, ta, tb, tc);
-    if (!(d2 < mine)) return lim;
+    if (!(d2 < mine)) {
+      if (which && d2 == mine && tri != 0xffffffffu) {
+        const Tied t = first_met(&g, p.x, p.y, p.z, tri, i, 0.0, ties);
+        tri = t.tri;
+        ties = t.ties;
+      }
+      return lim;
+    }
     mine = d2;
     tri = i;
+    ties = 0u;
     return cull_limit(d2, c.margin);
   });
+  const double own = mine;
+  const uint32_t own_tri = tri;
   warp_best(mine, tri);
   err |= overrun;
   if (tri == 0xffffffffu)
     return overrun == 0u && reach2 < best2 && nearest_plain(g, p, best2, best_tri, err);
+  if (which) {
+    const unsigned full = 0xffffffffu;
+    const bool holds = own == mine && own_tri != 0xffffffffu;
+    ties = __reduce_or_sync(full, holds ? ties : 0u);
+    for (unsigned m = __ballot_sync(full, holds && own_tri != tri); m != 0u; m &= m - 1u) {
+      const Tied t = first_met(&g, p.x, p.y, p.z, tri, __shfl_sync(full, own_tri, __ffs(m) - 1), 0.0, ties);
+      tri = t.tri;
+      ties = t.ties;
+    }
+    if (ties & kTieOpen) tri = first_of_tied(g, p, mine, tri);
+  }
   best2 = mine;
   best_tri = tri;
   return true;
@@ -2334,7 +2425,7 @@ __global__ void __launch_bounds__(kWosBlock) site_prepass_kernel(const WosLaunch
     const Vec<T> p = to_frame<T>(L.sites + 3ull * (J.site_begin + (g - J.site_rank)), G);
     T best2 = static_cast<T>(J.query_radius2);
     uint32_t tri = 0;
-    const bool found = warp_nearest(G, p, best2, tri, stack, err);
+    const bool found = warp_nearest(G, p, best2, tri, stack, err, L.site_tri != nullptr);
     if ((threadIdx.x & 31u) == 0) {
       out[g] = found ? best2 : T(-1);
       if (L.site_tri) L.site_tri[g] = tri;
@@ -2801,7 +2892,7 @@ __global__ void __launch_bounds__(kWosBlock) closest_warp_kernel(const GeoDesc *
     const Vec<T> p = to_frame<T>(pts + 3 * i, G);
     T best2 = static_cast<T>(query_radius2);
     uint32_t best_tri = 0;
-    const bool found = warp_nearest(G, p, best2, best_tri, stack, err);
+    const bool found = warp_nearest(G, p, best2, best_tri, stack, err, closest != nullptr);
     if ((threadIdx.x & 31u) == 0) closest_store(G, p, found, best2, best_tri, i, dist, closest);
   }
   if (err) atomicOr(error, err);
@@ -2829,13 +2920,14 @@ __global__ void __launch_bounds__(kWosBlock) closest_kernel(const GeoDesc *geo, 
   Vec<T> p{T(0), T(0), T(0)};
   Cull c{{0.f, 0.f, 0.f}, 0.f, 0.f, 0};  // FP32: p and the threshold best2
   T best2 = T(0);
-  uint32_t best_tri = 0, tri_cur = 0, tri_end = 0, iter = 0;
+  uint32_t best_tri = 0, tri_cur = 0, tri_end = 0, iter = 0, ties = 0;
   int node = 0, sp = 0;
   bool have = false, found = false, exhausted = false;  // exhausted is warp-uniform
+  float mark = 0.f;
   int phase = kIdle;
   for (;;) {
     if (phase == kStep) {
-      if constexpr (sizeof(T) == 8) found |= cull_flush(G, p, c, best2, best_tri, cand, kWosBlock);
+      if constexpr (sizeof(T) == 8) found |= cull_flush<true>(G, p, c, best2, best_tri, cand, kWosBlock, &ties, &mark);
       if (have || tri_cur < tri_end || sp > 0) {
         phase = kTraverse;  // the candidate list was full: the search goes on
       } else {
@@ -2848,6 +2940,9 @@ __global__ void __launch_bounds__(kWosBlock) closest_kernel(const GeoDesc *geo, 
           iter = 0;
           phase = kTraverse;
         } else {
+          if constexpr (sizeof(T) == 8) {
+            if (found && closest && (ties & kTieOpen)) best_tri = first_of_tied(G, p, best2, best_tri);
+          }
           closest_store(G, p, found, best2, best_tri, i, dist, closest);
           phase = kIdle;
         }
@@ -2867,7 +2962,7 @@ __global__ void __launch_bounds__(kWosBlock) closest_kernel(const GeoDesc *geo, 
         best2 = static_cast<T>(query_radius2);
         found = false;
         sp = 0;
-        tri_cur = tri_end = iter = 0;
+        tri_cur = tri_end = iter = ties = 0;
         bool search = true;
         if constexpr (sizeof(T) == 4) {
           c.p = p;

@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(kWosBlock) validate_center_kernel(const Valida
     double best2 = CUDART_INF;
     uint32_t tri = 0;
     double d = CUDART_INF;
-    if (warp_nearest(G, v, best2, tri, stack, err)) d = sqrt(best2);
+    if (warp_nearest(G, v, best2, tri, stack, err, false)) d = sqrt(best2);
     double dm = CUDART_INF;
     Cull c;
     if (cull_begin(G, v, best2, c)) {
