@@ -1,6 +1,7 @@
 """Where a closest-point query's bounds are tight: candidate lists that do and
 do not fit, and the limits of the searches."""
 import ctypes
+import time
 
 import numpy as np
 import pytest
@@ -356,3 +357,25 @@ def test_of_equidistant_triangles_the_same_one_is_met(tb, shape):
     np.testing.assert_array_equal(np.concatenate([x[1] for x in small]), q / a)
     np.testing.assert_array_equal(bulk[0], d / a)
     np.testing.assert_allclose(bulk[1], q / a, rtol=0, atol=2.0 ** -47)
+
+
+@pytest.mark.parametrize("n", [12000, 20000])
+@pytest.mark.parametrize("distance", [1e4, 1e6])
+def test_a_far_point_takes_no_longer_than_without_fp32(tb, n, distance):
+    """FP32 prunes less the farther a point is: a call with far points takes at
+    most twice what it takes for a mesh beyond FP32's range, which is searched
+    by the FP64 nodes, and gives its distances."""
+    V, F = tb.geometry.noise_sphere(5, 1)
+    P = np.random.default_rng(2).normal(size=(n, 3))
+    P *= distance / np.linalg.norm(P, axis=1)[:, None]
+    got = []
+    for a in (1.0, 2.0 ** 41):
+        with tb.Mesh(V * a, F) as m:
+            t = []
+            for _ in range(6):
+                t0 = time.perf_counter()
+                d = m.closest_point(P * a, precision="fp64", with_points=False) / a
+                t.append(time.perf_counter() - t0)
+        got.append((min(t), d))
+    np.testing.assert_array_equal(got[0][1], got[1][1])
+    assert got[0][0] < 2 * got[1][0]
