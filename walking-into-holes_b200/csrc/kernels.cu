@@ -966,12 +966,17 @@ struct Plain64 {
   uint32_t tri;
   uint32_t flags;  // error bits | found << 31
 };
-__device__ __noinline__ Plain64 nearest_plain64(const GeoDesc *g, double x, double y, double z, double best2) {
+// `warm`: a triangle to be tested first (kNoTri: none).
+constexpr uint32_t kNoTri = 0xffffffffu;
+__device__ __noinline__ Plain64 nearest_plain64(const GeoDesc *g, double x, double y, double z, double best2,
+                                                uint32_t warm = kNoTri) {
   uint2 stack[kStack];
   Plain64 r{best2, 0u, 0u};
-  uint32_t err = 0;
-  const bool found = nearest<double>(g->nodes_d, g->tris_d, g->max_iter, Vec<double>{x, y, z}, r.best2, r.tri, stack,
-                                     1, err);
+  const Vec<double> p{x, y, z};
+  uint32_t err = 0, full = 0;
+  bool found = warm != kNoTri && tri_test(g->tris_d, warm, p, r.best2, full);
+  if (found) r.tri = warm;
+  found |= nearest<double>(g->nodes_d, g->tris_d, g->max_iter, p, r.best2, r.tri, stack, 1, err);
   r.flags = err | (found ? 0x80000000u : 0u);
   return r;
 }
@@ -1423,7 +1428,8 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
     // four-wide form starts at its root: the table holds binary nodes.)
     if constexpr (sizeof(T) == 8) {
       if (!cull_begin(G, pos, best2, cull)) {
-        const Plain64 r = nearest_plain64(&G, pos.x, pos.y, pos.z, best2);
+        const Plain64 r =
+            nearest_plain64(&G, pos.x, pos.y, pos.z, best2, L.warm && tri_ok ? static_cast<uint32_t>(best_tri) : kNoTri);
         err |= r.flags & 0x7fffffffu;
         found = tri_ok = r.flags >> 31;
         set_best2(r.best2);
