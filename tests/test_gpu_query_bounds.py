@@ -379,3 +379,26 @@ def test_a_far_point_takes_no_longer_than_without_fp32(tb, n, distance):
         got.append((min(t), d))
     np.testing.assert_array_equal(got[0][1], got[1][1])
     assert got[0][0] < 2 * got[1][0]
+
+
+@pytest.mark.parametrize("offset", [1e5, 1e8, 1e9])
+def test_a_mesh_far_from_the_origin_is_searched_like_one_at_it(tb, offset):
+    """Coordinates a hundred thousand to a billion half extents from the
+    origin: candidate lists, and the FP64 distances and estimates of the FP64
+    nodes (which the same mesh beyond FP32's range takes)."""
+    V, F = tb.geometry.noise_sphere(4, 1)
+    V = V + offset * np.array([1.0, -0.7, 0.4])
+    rng = np.random.default_rng(5)
+    o = V.mean(0)
+    P, sites, cav = o + rng.uniform(-1.2, 1.2, (20000, 3)), o + rng.uniform(-0.4, 0.4, (40, 3)), o + np.array([[0.3, 0.1, 0.0], [-0.4, 0.2, 0.1]])
+    got = []
+    for a in (1.0, 2.0 ** 41):
+        cfg = tb.Config(walks=100, precision="fp64", seed=7, epsilon=1e-4 * a, max_steps=4096, cavity_radius=0.1 * a,
+                        query_radius=None, source=tb.sources.constant(1.0))
+        with tb.Mesh(V * a, F) as m:
+            assert (m.candidate_lists()["listed_cells"] > 0) == (a == 1.0)
+            d = [m.closest_point(p * a, precision="fp64", with_points=False) / a for p in (P, P[:500])]
+            rows = [m.estimate(sites * a, cfg, cavities=c)[0] for c in (None, cav * a)]
+        got.append((*d, *(r["u"] / a**2 for r in rows), *(r["steps"] for r in rows)))
+    for x, y in zip(*got):
+        np.testing.assert_array_equal(x, y)

@@ -307,11 +307,11 @@ int open_impl(std::vector<double> &&v, std::vector<uint32_t> &&f, int device, tw
     g.delta = static_cast<float>(m->delta);
     // FP64 queries prune with FP32 bounds where FP32 can hold them: squares
     // of coordinates and of the margin stay in range, and the FP64 rounding
-    // of coordinates far from the origin (2^-46 of their size, more than the
-    // closest-point arithmetic loses) stays far below the margin.
+    // of coordinates far from the origin (2^-46 of their size, a hundred times
+    // what the closest-point arithmetic loses) is at most eight times delta.
     double far = 0.0;
     for (int a = 0; a < 3; ++a) far = std::max(far, std::max(std::fabs(m->bmin[a]), std::fabs(m->bmax[a])));
-    g.cull_margin = reach >= 1e-12 && reach <= 1e12 && far <= 1e6 * reach
+    g.cull_margin = reach >= 1e-12 && reach <= 1e12 && far <= 0x1p30 * reach
                         ? static_cast<float>(1.0001 * (m->delta + std::ldexp(far, -46)))
                         : 0.f;
     double extent2 = 0.0, small2 = 0.0;
