@@ -1018,8 +1018,8 @@ __device__ __forceinline__ bool nearest_geo(const GeoDesc &g, const Vec<T> &p, T
   uint2 *cand = stack + kNearShared * stride;
   uint2 deep[kStack + 1 - kNearShared];
   float upper;
-  int node, sp = 0;
-  bool found = false, have = true;
+  int node;
+  bool found = false;
   const T from = best2;
   if constexpr (sizeof(T) == 4) {
     c.p = p;
@@ -1032,95 +1032,96 @@ __device__ __forceinline__ bool nearest_geo(const GeoDesc &g, const Vec<T> &p, T
     c.limit = fminf(c.limit, reach2);
     best2 = fmin(best2, static_cast<double>(reach2));
   }
-  uint32_t tri_cur = 0, tri_end = 0, iter = 0;
 #pragma unroll 1
   for (;;) {
-    const float limit = [&]() -> float {
-      if constexpr (sizeof(T) == 4)
-        return best2;
-      else
-        return c.limit;
-    }();
-    bool flush = false, done = false;
-    if (tri_cur >= tri_end) {
-      while (!have && sp > 0) {
-        --sp;
-        const uint2 e = sp < kNearShared ? stack[sp * stride] : deep[sp - kNearShared];
-        if (__uint_as_float(e.y) < limit) {
-          node = static_cast<int>(e.x);
-          have = true;
-        }
-      }
-      done = !have;
-      if (have && node < 0) {
-        const uint32_t enc = ~static_cast<uint32_t>(node);
-        tri_cur = enc >> 3;
-        tri_end = tri_cur + (enc & 7u);
-        have = false;
-      }
-    }
-    if (!done && (++iter > g.max_iter || sp > kStack)) {
-      err |= sp > kStack ? TWOS_DEVERR_STACK : TWOS_DEVERR_ITER;
-      done = true;
-      best2 = fmax(best2, from);  // no second search
-    }
-    if (!done) {
-      const bool on_tri = tri_cur < tri_end;
-      const char *at = on_tri ? reinterpret_cast<const char *>(g.tris_f + tri_cur)
-                              : reinterpret_cast<const char *>(g.nodes_f + node);
-      float4 r0, r1, r2, r3, r4{}, r5{};
-      ldg32(at, r0, r1);
-      ldg32(at + 32, r2, r3);
-      ldg32_if(!on_tri, at + 64, r4, r5);
-      if (on_tri) {
-        if constexpr (sizeof(T) == 4) {
-          if (plane_gap2(r0, r1, c.p) < best2) {
-            const float d2 = tri_dist2(c.p, Vec<float>{r1.x, r1.y, r1.z}, Vec<float>{r2.x, r2.y, r2.z},
-                                       Vec<float>{r3.x, r3.y, r3.z});
-            if (d2 < best2) {
-              best2 = d2;
-              best_tri = tri_cur;
-              found = true;
-            }
+    uint32_t tri_cur = 0, tri_end = 0, iter = 0;
+    int sp = 0;
+    bool have = true;
+#pragma unroll 1
+    for (;;) {
+      const float limit = [&]() -> float {
+        if constexpr (sizeof(T) == 4)
+          return best2;
+        else
+          return c.limit;
+      }();
+      bool flush = false, done = false;
+      if (tri_cur >= tri_end) {
+        while (!have && sp > 0) {
+          --sp;
+          const uint2 e = sp < kNearShared ? stack[sp * stride] : deep[sp - kNearShared];
+          if (__uint_as_float(e.y) < limit) {
+            node = static_cast<int>(e.x);
+            have = true;
           }
-          ++tri_cur;
-        } else {
-          // A full candidate list is tested first; the triangle comes again.
-          uint32_t full = 0;
-          flush = cull_tri(tri_cur, r0, r1, r2, r3, c, cand, stride, full);
-          if (!flush) ++tri_cur;
         }
-      } else {
-        float dl, dr;
-        int cl, cr;
-        node_bounds(r0, r1, r2, r3, r4, r5, c.p, dl, dr, cl, cr);
-        const bool vl = dl < limit, vr = dr < limit, swap = dr < dl;
-        if (vl && vr) {
-          const uint2 e = make_uint2(static_cast<uint32_t>(swap ? cl : cr), __float_as_uint(swap ? dl : dr));
-          if (sp < kNearShared)
-            stack[sp * stride] = e;
-          else
-            deep[sp - kNearShared] = e;
-          ++sp;
+        done = !have;
+        if (have && node < 0) {
+          const uint32_t enc = ~static_cast<uint32_t>(node);
+          tri_cur = enc >> 3;
+          tri_end = tri_cur + (enc & 7u);
+          have = false;
         }
-        have = vl || vr;
-        node = vl && !(vr && swap) ? cl : cr;
       }
+      if (!done && (++iter > g.max_iter || sp > kStack)) {
+        err |= sp > kStack ? TWOS_DEVERR_STACK : TWOS_DEVERR_ITER;
+        done = true;
+        best2 = fmax(best2, from);  // no second search
+      }
+      if (!done) {
+        const bool on_tri = tri_cur < tri_end;
+        const char *at = on_tri ? reinterpret_cast<const char *>(g.tris_f + tri_cur)
+                                : reinterpret_cast<const char *>(g.nodes_f + node);
+        float4 r0, r1, r2, r3, r4{}, r5{};
+        ldg32(at, r0, r1);
+        ldg32(at + 32, r2, r3);
+        ldg32_if(!on_tri, at + 64, r4, r5);
+        if (on_tri) {
+          if constexpr (sizeof(T) == 4) {
+            if (plane_gap2(r0, r1, c.p) < best2) {
+              const float d2 = tri_dist2(c.p, Vec<float>{r1.x, r1.y, r1.z}, Vec<float>{r2.x, r2.y, r2.z},
+                                         Vec<float>{r3.x, r3.y, r3.z});
+              if (d2 < best2) {
+                best2 = d2;
+                best_tri = tri_cur;
+                found = true;
+              }
+            }
+            ++tri_cur;
+          } else {
+            // A full candidate list is tested first; the triangle comes again.
+            uint32_t full = 0;
+            flush = cull_tri(tri_cur, r0, r1, r2, r3, c, cand, stride, full);
+            if (!flush) ++tri_cur;
+          }
+        } else {
+          float dl, dr;
+          int cl, cr;
+          node_bounds(r0, r1, r2, r3, r4, r5, c.p, dl, dr, cl, cr);
+          const bool vl = dl < limit, vr = dr < limit, swap = dr < dl;
+          if (vl && vr) {
+            const uint2 e = make_uint2(static_cast<uint32_t>(swap ? cl : cr), __float_as_uint(swap ? dl : dr));
+            if (sp < kNearShared)
+              stack[sp * stride] = e;
+            else
+              deep[sp - kNearShared] = e;
+            ++sp;
+          }
+          have = vl || vr;
+          node = vl && !(vr && swap) ? cl : cr;
+        }
+      }
+      if constexpr (sizeof(T) == 8) {
+        if (flush || done) found |= cull_flush(g, p, c, best2, best_tri, cand, stride);
+      }
+      if (done) break;
     }
-    if constexpr (sizeof(T) == 8) {
-      if (flush || done) found |= cull_flush(g, p, c, best2, best_tri, cand, stride);
-    }
-    if (done) {
-      if (found || !(best2 < from)) break;
-      // None below the grid's bound (grid_start): without it, from the root.
-      best2 = from;
-      if constexpr (sizeof(T) == 8) c.limit = cull_limit(from, c.margin);
-      node = sp = 0;
-      have = true;
-      tri_cur = tri_end = iter = 0;
-    }
+    if (found || !(best2 < from)) return found;
+    // None below the grid's bound (grid_start): without it, from the root.
+    best2 = from;
+    if constexpr (sizeof(T) == 8) c.limit = cull_limit(from, c.margin);
+    node = 0;
   }
-  return found;
 }
 
 __device__ __forceinline__ uint32_t find_job(const JobDesc *jobs, uint32_t n, uint64_t wid) {
