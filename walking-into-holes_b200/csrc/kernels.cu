@@ -1225,6 +1225,10 @@ enum : int { kIdle = 0, kTraverse = 1, kStep = 2, kBegin = 3, kFirst = 4, kAgain
 // (double-double) 128 (512 threads: they spill below, and their local memory
 // then shares the L1 with the BVH; 2,000 x 512 FP64 walks on 81,920 triangles
 // 39 ms with 80 registers and 32 with 120, the gradient form 4.2 and 2.7).
+// The FP64 forms and the mixed compliance and hot forms (on the binary BVH) do
+// not spill; of the mixed forms, boundary mode spills 4 bytes, paired
+// centre-source walks 12 (28 with claims), four-wide ones 12 to 18, and the
+// gradient 20 to 64.
 template <typename T, int MODE, int SRC>
 constexpr int wos_min_blocks(int block) {
   const int threads = sizeof(T) == 8 || SRC == TWOS_SOURCE_EXACT           ? 512
@@ -1245,8 +1249,10 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
   constexpr bool EXACT = SRC == TWOS_SOURCE_EXACT && MODE != kModeBoundary;
   constexpr bool GRAD = MODE == kModeGradient;
   constexpr bool PAIRED = MODE == TWOS_MODE_PAIRED || GRAD;
-  // Dynamic shared memory: the traversal stacks (kStack entries per thread,
-  // column-major so a warp's accesses hit distinct banks), then the tables.
+  // Dynamic shared memory: per thread the first kShared entries of the
+  // traversal stack and, in the FP64 form, kCand candidates (column-major so a
+  // warp's accesses hit distinct banks), then the walks' state (Cell), then
+  // the tables.
   extern __shared__ __align__(16) unsigned char s_dyn[];
   uint2 *s_stack = reinterpret_cast<uint2 *>(s_dyn);
   unsigned char *s_cold = s_dyn + wos_stack_entries<T>() * BLOCK * sizeof(uint2);
@@ -1429,8 +1435,8 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
     // four-wide form starts at its root: the table holds binary nodes.)
     if constexpr (sizeof(T) == 8) {
       if (!cull_begin(G, pos, best2, cull)) {
-        const Plain64 r =
-            nearest_plain64(&G, pos.x, pos.y, pos.z, best2, L.warm && tri_ok ? static_cast<uint32_t>(best_tri) : kNoTri);
+        const uint32_t warm = L.warm && tri_ok ? static_cast<uint32_t>(best_tri) : kNoTri;
+        const Plain64 r = nearest_plain64(&G, pos.x, pos.y, pos.z, best2, warm);
         err |= r.flags & 0x7fffffffu;
         found = tri_ok = r.flags >> 31;
         set_best2(r.best2);
@@ -1878,10 +1884,9 @@ __global__ void __launch_bounds__(BLOCK, wos_min_blocks<T, MODE, SRC>(BLOCK)) wo
       continue;
     }
 
-    // ---- one unit of closest-point traversal.  The warp runs one kind of
-    // unit per iteration -- triangle tests or node tests/pops -- whichever
-    // more of its traversing lanes need, so each iteration executes one code
-    // path instead of the union of both.
+    // ---- a batch of traversal units for every traversing lane.  With `vote`
+    // only the lanes whose next unit is of the commoner kind -- triangle, or
+    // node and pops -- take it.
     bool take = phase == kTraverse;
     if (L.vote) {  // warp-uniform; the ballots cost nothing when it is off
       const bool want_tri = phase == kTraverse && tri_cur < tri_end;
@@ -2976,8 +2981,9 @@ __device__ __forceinline__ void closest_store(const GeoDesc &G, const Vec<T> &p,
 }
 
 // A warp per point: a call with few points is as long as its longest query,
-// and a lane alone waits for memory at every node (3,000 points, 81,920
-// triangles, FP64: 1.70 ms with a lane each, 0.20 with a warp).
+// and a lane alone waits for memory at every node (5,000 points, 81,920
+// triangles, FP64: 1.69 ms with a lane each, 0.25 with a warp, of which 0.03
+// settle ties).
 template <typename T>
 __global__ void __launch_bounds__(kWosBlock) closest_warp_kernel(const GeoDesc *geo, const double *pts, uint64_t n,
                                                                  double query_radius2, double *dist, double *closest,
@@ -3003,7 +3009,7 @@ __global__ void __launch_bounds__(kWosBlock) closest_warp_kernel(const GeoDesc *
 // its search, one set of loads per unit, and takes the next point from the
 // queue when it ends, so a warp does not wait for its longest query (call of
 // 122,591 points, 81,920 triangles, FP64: 3.1 ms with a fixed point per
-// thread, 1.9 with the queue).
+// thread, 1.96 with the queue).
 template <typename T>
 __global__ void __launch_bounds__(kWosBlock) closest_kernel(const GeoDesc *geo, const double *pts, uint64_t n,
                                                             double query_radius2, double *dist, double *closest,
@@ -3201,8 +3207,10 @@ cudaError_t launch_ball_green(const double *cases, uint32_t n, double *out, uint
 // Points up to which each gets a warp.  The warp's search costs more
 // instructions in all, so it wins where a call is as long as its longest query
 // (calls, ms, lane / warp, FP64, 327,680 triangles: 3,000 points of the solid
-// 3.6 / 0.28, 30,000 2.4 / 1.3, 122,591 3.5 / 3.8; 30,000 near the surface
-// 0.26 / 0.32).
+// 2.5 / 0.34, 30,000 2.8 / 1.4, 60,000 3.2 / 2.7, 122,591 3.9 / 5.2; near the
+// surface 10,000 0.15 / 0.16, 30,000 0.24 / 0.33, 122,591 0.68 / 1.28).  The
+// line lies between the two: calls in the solid would gain by a warp up to
+// some 80,000 points, those near the surface lose from 10,000 on.
 constexpr uint64_t kWarpPoints = 16384;
 
 cudaError_t launch_closest(int precision, const GeoDesc *geo_dev, const double *pts, uint64_t n,
@@ -3601,13 +3609,13 @@ cudaError_t launch_topk(const double *keys, uint32_t n, uint32_t k, uint32_t *in
 
 }  // namespace twos
 
-// Differential WoS kernels (use nearest<double> above).
+// Differential WoS kernels (use nearest_geo and cull_begin above).
 #include "diffwos.cuh"
 
-// Certified validation kernels (use the stream, direction and nearest<double> above).
+// Certified validation kernels (use the stream, direction, warp_nearest and warp_search above).
 #include "validate.cuh"
 
-// Array-RQMC / matched MC lockstep walks (use nearest<T>, the stream and warp sums above).
+// Array-RQMC / matched MC lockstep walks (use nearest_geo, warp_nearest, the stream and warp sums above).
 #include "rqmc.cuh"
 
 #include "wavefront.cuh"

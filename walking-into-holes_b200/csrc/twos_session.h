@@ -41,8 +41,11 @@ struct DevBuf {
 // the next, since allocating and freeing a dozen buffers took 2 to 8 ms of a
 // call and waited for the device each time.  trim(), at the end of a call,
 // gives back what is larger than kKeepBytes, so a session holds at most
-// kScratch * kKeepBytes; closing it frees the rest.  A session's calls run one
-// at a time on its stream and wait for it before they return.
+// kScratch * kKeepBytes; closing it frees the rest.  A call that needs more of
+// a buffer allocates and frees that one each time, as all calls did before: a
+// Differential WoS chunk of more than 599,186 walks, 56 bytes each, is the
+// smallest.  A session's calls run one at a time on its stream and wait for it
+// before they return.
 constexpr int kScratch = 18;
 constexpr size_t kKeepBytes = size_t(32) << 20;
 struct Scratch {

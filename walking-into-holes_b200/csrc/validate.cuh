@@ -169,14 +169,16 @@ constexpr int kCertStack = 8;  // traversal-stack entries per thread in shared m
 // Here a node costs two FP32 boxes; a query starts from the smaller of the
 // grid's upper bound and the previous distance plus the step (the distance is
 // 1-Lipschitz), at the grid's entry node; each site's first distance comes
-// from V.mesh_distance (40 ms, bound by the ~100 units of a query far from
-// the surface, whose triangles' boxes are nearly equidistant).  A distance d matters only below radius_cap / 0.95:
-// beyond, the step is radius_cap and its points lie within d whatever d is, so
-// a query looks no farther, and there is none where the distance is known to
-// be beyond -- by the previous distance less the steps since, or by the
-// grid's lower bound of the distance to the triangles less the largest extent
-// of a triangle's box: 6.3 ms.  What is left is the chain of up to max_steps
-// FP64 steps and near-surface queries of the longest walks.
+// from V.mesh_distance.  With that the same walks took 40 ms, bound by the
+// ~100 units of a query far from the surface, whose triangles' boxes are nearly
+// equidistant.  But a distance d matters only below radius_cap / 0.95: beyond,
+// the step is radius_cap and its points lie within d whatever d is.  So a query
+// looks no farther, and there is none where the distance is known to be beyond
+// -- by the previous distance less the steps since, or by the grid's lower
+// bound of the distance to the triangles less the largest extent of a
+// triangle's box: 6.3 ms.  What is left is the chain of up to max_steps FP64
+// steps and near-surface queries of the longest walks.  Six blocks per SM leave
+// 80 registers a thread, which spill 40 bytes.
 __global__ void __launch_bounds__(kCertBlock, 6) cert_walk_kernel(const ValidateLaunch V, int lanes) {
   __shared__ uint2 s_stack[(kCertStack + kCand) * kCertBlock];
   __shared__ GeoDesc G;
